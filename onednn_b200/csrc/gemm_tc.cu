@@ -104,7 +104,7 @@ __device__ __forceinline__ ColTerms load_col_terms(const MatmulArgs &a, const Tc
         if (a.wei_zp.ptr) c.wei_zp = load_int(a.wei_zp.dt, a.wei_zp.ptr, (a.wei_zp.mask & 2) ? n : 0);
         if (a.src_zp.ptr) {
             const int zs = ((const int *)a.src_zp.ptr)[0];
-            c.zs_colsum = zs * tp.colsum[n] - (int)a.K * zs * c.wei_zp;
+            c.zs_colsum = zs * ptx::ld_dependent(tp.colsum + n) - (int)a.K * zs * c.wei_zp;
         }
     }
     return c;
@@ -191,7 +191,7 @@ __device__ __forceinline__ void epilogue_rows(const MatmulArgs &a, const TcParam
         if (t.row_sum) {
 #pragma unroll
             for (int j = 0; j < R; ++j)
-                d[j] = (float)((int)r[j] - c.zs_colsum - c.wei_zp * __ldg(tp.rowsum + (FULL ? m0 + j : min(m0 + j, a.M - 1))));
+                d[j] = (float)((int)r[j] - c.zs_colsum - c.wei_zp * ptx::ld_dependent(tp.rowsum + (FULL ? m0 + j : min(m0 + j, a.M - 1))));
         } else {
 #pragma unroll
             for (int j = 0; j < R; ++j) d[j] = (float)((int)r[j] - c.zs_colsum);
@@ -392,7 +392,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         const TensorTerms tt = load_tensor_terms<INT>(a, tp);
         // the zero-point sums come from the kernel launched before this one, which runs beside this
         // kernel's set-up and first mainloop: only the epilogue warps wait for it
-        if (tp.after_prekernel) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (tp.after_prekernel) ptx::grid_dependency_wait();
         uint32_t acc_it = 0;
         for (int tile = blockIdx.x; tile < num_tiles && !*abort_flag; tile += gridDim.x, ++acc_it) {
             const int as = acc_it % ACC_STAGES;

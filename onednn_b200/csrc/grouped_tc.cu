@@ -241,13 +241,13 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     const uint32_t tmem_base = *tmem_base_slot;
     // launched as the programmatic dependent of the planning (or row-sum) kernel: everything above ran
     // beside it; the plan and the row sums are read from here on
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int4 head = __ldg(&plan_global[0]);
+    ptx::grid_dependency_wait();
+    const int4 head = ptx::ld_dependent_int4(&plan_global[0]);
     const int num_tiles = head.x, groups = head.y;
     const int4 *plan = plan_global;
     if (groups <= PLAN_CACHE_GROUPS) {
         int4 *cache = reinterpret_cast<int4 *>(smem + G_PLAN_OFFSET);
-        for (int i = threadIdx.x; i <= groups; i += blockDim.x) cache[i] = __ldg(&plan_global[i]);
+        for (int i = threadIdx.x; i <= groups; i += blockDim.x) cache[i] = ptx::ld_dependent_int4(&plan_global[i]);
         __syncthreads();
         plan = cache;
     }
@@ -470,7 +470,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                             if (j >= m_hi) continue;
                             const int64_t m = row0 + j;
                             float acc = __uint_as_float(r[j]);
-                            if (a.wei_zp.ptr) acc = fmaf(-zp, __ldg(rowsum + tl.src_row + cidx * 32 + j), acc);
+                            if (a.wei_zp.ptr) acc = fmaf(-zp, ptx::ld_dependent(rowsum + tl.src_row + cidx * 32 + j), acc);
                             float d = __fmul_rn(acc, scale);
                             if (a.bias)
                                 d = __fadd_rn(d,

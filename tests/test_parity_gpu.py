@@ -188,6 +188,25 @@ def test_tcgen05_grouped_matches_oracle(gpu, name):
     assert_parity(got, want, p.dst_dt, name, summation_slack_grouped(p))
 
 
+@pytest.mark.parametrize("M,experts", [(24, 8), (1500, 64)])
+def test_grouped_first_execution_of_a_fresh_primitive(gpu, M, experts):
+    """The tile plan is made by a kernel that the main kernel is launched beside: it must not be read before
+    that kernel has finished.  A fresh primitive has no older plan to read, so its first execution decides,
+    and only when both kernels are in the stream before the first one starts (work of another primitive ahead)."""
+    from onednn_b200.runner import Prepared
+    eng, strm = gpu
+    p = W.moe_grouped(M, 256, 1024, experts)
+    want = O.run_port(p)
+    ahead = Prepared(W.fp8_prefill(2048, 4096, 4096), eng).upload()
+    for attempt in range(8):
+        r = Prepared(p, eng).upload()
+        for _ in range(4):
+            ahead.execute(strm)
+        r.execute(strm)
+        strm.wait()
+        assert_parity(r.download(), want, p.dst_dt, "attempt %d" % attempt, summation_slack_grouped(p))
+
+
 def _woq8(M, K, N, per_n=True, dst_dt=W.BF16, seed=31):
     """bf16 src x s8 weights, one weight scale per column (or per tensor), nothing else."""
     r = np.random.Generator(np.random.PCG64(seed))
