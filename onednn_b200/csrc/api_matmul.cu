@@ -391,17 +391,17 @@ dnnl_status_t tc_accepts(const dnnl_primitive_desc &pd) {
     return dnnl_success;
 }
 
-// Skinny weight-decompression GEMM: few src rows (decode), bf16/f16 src,
-// s4/u4 `ab` weights, weight scales per N or per (K-group, N), optional
+// int4 weight decompression on the tensor cores, any number of rows: bf16/f16
+// src, s4/u4 `ab` weights, weight scales per N or per (K-group, N), optional
 // zero-points with the same grouping (or per tensor).
-dnnl_status_t woq_accepts(const dnnl_primitive_desc &pd) {
+dnnl_status_t woq4_accepts(const dnnl_primitive_desc &pd) {
     if (ref_dense_accepts(pd) != dnnl_success) return dnnl_unimplemented;
     const auto s = pd.src.data_type, w = pd.wei.data_type;
     const auto &attr = pd.attr;
     UNIMPL_IF(!(s == dnnl_bf16 || s == dnnl_f16) || !(w == dnnl_s4 || w == dnnl_u4));
     UNIMPL_IF(is_fp8(pd.dst.data_type) || (pd.bias.ndims && is_fp8(pd.bias.data_type)));
     const dnnl_dim_t M = pd.M(), N = pd.N(), K = pd.K();
-    UNIMPL_IF(M < 1 || M > 32 || N % 32 != 0 || K % 16 != 0 || K < 16);
+    UNIMPL_IF(M < 1 || N % 32 != 0 || K % 16 != 0 || K < 16);
     UNIMPL_IF(N >= (1LL << 31) || K >= (1LL << 31));
     UNIMPL_IF(pd.src.strides[1] != 1 || pd.src.strides[0] % 2 != 0);
     UNIMPL_IF(pd.wei.strides[1] != 1 || pd.wei.strides[0] % 32 != 0 || pd.wei.strides[0] < N);
@@ -420,6 +420,23 @@ dnnl_status_t woq_accepts(const dnnl_primitive_desc &pd) {
             UNIMPL_IF(!wz.group_ndims || wz.groups[1] != 1 || wz.groups[0] != group);
         } else UNIMPL_IF(wz.mask != 0);
     }
+    return dnnl_success;
+}
+
+// Skinny weight-decompression GEMM: few src rows (decode)
+dnnl_status_t woq_accepts(const dnnl_primitive_desc &pd) {
+    UNIMPL_IF(pd.M() > 32);
+    return woq4_accepts(pd);
+}
+
+// More rows than the decode kernels take: src rows by TMA, and weights less zero-points that stay exact
+// in the src's type - bf16 holds every integer up to 256, w - zp with 4-bit zero-points; f16 up to 2048
+dnnl_status_t woq_rows_accepts(const dnnl_primitive_desc &pd) {
+    if (woq4_accepts(pd) != dnnl_success) return dnnl_unimplemented;
+    UNIMPL_IF(pd.M() <= 32 || pd.M() >= (1LL << 31) || pd.src.strides[0] % 8 != 0 || pd.src.strides[0] < pd.K());
+    const auto &wz = pd.attr.zp(DNNL_ARG_WEIGHTS);
+    if (wz.set)
+        UNIMPL_IF(!one_of(wz.dt, {dnnl_s4, dnnl_u4}) && !(pd.src.data_type == dnnl_f16 && one_of(wz.dt, {dnnl_s8, dnnl_u8})));
     return dnnl_success;
 }
 
@@ -508,6 +525,10 @@ dnnl_status_t impl_accepts(const dnnl_primitive_desc &pd, int impl, std::string 
             if (pd.grouped) return dnnl_unimplemented;
             name = "cuda:woq:skinny";
             return woq_accepts(pd);
+        case IMPL_WOQ_ROWS:
+            if (pd.grouped) return dnnl_unimplemented;
+            name = "cuda:tcgen05:woq4_rows";
+            return woq_rows_accepts(pd);
         case IMPL_TCGEN05_GEMM:
             if (pd.grouped) return dnnl_unimplemented;
             name = is_int8(pd.src.data_type) ? "cuda:tcgen05:int8" : "cuda:tcgen05:fp8";
@@ -1150,6 +1171,10 @@ static dnnl_status_t execute_matmul_2d(const_dnnl_primitive_t primitive, const d
                     cudaMemsetAsync(scratch, 0, ((pd.N() + 255) / 256) * sizeof(int), stream->stream);
                 rc = launch_woq_skinny(a, scratch, pd.engine->sm_count, stream->stream);
             }
+            break;
+        case IMPL_WOQ_ROWS:
+            if (!woq_rows_pointers_ok(a)) rc = launch_ref(a, stream->stream); // misaligned user pointers
+            else rc = launch_woq_rows(a, pd.engine->sm_count, stream->stream);
             break;
         case IMPL_GROUPED_TC:
             if (!grouped_tc_pointers_ok(a)) rc = launch_ref(a, stream->stream);

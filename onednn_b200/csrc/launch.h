@@ -56,6 +56,10 @@ size_t woq_tc_scratch_bytes(int64_t M, int64_t N, int64_t K, int sm_count);
 bool woq_tc_pointers_ok(const MatmulArgs &a);
 bool woq_tc_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_dt);
 
+// int4 weight-decompression GEMM for M > 32 on tcgen05 (woq_rows.cu)
+int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st);
+bool woq_rows_pointers_ok(const MatmulArgs &a);
+
 // tcgen05 grouped (MoE) GEMM, bf16 src x s8 weights (grouped_tc.cu).
 // `scratch`: grouped_tc_scratch_bytes(group_count, M) bytes, no initialisation
 // (tile ranges per group, and the src row sums that weight zero-points need).

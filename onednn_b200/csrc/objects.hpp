@@ -139,6 +139,7 @@ enum impl_id_t : int {
     IMPL_TCGEN05_GEMM = 0, // tensor-core int8 / fp8 GEMM
     IMPL_WOQ_TC, // int4 weight decompression through tensor memory (M <= 32)
     IMPL_WOQ_GEMV, // weight-decompression skinny GEMM (M <= 32), mma.sync
+    IMPL_WOQ_ROWS, // int4 weight decompression through tensor memory, M > 32
     IMPL_GROUPED_TC, // grouped (MoE) tensor-core GEMM
     IMPL_REF, // generic kernels, every attribute
     IMPL_COUNT

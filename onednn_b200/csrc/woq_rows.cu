@@ -1,0 +1,577 @@
+// "cuda:tcgen05:woq4_rows": int4 weight-decompression matmul for more rows than the decode kernels take
+// (prompt processing, M > 32):
+//   dst[M,N] = src[M,K] (bf16/f16) x dequant(weights[K,N] s4/u4 `ab`),
+// scales per column or per (K-group, column), optional 4-bit zero-points (f16 src: 8-bit ones too) with the
+// same grouping or per tensor (fpmath apply_to_int; reference arithmetic: src/cpu/matmul/ref_matmul.cpp:193-233).
+//
+// w - zero_point is an integer that bf16 (f16) holds exactly, so the operand of the MMAs is exact: a nibble
+// becomes 128 + u (f16: 1024 + u) with one LOP3 per two weights and one packed subtraction takes off
+// 128 (+ 8 for s4) + zero_point.  The sums of a K-group are then exact products added in f32, and the group's
+// scale multiplies the finished group sum: tot += scale * sum, in f32 registers of the epilogue.  Nothing is
+// rounded to 16 bits before dst, and no correction by row sums is needed.
+//
+// As in the other decompression kernels the weights are the A operand, in TENSOR MEMORY (128 dst columns = TMEM
+// lanes), and the src rows the B operand from shared memory, so an epilogue lane owns one dst column.  A tile is
+// 128 columns x up to 128 rows: an MMA of up to 128 rows takes about 64 cycles to execute and about as many to
+// issue, so narrower tiles would be paid in issue slots and wider ones would not leave tensor memory for three
+// accumulators (a group of 32 k is two MMAs: with three buffers the fold of one group overlaps the next two).
+// Per-stage (64 k) cost at 128 rows: 4 MMAs = 256 tensor cycles, about 100 converter instructions per warp with
+// two warps per lane quarter, and 64 FMAs per epilogue lane and group.
+//
+// Roles (20 warps): 0 weight tiles by TMA (ring of 4 KB nibble tiles), 1 src tiles by TMA (ring of 128-k tiles:
+// one release per two stages), 2 issues all MMAs, 4-11 converters (two per lane quarter, alternating
+// stages), 12-19 epilogue (two per lane quarter, each half of the rows).  Every mbarrier wait is bounded.
+//
+// Measured on a B200 at K = N = 4096, M = 300, groups of 128, u4 zero-points: 66 us a call; the generic kernel,
+// which such calls took before, 54.3 ms.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <string>
+
+#include "device_math.cuh"
+#include "launch.h"
+#include "objects.hpp"
+#include "sm100_ptx.cuh"
+
+namespace qmm {
+
+namespace {
+
+constexpr int RT_N = 128; // dst columns per tile = TMEM lanes
+constexpr int RT_M = 128; // most src rows per tile
+constexpr int RK = 64; // k per operand stage
+constexpr int RKB = 2 * RK; // k per src stage: two 128-byte swizzle rows of 16-bit values
+constexpr int W_STAGES = 12, A_SLOTS = 4, B_STAGES = 4, ACC_BUFS = 3;
+constexpr int W_BYTES = RK * RT_N / 2; // nibbles as loaded: 64-byte rows
+constexpr int B_BYTES = RT_M * RKB * 2;
+constexpr int R_CONV_WARPS = 8, R_EPI_WARPS = 8;
+constexpr int R_CONV0 = 4, R_EPI0 = R_CONV0 + R_CONV_WARPS;
+constexpr int R_THREADS = 32 * (R_EPI0 + R_EPI_WARPS);
+constexpr int A_SLOT_COLS = RK / 2;
+constexpr int R_A_COL0 = ACC_BUFS * RT_M;
+static_assert(R_A_COL0 + A_SLOTS * A_SLOT_COLS <= 512, "tensor memory");
+constexpr int R_B_OFFSET = 0, R_W_OFFSET = B_STAGES * B_BYTES;
+constexpr int R_BAR_OFFSET = R_W_OFFSET + W_STAGES * W_BYTES;
+constexpr int R_SMEM_BYTES = R_BAR_OFFSET + 512 + 1024;
+static_assert(R_SMEM_BYTES <= 227 * 1024, "shared memory");
+
+struct RowsParams {
+    int num_m_tiles, num_tiles;
+    int tile_rows; // a multiple of 16, at most RT_M: the MMAs' N and the rows of a src box
+    int ksteps; // K / 16
+    int kstages; // ceil(K / 64)
+    int group_steps; // k16 steps per quantization group (ksteps when not grouped along K)
+    int sgn4; // weights are s4 (else u4)
+    int zp_mode; // 0 none, 1 per (group, column), 2 per tensor
+    int fast_store; // no post-ops / dst scale: the value is converted and stored
+    uint32_t idesc;
+};
+
+__device__ __forceinline__ uint32_t and_xor(uint32_t x, uint32_t mask, uint32_t magic) { // (x & mask) ^ magic
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(r) : "r"(x), "r"(mask), "r"(magic));
+    return r;
+}
+__device__ __forceinline__ uint32_t perm(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+}
+__device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t sub_f16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t fma_f16x2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+// 16 TMEM lanes x 32 columns (four k16 steps): see the s8 kernel (grouped_tc.cu) for the fragment
+__device__ __forceinline__ void st_16x128b_x8(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+            "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+            "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+            "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+            : "memory");
+}
+__device__ __forceinline__ void ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr)
+            : "memory");
+}
+__device__ __forceinline__ void mma_ts_16bit(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, bool acc) {
+    asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"((uint32_t)acc)
+            : "memory");
+}
+// post-ops, dst scale, any dst type: rare and large, out of line
+__device__ __noinline__ void finish_store_general(const MatmulArgs &a, float d, int64_t m, int64_t n) {
+    finish_store(a, d, m, n, false);
+}
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity));
+}
+
+// The zero-points of a lane's four columns (n .. n + 3) in group g, as loaded: four nibbles or four bytes
+__device__ __forceinline__ uint32_t load_zp4(const MatmulArgs &a, int g, int64_t n) {
+    if (n >= a.N) return 0u;
+    const int64_t e = (int64_t)g * a.wei_zp.ld + n;
+    if (a.wei_zp.dt == DT_U4 || a.wei_zp.dt == DT_S4) return __ldg((const unsigned short *)a.wei_zp.ptr + (e >> 2));
+    return __ldg((const unsigned *)a.wei_zp.ptr + (e >> 2));
+}
+__device__ __forceinline__ int zp_of(int dt, uint32_t raw, int i) {
+    if (dt == DT_U4 || dt == DT_S4) {
+        const int v = (int)((raw >> (4 * i)) & 15u);
+        return dt == DT_S4 ? (v ^ 8) - 8 : v;
+    }
+    const int v = (int)((raw >> (8 * i)) & 255u);
+    return dt == DT_S8 ? (int)(signed char)v : v;
+}
+
+// MULTI: a 64-k stage may touch several groups (group size not a multiple of 64): the offsets are looked up
+// per k16 step instead of per stage.
+template <bool F16, bool MULTI>
+__global__ void __launch_bounds__(R_THREADS, 1)
+woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
+        const __grid_constant__ MatmulArgs a, const __grid_constant__ RowsParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t *w_full = (uint64_t *)(smem + R_BAR_OFFSET);
+    uint64_t *w_empty = w_full + W_STAGES;
+    uint64_t *b_full = w_empty + W_STAGES;
+    uint64_t *b_empty = b_full + B_STAGES;
+    uint64_t *a_full = b_empty + B_STAGES;
+    uint64_t *a_empty = a_full + A_SLOTS;
+    uint64_t *acc_full = a_empty + A_SLOTS;
+    uint64_t *acc_empty = acc_full + ACC_BUFS;
+    uint32_t *tmem_slot = (uint32_t *)(acc_empty + ACC_BUFS);
+    volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < W_STAGES; ++s) {
+            ptx::mbar_init(&w_full[s], 1);
+            ptx::mbar_init(&w_empty[s], R_CONV_WARPS / 2); // the stage's four converter warps
+        }
+        for (int s = 0; s < B_STAGES; ++s) {
+            ptx::mbar_init(&b_full[s], 1);
+            ptx::mbar_init(&b_empty[s], 1);
+        }
+        for (int s = 0; s < A_SLOTS; ++s) {
+            ptx::mbar_init(&a_full[s], R_CONV_WARPS / 2);
+            ptx::mbar_init(&a_empty[s], 1);
+        }
+        for (int s = 0; s < ACC_BUFS; ++s) {
+            ptx::mbar_init(&acc_full[s], 1);
+            ptx::mbar_init(&acc_empty[s], R_EPI_WARPS);
+        }
+        *abort_flag = 0;
+        ptx::fence_barrier_init();
+        ptx::prefetch_tensormap(&tmW);
+        ptx::prefetch_tensormap(&tmS);
+    }
+    if (warp == 3) ptx::tmem_alloc(tmem_slot, 512);
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    ptx::tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        // ------------------------------------------------ TMA producer of the nibble tiles
+        int s = 0;
+        uint32_t ph = 1;
+        bool ok = true;
+        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+            const int x = (t / p.num_m_tiles) * (RT_N / 2);
+            for (int st = 0; st < p.kstages; ++st) {
+                if (!warp_wait(&w_empty[s], ph)) { ok = false; break; }
+                if (ptx::elect_one()) {
+                    ptx::mbar_arrive_expect_tx(&w_full[s], W_BYTES);
+                    ptx::tma_load_2d(smem + R_W_OFFSET + s * W_BYTES, &tmW, &w_full[s], x, st * RK);
+                }
+                __syncwarp();
+                if (++s == W_STAGES) { s = 0; ph ^= 1; }
+            }
+        }
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(a.status, 5); }
+    } else if (warp == 1) {
+        // ------------------------------------------------ TMA producer of the src tiles (128 k each)
+        int s = 0;
+        uint32_t ph = 1;
+        bool ok = true;
+        const uint32_t half = (uint32_t)p.tile_rows * 128;
+        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+            const int m0 = (t % p.num_m_tiles) * p.tile_rows;
+            for (int st = 0; st < p.kstages; st += 2) {
+                if (!warp_wait(&b_empty[s], ph)) { ok = false; break; }
+                uint8_t *d = smem + R_B_OFFSET + s * B_BYTES;
+                if (ptx::elect_one()) {
+                    const bool two = st + 1 < p.kstages;
+                    ptx::mbar_arrive_expect_tx(&b_full[s], two ? 2 * half : half);
+                    ptx::tma_load_2d(d, &tmS, &b_full[s], st * RK, m0);
+                    if (two) ptx::tma_load_2d(d + B_BYTES / 2, &tmS, &b_full[s], (st + 1) * RK, m0);
+                }
+                __syncwarp();
+                if (++s == B_STAGES) { s = 0; ph ^= 1; }
+            }
+        }
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(a.status, 5); }
+    } else if (warp == 2) {
+        // ------------------------------------------------ MMA issuer
+        int sa = 0, sb = 0, buf = 0;
+        uint32_t pa = 0, pb = 0, pacc = 1;
+        bool ok = true;
+        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+            int left = 0; // k16 steps left in the open group (0: none open)
+            for (int st = 0; st < p.kstages; ++st) {
+                if ((st & 1) == 0 && !warp_wait(&b_full[sb], pb)) { ok = false; break; }
+                if (!warp_wait(&a_full[sa], pa)) { ok = false; break; }
+                ptx::tc_fence_after_sync();
+                const uint64_t bd = ptx::smem_desc_sw128(
+                        ptx::smem_u32(smem + R_B_OFFSET + sb * B_BYTES + (st & 1) * (B_BYTES / 2)), 0, 1024);
+                const uint32_t ta = tmem_base + R_A_COL0 + sa * A_SLOT_COLS;
+                const int nst = min(4, p.ksteps - 4 * st);
+                const bool b_done = (st & 1) || st + 1 == p.kstages;
+                if (nst == 4 && (left >= 4 || (left == 0 && p.group_steps >= 4))) {
+                    // the common stage, whole and inside one group: straight-line code
+                    const bool fresh = left == 0;
+                    if (fresh) {
+                        if (!warp_wait(&acc_empty[buf], pacc)) { ok = false; break; }
+                        ptx::tc_fence_after_sync();
+                        left = min(p.group_steps, p.ksteps - 4 * st);
+                    }
+                    left -= 4;
+                    const uint32_t d = tmem_base + buf * RT_M;
+                    if (ptx::elect_one()) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) mma_ts_16bit(d, ta + 8 * q, bd + 2 * q, p.idesc, q > 0 || !fresh);
+                        if (left == 0) ptx::tc_commit(&acc_full[buf]);
+                        ptx::tc_commit(&a_empty[sa]);
+                        if (b_done) ptx::tc_commit(&b_empty[sb]);
+                    }
+                    __syncwarp();
+                    if (left == 0 && ++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
+                } else {
+                    for (int q = 0; q < nst; ++q) {
+                        const bool fresh = left == 0;
+                        if (fresh) {
+                            if (!warp_wait(&acc_empty[buf], pacc)) { ok = false; break; }
+                            ptx::tc_fence_after_sync();
+                            left = min(p.group_steps, p.ksteps - (4 * st + q));
+                        }
+                        --left;
+                        if (ptx::elect_one()) {
+                            mma_ts_16bit(tmem_base + buf * RT_M, ta + 8 * q, bd + 2 * q, p.idesc, !fresh);
+                            if (left == 0) ptx::tc_commit(&acc_full[buf]);
+                        }
+                        __syncwarp();
+                        if (left == 0 && ++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
+                    }
+                    if (!ok) break;
+                    if (ptx::elect_one()) {
+                        ptx::tc_commit(&a_empty[sa]);
+                        if (b_done) ptx::tc_commit(&b_empty[sb]);
+                    }
+                    __syncwarp();
+                }
+                if (++sa == A_SLOTS) { sa = 0; pa ^= 1; }
+                if (b_done && ++sb == B_STAGES) { sb = 0; pb ^= 1; }
+            }
+        }
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(a.status, 5); }
+    } else if (warp >= R_CONV0 && warp < R_EPI0) {
+        // ------------------------------------------------ converters: nibbles -> exact 16-bit w - zero_point
+        // Warp (q = warp % 4, r): TMEM lanes 32q .. 32q+31, the stages of parity r.  Lane (g, tq) owns the
+        // columns 32q + 4g .. +3 (two bytes of a row) and, per k16 step, the k-rows 2tq, 2tq+1, 2tq+8, 2tq+9.
+        // Byte h, low nibble goes to TMEM lane 32q + 16h + g, the high one to 32q + 16h + 8 + g.
+        const int q = warp & 3, r = (warp - R_CONV0) >> 2;
+        const int g = lane >> 2, tq = lane & 3;
+        uint32_t off[4]; // 64-byte rows, 64B swizzle: 16-byte chunk index XOR ((row >> 1) & 3)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t row = 2 * tq + (i & 1) + 8 * (i >> 1);
+            off[i] = row * 64 + (((uint32_t)q ^ ((row >> 1) & 3)) << 4) + 2 * g;
+        }
+        const uint32_t magic = F16 ? (p.sgn4 ? 0x64086408u : 0x64006400u) : (p.sgn4 ? 0x43084308u : 0x43004300u);
+        const uint32_t magic_hi = p.sgn4 ? 0x64806480u : 0x64006400u; // f16, nibble in place: 1024 + 16 u
+        const int base_off = p.sgn4 ? 8 : 0;
+        const int zt = p.zp_mode == 2 ? load_int(a.wei_zp.dt, a.wei_zp.ptr, 0) : 0;
+        constexpr int NZ = MULTI ? 4 : 1;
+        // offsets of the four columns, as packed pairs: what the packed subtraction (or the f16 fma) takes
+        uint32_t o2[4];
+        auto set_offsets = [&](uint32_t raw) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int z = base_off + (p.zp_mode == 1 ? zp_of(a.wei_zp.dt, raw, c) : zt);
+                uint32_t b;
+                if (F16) b = __half_as_ushort(__int2half_rn((c & 1) ? -(64 + z) : 1024 + z));
+                else b = __bfloat16_as_ushort(__float2bfloat16_rn((float)(128 + z)));
+                o2[c] = b * 0x10001u;
+            }
+        };
+        set_offsets(0u);
+        uint32_t it = 0;
+        int s = 0, sa = 0;
+        uint32_t ph = 0, pa = 1;
+        bool ok = true;
+        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+            const int64_t n = (int64_t)(t / p.num_m_tiles) * RT_N + 32 * q + 4 * g;
+            // zero-points of this warp's next two stages, loaded ahead (a load takes longer than a stage)
+            uint32_t z0[NZ], z1[NZ], zz[NZ];
+            auto fetch = [&](int st, uint32_t (&z)[NZ]) {
+#pragma unroll
+                for (int j = 0; j < NZ; ++j) {
+                    z[j] = 0u;
+                    if (p.zp_mode == 1 && 4 * st + j < p.ksteps) z[j] = load_zp4(a, (4 * st + j) / p.group_steps, n);
+                }
+            };
+            const int first = (int)((it & 1) == (uint32_t)r ? 0 : 1);
+            fetch(first, z0);
+            fetch(first + 2, z1);
+            for (int st = 0; st < p.kstages; ++st, ++it) {
+                if ((int)(it & 1) == r) {
+#pragma unroll
+                    for (int j = 0; j < NZ; ++j) { zz[j] = z0[j]; z0[j] = z1[j]; }
+                    fetch(st + 4, z1);
+                    if (!warp_wait(&w_full[s], ph)) { ok = false; break; }
+                    const uint8_t *raw = smem + R_W_OFFSET + s * W_BYTES;
+                    uint32_t w[4][4]; // [step][k-row], two bytes each
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) w[k][i] = *reinterpret_cast<const unsigned short *>(raw + k * 1024 + off[i]);
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(&w_empty[s]);
+                    if (!MULTI && p.zp_mode == 1) set_offsets(zz[0]);
+                    uint32_t o[2][16];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (MULTI && p.zp_mode == 1) set_offsets(zz[MULTI ? k : 0]);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint32_t sel = h ? 0x5511u : 0x4400u; // byte h of both rows
+                            const uint32_t x01 = perm(w[k][0], w[k][1], sel), x23 = perm(w[k][2], w[k][3], sel);
+                            if (F16) {
+                                o[h][4 * k + 0] = sub_f16x2(and_xor(x01, 0x000F000Fu, magic), o2[2 * h]);
+                                o[h][4 * k + 1] = fma_f16x2(and_xor(x01, 0x00F000F0u, magic_hi), 0x2C002C00u, o2[2 * h + 1]);
+                                o[h][4 * k + 2] = sub_f16x2(and_xor(x23, 0x000F000Fu, magic), o2[2 * h]);
+                                o[h][4 * k + 3] = fma_f16x2(and_xor(x23, 0x00F000F0u, magic_hi), 0x2C002C00u, o2[2 * h + 1]);
+                            } else {
+                                o[h][4 * k + 0] = sub_bf16x2(and_xor(x01, 0x000F000Fu, magic), o2[2 * h]);
+                                o[h][4 * k + 1] = sub_bf16x2(and_xor(x01 >> 4, 0x000F000Fu, magic), o2[2 * h + 1]);
+                                o[h][4 * k + 2] = sub_bf16x2(and_xor(x23, 0x000F000Fu, magic), o2[2 * h]);
+                                o[h][4 * k + 3] = sub_bf16x2(and_xor(x23 >> 4, 0x000F000Fu, magic), o2[2 * h + 1]);
+                            }
+                        }
+                    }
+                    if (!warp_wait(&a_empty[sa], pa)) { ok = false; break; }
+                    ptx::tc_fence_after_sync();
+                    const uint32_t slot = tmem_base + ((uint32_t)(32 * q) << 16) + R_A_COL0 + sa * A_SLOT_COLS;
+                    st_16x128b_x8(slot, o[0]);
+                    st_16x128b_x8(slot + (16u << 16), o[1]);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    ptx::tc_fence_before_sync();
+                    __syncwarp(); // every lane's stores to tensor memory are done
+                    if (lane == 0) ptx::mbar_arrive(&a_full[sa]);
+                }
+                if (++s == W_STAGES) { s = 0; ph ^= 1; }
+                if (++sa == A_SLOTS) { sa = 0; pa ^= 1; }
+            }
+        }
+        if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
+    } else if (warp >= R_EPI0) {
+        // ------------------------------------------------ epilogue: tot += scale * group sum, then the store
+        const int q = warp & 3, h = (warp - R_EPI0) >> 2;
+        const int chunks = p.tile_rows / 16; // 16-row pieces of a tile: the first half of them to h = 0
+        const int c0 = h ? (chunks + 1) / 2 : 0, cn = h ? chunks / 2 : (chunks + 1) / 2;
+        const int col = 32 * q + 4 * (lane & 7) + 2 * (lane >> 4) + ((lane >> 3) & 1);
+        const int groups = (p.ksteps + p.group_steps - 1) / p.group_steps;
+        float ssc = 1.f;
+        if (a.src_scale.ptr) ssc = load_float(a.src_scale.dt, a.src_scale.ptr, 0);
+        else if (a.src_scale.on_host) ssc = a.src_scale.host_value;
+        int buf = 0;
+        uint32_t pacc = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+            const int64_t n = (int64_t)(t / p.num_m_tiles) * RT_N + col;
+            const int m0 = (t % p.num_m_tiles) * p.tile_rows;
+            float tot[4][16];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) tot[c][j] = 0.f;
+            auto scale_at = [&](int g) {
+                if (g >= groups || n >= a.N) return 0.f;
+                return load_float(a.wei_scale.dt, a.wei_scale.ptr, ((a.wei_scale.mask & 1) ? (int64_t)g * a.wei_scale.ld : 0) + n);
+            };
+            float nx[4]; // scales of the next groups, loaded ahead
+#pragma unroll
+            for (int i = 0; i < 4; ++i) nx[i] = scale_at(i);
+            for (int g = 0; g < groups && ok; ++g) {
+                const float sc = nx[0];
+                nx[0] = nx[1]; nx[1] = nx[2]; nx[2] = nx[3];
+                nx[3] = scale_at(g + 4);
+                if (!warp_wait(&acc_full[buf], pacc)) { ok = false; break; }
+                ptx::tc_fence_after_sync();
+                const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + buf * RT_M + c0 * 16;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c < cn) {
+                        uint32_t v[16];
+                        ld_32x16(acc + 16 * c, v);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) tot[c][j] = fmaf(sc, __uint_as_float(v[j]), tot[c][j]);
+                    }
+                }
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&acc_empty[buf]);
+                if (++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
+            }
+            if (!ok) break;
+            if (n < a.N) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c >= cn) continue;
+                    const int64_t mc = m0 + (c0 + c) * 16;
+                    const int rows = (int)min((int64_t)16, min((int64_t)m0 + p.tile_rows, a.M) - mc);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (j >= rows) continue;
+                        const int64_t m = mc + j;
+                        float d = tot[c][j] * ssc;
+                        if (a.bias) d = __fadd_rn(d, load_float(a.bias_dt, a.bias, m * a.bias_sm + n * a.bias_sn));
+                        if (p.fast_store) {
+                            const int64_t o = m * a.dst_sm + n * a.dst_sn;
+                            if (a.dst_dt == DT_BF16) ((unsigned short *)a.dst)[o] = f32_to_bf16_bits(d);
+                            else if (a.dst_dt == DT_F16) ((__half *)a.dst)[o] = __float2half_rn(d);
+                            else ((float *)a.dst)[o] = d;
+                        } else {
+                            finish_store_general(a, d, m, n);
+                        }
+                    }
+                }
+            }
+        }
+        if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
+    }
+
+    // ---------------------------------------------------- teardown
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 3) {
+        __syncwarp();
+        ptx::tc_fence_after_sync();
+        ptx::tmem_dealloc(tmem_base, 512);
+    }
+}
+
+typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+        const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+        CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+encode_tiled_fn rows_get_encode() {
+    static encode_tiled_fn fn = nullptr;
+    if (!fn) {
+        void *ptr = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess
+                && q == cudaDriverEntryPointSuccess)
+            fn = (encode_tiled_fn)ptr;
+    }
+    return fn;
+}
+
+template <bool F16, bool MULTI>
+int rows_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a, const RowsParams &p, int sm_count,
+        cudaStream_t st) {
+    auto kern = woq_rows_kernel<F16, MULTI>;
+    static std::atomic<unsigned long long> configured;
+    if (!opt_in_dynamic_smem(kern, R_SMEM_BYTES, configured)) return 5;
+    kern<<<p.num_tiles < sm_count ? p.num_tiles : sm_count, R_THREADS, R_SMEM_BYTES, st>>>(tw, ts, a, p);
+    count_launch();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        set_last_error(std::string("cuda:tcgen05:woq4_rows launch: ") + cudaGetErrorString(e));
+        return 5;
+    }
+    return 0;
+}
+
+} // namespace
+
+// TMA bases on 16 bytes; a lane reads the zero-points of four columns at once
+bool woq_rows_pointers_ok(const MatmulArgs &a) {
+    return (uintptr_t)a.wei % 16 == 0 && (uintptr_t)a.src % 16 == 0 && (uintptr_t)a.wei_zp.ptr % 4 == 0;
+}
+
+int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st) {
+    if (a.M == 0 || a.N == 0) return 0;
+    encode_tiled_fn enc = rows_get_encode();
+    if (!enc) return 5;
+    if (sm_count < 1) sm_count = 148;
+    RowsParams p {};
+    // as few row tiles as cover M, of equal size
+    p.num_m_tiles = (int)((a.M + RT_M - 1) / RT_M);
+    p.tile_rows = (int)(((a.M + p.num_m_tiles - 1) / p.num_m_tiles + 15) / 16 * 16);
+    const int64_t tiles = (int64_t)p.num_m_tiles * ((a.N + RT_N - 1) / RT_N);
+    if (tiles >= (1LL << 31)) return 3;
+    p.num_tiles = (int)tiles;
+    CUtensorMap tw, ts;
+    {
+        cuuint64_t dims[2] = {(cuuint64_t)(a.N / 2), (cuuint64_t)a.K};
+        cuuint64_t strides[1] = {(cuuint64_t)(a.wei_sk / 2)};
+        cuuint32_t box[2] = {RT_N / 2, RK};
+        cuuint32_t estr[2] = {1, 1};
+        if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(a.wei), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+                != CUDA_SUCCESS)
+            return 5;
+    }
+    {
+        cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M};
+        cuuint64_t strides[1] = {(cuuint64_t)(a.src_sm * 2)};
+        cuuint32_t box[2] = {RK, (cuuint32_t)p.tile_rows};
+        cuuint32_t estr[2] = {1, 1};
+        if (enc(&ts, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(a.src), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+                != CUDA_SUCCESS)
+            return 5;
+    }
+    p.ksteps = (int)(a.K / 16);
+    p.kstages = (int)((a.K + RK - 1) / RK);
+    const int64_t group = (a.wei_scale.ptr && (a.wei_scale.mask & 1)) ? a.wei_scale.g0
+            : (a.wei_zp.ptr && (a.wei_zp.mask & 1))                    ? a.wei_zp.g0
+                                                                       : a.K;
+    p.group_steps = (int)(group / 16);
+    if (p.group_steps < 1 || p.group_steps > p.ksteps) p.group_steps = p.ksteps;
+    p.sgn4 = a.wei_dt == DT_S4;
+    p.zp_mode = !a.wei_zp.ptr ? 0 : (a.wei_zp.mask ? 1 : 2);
+    p.fast_store = a.n_po == 0 && !a.dst_scale.ptr && !a.dst_scale.on_host
+            && (a.dst_dt == DT_F32 || a.dst_dt == DT_BF16 || a.dst_dt == DT_F16);
+    const bool f16 = a.src_dt == DT_F16;
+    const uint32_t fmt = f16 ? ptx::FMT_F16 : ptx::FMT_BF16;
+    p.idesc = ptx::make_idesc(ptx::CFMT_F32, fmt, fmt, false, false, RT_N, (uint32_t)p.tile_rows);
+    const bool multi = p.group_steps % 4 != 0 && p.zp_mode == 1;
+    if (f16) return multi ? rows_launch<true, true>(tw, ts, a, p, sm_count, st) : rows_launch<true, false>(tw, ts, a, p, sm_count, st);
+    return multi ? rows_launch<false, true>(tw, ts, a, p, sm_count, st) : rows_launch<false, false>(tw, ts, a, p, sm_count, st);
+}
+
+} // namespace qmm

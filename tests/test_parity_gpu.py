@@ -168,6 +168,36 @@ def test_woq_decode_matches_oracle(gpu, name, kernel):
     assert np.array_equal(got, got2)
 
 
+WOQ_ROWS_CASES = {
+    "m33_one_tile": lambda: W.int4_decode(33, 256, 128),
+    "m129_two_tiles": lambda: W.int4_decode(129, 512, 288),
+    "m300_n_tail": lambda: W.int4_decode(300, 512, 352, group=64),
+    "group16_several_per_stage": lambda: W.int4_decode(40, 272, 160, group=16, zp_dt=W.S4),
+    "group48_across_stages": lambda: W.int4_decode(100, 1104, 256, group=48),
+    "group32_k_tail_stage": lambda: W.int4_decode(64, 416, 256, group=32, wei_dt=W.U4),
+    "f16_u4": lambda: W.int4_decode(77, 512, 256, group=32, wei_dt=W.U4, src_dt=W.F16, dst_dt=W.F16),
+    "f16_s4_u8zp": lambda: W.int4_decode(65, 384, 256, zp_dt=W.U8, src_dt=W.F16, dst_dt=W.F16),
+    "no_zp_f32_dst": lambda: W.int4_decode(50, 256, 160, with_zp=False, dst_dt=W.F32),
+    "per_n_scale": lambda: _per_n_scale(W.int4_decode(36, 384, 256)),
+    "bias_relu": lambda: _with_bias_relu(W.int4_decode(48, 512, 256)),
+    "more_tiles_than_sms": lambda: W.int4_decode(140, 192, 9632, group=64),
+}
+
+
+@pytest.mark.parametrize("name", sorted(WOQ_ROWS_CASES))
+def test_woq_rows_matches_oracle(gpu, name):
+    """int4 decompression for more than 32 rows: edges of row tiles, of column tiles and of K stages, groups
+    smaller and larger than a stage, both source types (the operand is exact, sums differ by f32 order)."""
+    eng, strm = gpu
+    p = WOQ_ROWS_CASES[name]()
+    want = O.run_port(p)
+    got, impl = run_problem(p, eng, strm)
+    assert impl == "cuda:tcgen05:woq4_rows"
+    assert_parity(got, want, p.dst_dt, name, slack_for(p, impl))
+    got2, _ = run_problem(p, eng, strm)
+    assert np.array_equal(got, got2)
+
+
 GROUPED_TC_CASES = {
     "small": lambda: W.moe_grouped(96, 256, 128, 8),
     "empty_groups": lambda: W.moe_grouped(40, 128, 64, 6, sizes=[0, 17, 0, 3, 20, 0]),
