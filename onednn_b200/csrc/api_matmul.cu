@@ -433,7 +433,7 @@ dnnl_status_t woq_accepts(const dnnl_primitive_desc &pd) {
 // in the src's type - bf16 holds every integer up to 256, w - zp with 4-bit zero-points; f16 up to 2048
 dnnl_status_t woq_rows_accepts(const dnnl_primitive_desc &pd) {
     if (woq4_accepts(pd) != dnnl_success) return dnnl_unimplemented;
-    UNIMPL_IF(pd.M() <= 32 || pd.M() >= (1LL << 31) || pd.src.strides[0] % 8 != 0 || pd.src.strides[0] < pd.K());
+    UNIMPL_IF(pd.M() <= 32 || pd.M() >= (1LL << 31) || pd.N() >= (1LL << 29) || pd.src.strides[0] % 8 != 0 || pd.src.strides[0] < pd.K());
     const auto &wz = pd.attr.zp(DNNL_ARG_WEIGHTS);
     if (wz.set)
         UNIMPL_IF(!one_of(wz.dt, {dnnl_s4, dnnl_u4}) && !(pd.src.data_type == dnnl_f16 && one_of(wz.dt, {dnnl_s8, dnnl_u8})));

@@ -12,17 +12,19 @@
 //
 // As in the other decompression kernels the weights are the A operand, in TENSOR MEMORY (128 dst columns = TMEM
 // lanes), and the src rows the B operand from shared memory, so an epilogue lane owns one dst column.  A tile is
-// 128 columns x up to 128 rows: an MMA of up to 128 rows takes about 64 cycles to execute and about as many to
-// issue, so narrower tiles would be paid in issue slots and wider ones would not leave tensor memory for three
-// accumulators (a group of 32 k is two MMAs: with three buffers the fold of one group overlaps the next two).
-// Per-stage (64 k) cost at 128 rows: 4 MMAs = 256 tensor cycles, about 100 converter instructions per warp with
-// two warps per lane quarter, and 64 FMAs per epilogue lane and group.
+// 128 columns x up to 128 rows (two accumulators of 128 columns and four operand slots of 64 fill the 512).
 //
-// Roles (20 warps): 0 weight tiles by TMA (ring of 4 KB nibble tiles), 1 src tiles by TMA (ring of 128-k tiles:
-// one release per two stages), 2 issues all MMAs, 4-11 converters (two per lane quarter, alternating
-// stages), 12-19 epilogue (two per lane quarter, each half of the rows).  Every mbarrier wait is bounded.
+// What bounds the kernel is the chain of dependent instructions of each role, not a pipe: a satisfied barrier
+// wait costs 150 to 300 cycles, the conversion of a warp's share of a 128-k stage about 1500, the fold of 32 rows
+// by an epilogue warp about 750, while one thread issues the eight MMAs of a stage in 100.  Hence stages of 128 k
+// with one barrier for operand and src tile together, 16 epilogue warps with 32 rows each, and loads of scales
+// and zero-points issued groups ahead.
 //
-// Measured on a B200 at K = N = 4096, M = 300, groups of 128, u4 zero-points: 66 us a call; the generic kernel,
+// Roles (28 warps): 0 weight tiles by TMA, 1 src tiles by TMA, 2 issues all MMAs, 4-11 converters (two per lane
+// quarter, taking the stages in turn), 12-27 epilogue (four per lane quarter, each a quarter of the rows).  Every mbarrier wait is bounded.
+//
+// Measured on a B200 at K = N = 4096, M = 300, groups of 128, u4 zero-points: 43 us a call (66 us with 64-k stages,
+// a warp-wide issuing loop and eight epilogue warps); the generic kernel,
 // which such calls took before, 54.3 ms.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -41,18 +43,22 @@ namespace {
 
 constexpr int RT_N = 128; // dst columns per tile = TMEM lanes
 constexpr int RT_M = 128; // most src rows per tile
-constexpr int RK = 64; // k per operand stage
-constexpr int RKB = 2 * RK; // k per src stage: two 128-byte swizzle rows of 16-bit values
-constexpr int W_STAGES = 12, A_SLOTS = 4, B_STAGES = 4, ACC_BUFS = 3;
+constexpr int RK = 128; // k per stage: eight MMAs share one pair of hand-offs
+constexpr int W_STAGES = 10; // nibble tiles (from HBM)
+constexpr int STAGES = 4; // operand slots in tensor memory and src tiles, used and released together
+constexpr int ACC_BUFS = 2;
 constexpr int W_BYTES = RK * RT_N / 2; // nibbles as loaded: 64-byte rows
-constexpr int B_BYTES = RT_M * RKB * 2;
-constexpr int R_CONV_WARPS = 8, R_EPI_WARPS = 8;
+constexpr int B_BYTES = RT_M * RK * 2; // src rows: two boxes of 64 k
+constexpr int CONV_SETS = 2; // sets of four converter warps, which take the stages in turn
+constexpr int R_CONV_WARPS = 4 * CONV_SETS, R_EPI_WARPS = 16;
+constexpr int EPI_PIECES = RT_M / 16 / (R_EPI_WARPS / 4); // 16-row pieces of the accumulator per epilogue warp
 constexpr int R_CONV0 = 4, R_EPI0 = R_CONV0 + R_CONV_WARPS;
 constexpr int R_THREADS = 32 * (R_EPI0 + R_EPI_WARPS);
+constexpr int SPS = RK / 16; // k16 steps per stage
 constexpr int A_SLOT_COLS = RK / 2;
 constexpr int R_A_COL0 = ACC_BUFS * RT_M;
-static_assert(R_A_COL0 + A_SLOTS * A_SLOT_COLS <= 512, "tensor memory");
-constexpr int R_B_OFFSET = 0, R_W_OFFSET = B_STAGES * B_BYTES;
+static_assert(R_A_COL0 + STAGES * A_SLOT_COLS <= 512, "tensor memory");
+constexpr int R_B_OFFSET = 0, R_W_OFFSET = STAGES * B_BYTES;
 constexpr int R_BAR_OFFSET = R_W_OFFSET + W_STAGES * W_BYTES;
 constexpr int R_SMEM_BYTES = R_BAR_OFFSET + 512 + 1024;
 static_assert(R_SMEM_BYTES <= 227 * 1024, "shared memory");
@@ -61,7 +67,7 @@ struct RowsParams {
     int num_m_tiles, num_tiles;
     int tile_rows; // a multiple of 16, at most RT_M: the MMAs' N and the rows of a src box
     int ksteps; // K / 16
-    int kstages; // ceil(K / 64)
+    int kstages; // ceil(K / 128)
     int group_steps; // k16 steps per quantization group (ksteps when not grouped along K)
     int sgn4; // weights are s4 (else u4)
     int zp_mode; // 0 none, 1 per (group, column), 2 per tensor
@@ -118,20 +124,48 @@ __device__ __forceinline__ void mma_ts_16bit(uint32_t tmem_d, uint32_t tmem_a, u
             "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"((uint32_t)acc)
             : "memory");
 }
-// post-ops, dst scale, any dst type: rare and large, out of line
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+// two fused multiply-adds: d = sc * {v0, v1} + d
+__device__ __forceinline__ void fma_f32x2(uint64_t &d, uint64_t sc, uint32_t v0, uint32_t v1) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(sc), "l"(pack2(v0, v1)));
+}
+// bias, post-ops, dst scale, any dst type: rare and large, out of line
 __device__ __noinline__ void finish_store_general(const MatmulArgs &a, float d, int64_t m, int64_t n) {
+    if (a.bias) d = __fadd_rn(d, load_float(a.bias_dt, a.bias, m * a.bias_sm + n * a.bias_sn));
     finish_store(a, d, m, n, false);
+}
+// A kernel parameter held in a register.  Read where they are used, parameters come from a constant cache
+// that five roles with their own corners of a 3 KB parameter block keep missing (hundreds of cycles a miss).
+__device__ __forceinline__ int in_reg(int v) {
+    asm volatile("" : "+r"(v));
+    return v;
 }
 __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
     return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity));
 }
 
+// Loads that must be issued where they stand, well before their use: the compiler is free to move an
+// ordinary one down to it.
+__device__ __forceinline__ uint32_t ld_early_u32(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_early_u16(const unsigned short *p) {
+    unsigned short v;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
 // The zero-points of a lane's four columns (n .. n + 3) in group g, as loaded: four nibbles or four bytes
 __device__ __forceinline__ uint32_t load_zp4(const MatmulArgs &a, int g, int64_t n) {
     if (n >= a.N) return 0u;
     const int64_t e = (int64_t)g * a.wei_zp.ld + n;
-    if (a.wei_zp.dt == DT_U4 || a.wei_zp.dt == DT_S4) return __ldg((const unsigned short *)a.wei_zp.ptr + (e >> 2));
-    return __ldg((const unsigned *)a.wei_zp.ptr + (e >> 2));
+    if (a.wei_zp.dt == DT_U4 || a.wei_zp.dt == DT_S4) return ld_early_u16((const unsigned short *)a.wei_zp.ptr + (e >> 2));
+    return ld_early_u32((const uint32_t *)a.wei_zp.ptr + (e >> 2));
 }
 __device__ __forceinline__ int zp_of(int dt, uint32_t raw, int i) {
     if (dt == DT_U4 || dt == DT_S4) {
@@ -142,7 +176,7 @@ __device__ __forceinline__ int zp_of(int dt, uint32_t raw, int i) {
     return dt == DT_S8 ? (int)(signed char)v : v;
 }
 
-// MULTI: a 64-k stage may touch several groups (group size not a multiple of 64): the offsets are looked up
+// MULTI: a 128-k stage may touch several groups (group size not a multiple of 128): the offsets are looked up
 // per k16 step instead of per stage.
 template <bool F16, bool MULTI>
 __global__ void __launch_bounds__(R_THREADS, 1)
@@ -152,11 +186,9 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *w_full = (uint64_t *)(smem + R_BAR_OFFSET);
     uint64_t *w_empty = w_full + W_STAGES;
-    uint64_t *b_full = w_empty + W_STAGES;
-    uint64_t *b_empty = b_full + B_STAGES;
-    uint64_t *a_full = b_empty + B_STAGES;
-    uint64_t *a_empty = a_full + A_SLOTS;
-    uint64_t *acc_full = a_empty + A_SLOTS;
+    uint64_t *ab_full = w_empty + W_STAGES; // src tile and operand slot of a stage
+    uint64_t *ab_empty = ab_full + STAGES;
+    uint64_t *acc_full = ab_empty + STAGES;
     uint64_t *acc_empty = acc_full + ACC_BUFS;
     uint32_t *tmem_slot = (uint32_t *)(acc_empty + ACC_BUFS);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
@@ -165,15 +197,11 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     if (threadIdx.x == 0) {
         for (int s = 0; s < W_STAGES; ++s) {
             ptx::mbar_init(&w_full[s], 1);
-            ptx::mbar_init(&w_empty[s], R_CONV_WARPS / 2); // the stage's four converter warps
+            ptx::mbar_init(&w_empty[s], 4); // the stage's four converter warps
         }
-        for (int s = 0; s < B_STAGES; ++s) {
-            ptx::mbar_init(&b_full[s], 1);
-            ptx::mbar_init(&b_empty[s], 1);
-        }
-        for (int s = 0; s < A_SLOTS; ++s) {
-            ptx::mbar_init(&a_full[s], R_CONV_WARPS / 2);
-            ptx::mbar_init(&a_empty[s], 1);
+        for (int s = 0; s < STAGES; ++s) {
+            ptx::mbar_init(&ab_full[s], 1 + 4); // the src tile's producer, the stage's converters
+            ptx::mbar_init(&ab_empty[s], 1);
         }
         for (int s = 0; s < ACC_BUFS; ++s) {
             ptx::mbar_init(&acc_full[s], 1);
@@ -190,109 +218,104 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
+    // The three single-thread roles: one elected thread runs the whole loop.  A role's time per stage is its
+    // chain of dependent instructions (about five cycles each), so these loops are kept short.
     if (warp == 0) {
         // ------------------------------------------------ TMA producer of the nibble tiles
-        int s = 0;
-        uint32_t ph = 1;
-        bool ok = true;
-        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
-            const int x = (t / p.num_m_tiles) * (RT_N / 2);
-            for (int st = 0; st < p.kstages; ++st) {
-                if (!warp_wait(&w_empty[s], ph)) { ok = false; break; }
-                if (ptx::elect_one()) {
+        if (ptx::elect_one()) {
+            const int kstages = in_reg(p.kstages);
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+                const int x = (t / p.num_m_tiles) * (RT_N / 2);
+                for (int st = 0; st < kstages; ++st) {
+                    if (!ptx::mbar_wait(&w_empty[s], ph)) { ok = false; break; }
                     ptx::mbar_arrive_expect_tx(&w_full[s], W_BYTES);
                     ptx::tma_load_2d(smem + R_W_OFFSET + s * W_BYTES, &tmW, &w_full[s], x, st * RK);
+                    if (++s == W_STAGES) { s = 0; ph ^= 1; }
                 }
-                __syncwarp();
-                if (++s == W_STAGES) { s = 0; ph ^= 1; }
             }
+            if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
-        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp == 1) {
-        // ------------------------------------------------ TMA producer of the src tiles (128 k each)
-        int s = 0;
-        uint32_t ph = 1;
-        bool ok = true;
-        const uint32_t half = (uint32_t)p.tile_rows * 128;
-        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
-            const int m0 = (t % p.num_m_tiles) * p.tile_rows;
-            for (int st = 0; st < p.kstages; st += 2) {
-                if (!warp_wait(&b_empty[s], ph)) { ok = false; break; }
-                uint8_t *d = smem + R_B_OFFSET + s * B_BYTES;
-                if (ptx::elect_one()) {
-                    const bool two = st + 1 < p.kstages;
-                    ptx::mbar_arrive_expect_tx(&b_full[s], two ? 2 * half : half);
-                    ptx::tma_load_2d(d, &tmS, &b_full[s], st * RK, m0);
-                    if (two) ptx::tma_load_2d(d + B_BYTES / 2, &tmS, &b_full[s], (st + 1) * RK, m0);
+        // ------------------------------------------------ TMA producer of the src tiles
+        if (ptx::elect_one()) {
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            const int kstages = in_reg(p.kstages);
+            const uint32_t bytes = (uint32_t)in_reg(p.tile_rows * RK * 2);
+            for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+                const int m0 = (t % p.num_m_tiles) * p.tile_rows;
+                for (int st = 0; st < kstages; ++st) {
+                    if (!ptx::mbar_wait(&ab_empty[s], ph)) { ok = false; break; }
+                    uint8_t *d = smem + R_B_OFFSET + s * B_BYTES;
+                    ptx::mbar_arrive_expect_tx(&ab_full[s], bytes); // (k beyond K reads as zeros and counts)
+                    ptx::tma_load_2d(d, &tmS, &ab_full[s], st * RK, m0);
+                    ptx::tma_load_2d(d + B_BYTES / 2, &tmS, &ab_full[s], st * RK + RK / 2, m0);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                __syncwarp();
-                if (++s == B_STAGES) { s = 0; ph ^= 1; }
             }
+            if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
-        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp == 2) {
         // ------------------------------------------------ MMA issuer
-        int sa = 0, sb = 0, buf = 0;
-        uint32_t pa = 0, pb = 0, pacc = 1;
-        bool ok = true;
-        for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
-            int left = 0; // k16 steps left in the open group (0: none open)
-            for (int st = 0; st < p.kstages; ++st) {
-                if ((st & 1) == 0 && !warp_wait(&b_full[sb], pb)) { ok = false; break; }
-                if (!warp_wait(&a_full[sa], pa)) { ok = false; break; }
-                ptx::tc_fence_after_sync();
-                const uint64_t bd = ptx::smem_desc_sw128(
-                        ptx::smem_u32(smem + R_B_OFFSET + sb * B_BYTES + (st & 1) * (B_BYTES / 2)), 0, 1024);
-                const uint32_t ta = tmem_base + R_A_COL0 + sa * A_SLOT_COLS;
-                const int nst = min(4, p.ksteps - 4 * st);
-                const bool b_done = (st & 1) || st + 1 == p.kstages;
-                if (nst == 4 && (left >= 4 || (left == 0 && p.group_steps >= 4))) {
-                    // the common stage, whole and inside one group: straight-line code
-                    const bool fresh = left == 0;
-                    if (fresh) {
-                        if (!warp_wait(&acc_empty[buf], pacc)) { ok = false; break; }
-                        ptx::tc_fence_after_sync();
-                        left = min(p.group_steps, p.ksteps - 4 * st);
-                    }
-                    left -= 4;
-                    const uint32_t d = tmem_base + buf * RT_M;
-                    if (ptx::elect_one()) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) mma_ts_16bit(d, ta + 8 * q, bd + 2 * q, p.idesc, q > 0 || !fresh);
-                        if (left == 0) ptx::tc_commit(&acc_full[buf]);
-                        ptx::tc_commit(&a_empty[sa]);
-                        if (b_done) ptx::tc_commit(&b_empty[sb]);
-                    }
-                    __syncwarp();
-                    if (left == 0 && ++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
-                } else {
-                    for (int q = 0; q < nst; ++q) {
+        if (ptx::elect_one()) {
+            const int kstages = in_reg(p.kstages), ksteps = in_reg(p.ksteps), group_steps = in_reg(p.group_steps);
+            const uint32_t idesc = (uint32_t)in_reg((int)p.idesc);
+            int s = 0, buf = 0;
+            uint32_t ph = 0, pacc = 1;
+            bool ok = true;
+            for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
+                int left = 0; // k16 steps left in the open group (0: none open)
+                int todo = ksteps;
+                for (int st = 0; st < kstages && ok; ++st) {
+                    if (!ptx::mbar_wait(&ab_full[s], ph)) { ok = false; break; }
+                    ptx::tc_fence_after_sync();
+                    const uint64_t bd = ptx::smem_desc_sw128(ptx::smem_u32(smem + R_B_OFFSET + s * B_BYTES), 0, 1024);
+                    const uint32_t ta = tmem_base + R_A_COL0 + s * A_SLOT_COLS;
+                    if (todo >= SPS && (left >= SPS || (left == 0 && group_steps >= SPS))) {
+                        // the common stage, whole and inside one group: straight-line code
                         const bool fresh = left == 0;
                         if (fresh) {
-                            if (!warp_wait(&acc_empty[buf], pacc)) { ok = false; break; }
+                            if (!ptx::mbar_wait(&acc_empty[buf], pacc)) { ok = false; break; }
                             ptx::tc_fence_after_sync();
-                            left = min(p.group_steps, p.ksteps - (4 * st + q));
+                            left = min(group_steps, todo);
                         }
-                        --left;
-                        if (ptx::elect_one()) {
-                            mma_ts_16bit(tmem_base + buf * RT_M, ta + 8 * q, bd + 2 * q, p.idesc, !fresh);
-                            if (left == 0) ptx::tc_commit(&acc_full[buf]);
+                        const uint32_t d = tmem_base + buf * RT_M;
+#pragma unroll
+                        for (int q = 0; q < SPS; ++q)
+                            mma_ts_16bit(d, ta + 8 * q, bd + (uint64_t)((q >> 2) * (B_BYTES / 2 >> 4) + (q & 3) * 2), idesc, q > 0 || !fresh);
+                        left -= SPS;
+                        if (left == 0) {
+                            ptx::tc_commit(&acc_full[buf]);
+                            if (++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
                         }
-                        __syncwarp();
-                        if (left == 0 && ++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
+                    } else {
+                        const int nst = min(SPS, todo);
+                        for (int q = 0; q < nst; ++q) {
+                            const bool fresh = left == 0;
+                            if (fresh) {
+                                if (!ptx::mbar_wait(&acc_empty[buf], pacc)) { ok = false; break; }
+                                ptx::tc_fence_after_sync();
+                                left = min(group_steps, todo - q);
+                            }
+                            mma_ts_16bit(tmem_base + buf * RT_M, ta + 8 * q,
+                                    bd + (uint64_t)((q >> 2) * (B_BYTES / 2 >> 4) + (q & 3) * 2), idesc, !fresh);
+                            if (--left == 0) {
+                                ptx::tc_commit(&acc_full[buf]);
+                                if (++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
+                            }
+                        }
                     }
-                    if (!ok) break;
-                    if (ptx::elect_one()) {
-                        ptx::tc_commit(&a_empty[sa]);
-                        if (b_done) ptx::tc_commit(&b_empty[sb]);
-                    }
-                    __syncwarp();
+                    todo -= SPS;
+                    ptx::tc_commit(&ab_empty[s]); // src tile and operand slot are free once these MMAs have read them
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                if (++sa == A_SLOTS) { sa = 0; pa ^= 1; }
-                if (b_done && ++sb == B_STAGES) { sb = 0; pb ^= 1; }
             }
+            if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
-        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp >= R_CONV0 && warp < R_EPI0) {
         // ------------------------------------------------ converters: nibbles -> exact 16-bit w - zero_point
         // Warp (q = warp % 4, r): TMEM lanes 32q .. 32q+31, the stages of parity r.  Lane (g, tq) owns the
@@ -306,100 +329,140 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
             const uint32_t row = 2 * tq + (i & 1) + 8 * (i >> 1);
             off[i] = row * 64 + (((uint32_t)q ^ ((row >> 1) & 3)) << 4) + 2 * g;
         }
-        const uint32_t magic = F16 ? (p.sgn4 ? 0x64086408u : 0x64006400u) : (p.sgn4 ? 0x43084308u : 0x43004300u);
-        const uint32_t magic_hi = p.sgn4 ? 0x64806480u : 0x64006400u; // f16, nibble in place: 1024 + 16 u
-        const int base_off = p.sgn4 ? 8 : 0;
-        const int zt = p.zp_mode == 2 ? load_int(a.wei_zp.dt, a.wei_zp.ptr, 0) : 0;
-        constexpr int NZ = MULTI ? 4 : 1;
+        const int kstages = in_reg(p.kstages), ksteps = in_reg(p.ksteps), group_steps = in_reg(p.group_steps);
+        const int zp_mode = in_reg(p.zp_mode), zp_dt = in_reg(a.wei_zp.dt);
+        const uint32_t magic = (uint32_t)in_reg(F16 ? (p.sgn4 ? 0x64086408 : 0x64006400) : (p.sgn4 ? 0x43084308 : 0x43004300));
+        const uint32_t magic_hi = (uint32_t)in_reg(p.sgn4 ? 0x64806480 : 0x64006400); // f16, nibble in place: 1024 + 16 u
+        const int base_off = in_reg(p.sgn4 ? 8 : 0);
+        const int zt = zp_mode == 2 ? load_int(zp_dt, a.wei_zp.ptr, 0) : 0;
         // offsets of the four columns, as packed pairs: what the packed subtraction (or the f16 fma) takes
         uint32_t o2[4];
+        // (v = zero-point + 8 for s4 as a 16-bit float 2^e + v, in units of the last place, which halve below 2^e;
+        // 8-bit zero-points, f16 only, go through a conversion)
+        const bool zp4 = zp_mode == 0 || zp_dt == DT_U4 || zp_dt == DT_S4;
         auto set_offsets = [&](uint32_t raw) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const int z = base_off + (p.zp_mode == 1 ? zp_of(a.wei_zp.dt, raw, c) : zt);
+                const int v = base_off + (zp_mode == 1 ? zp_of(zp_dt, raw, c) : zt);
+                const int u = v + min(v, 0);
                 uint32_t b;
-                if (F16) b = __half_as_ushort(__int2half_rn((c & 1) ? -(64 + z) : 1024 + z));
-                else b = __bfloat16_as_ushort(__float2bfloat16_rn((float)(128 + z)));
+                if (!F16) b = 0x4300u + u;
+                else if (zp4) b = (c & 1) ? 0xD400u + 16 * u : 0x6400u + u;
+                else b = __half_as_ushort(__int2half_rn((c & 1) ? -(64 + v) : 1024 + v));
                 o2[c] = b * 0x10001u;
             }
         };
         set_offsets(0u);
-        uint32_t it = 0;
-        int s = 0, sa = 0;
-        uint32_t ph = 0, pa = 1;
+        int turn = r; // stages until this warp's next one
+        int sw = 0, s = 0;
+        uint32_t pw = 0, ph = 1;
         bool ok = true;
         for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
             const int64_t n = (int64_t)(t / p.num_m_tiles) * RT_N + 32 * q + 4 * g;
-            // zero-points of this warp's next two stages, loaded ahead (a load takes longer than a stage)
-            uint32_t z0[NZ], z1[NZ], zz[NZ];
-            auto fetch = [&](int st, uint32_t (&z)[NZ]) {
-#pragma unroll
-                for (int j = 0; j < NZ; ++j) {
-                    z[j] = 0u;
-                    if (p.zp_mode == 1 && 4 * st + j < p.ksteps) z[j] = load_zp4(a, (4 * st + j) / p.group_steps, n);
+            // Zero-points: the four lanes of a column group load those of four K-groups, one each, and the next
+            // four while these are in use (a load under this kernel's own traffic takes longer than a stage)
+            const int groups = zp_mode == 1 ? (ksteps + group_steps - 1) / group_steps : 0;
+            auto fetch = [&](int batch) { return 4 * batch + tq < groups ? load_zp4(a, 4 * batch + tq, n) : 0u; };
+            int batch = 0, gi = 0, left = group_steps; // batch held in zcur; group of the next step, its steps left
+            bool fresh = true; // the offsets of group gi are not set yet
+            uint32_t zcur = fetch(0), znext = fetch(1);
+            auto open_group = [&]() {
+                if (!fresh || gi >= groups) return;
+                fresh = false;
+                if (gi >> 2 != batch) {
+                    zcur = gi >> 2 == batch + 1 ? znext : fetch(gi >> 2); // (the other converter's stage held a whole batch)
+                    batch = gi >> 2;
+                    znext = fetch(batch + 1);
                 }
+                set_offsets(__shfl_sync(0xffffffffu, zcur, (lane & ~3) | (gi & 3)));
             };
-            const int first = (int)((it & 1) == (uint32_t)r ? 0 : 1);
-            fetch(first, z0);
-            fetch(first + 2, z1);
-            for (int st = 0; st < p.kstages; ++st, ++it) {
-                if ((int)(it & 1) == r) {
+            auto advance = [&](int steps) {
+                left -= steps;
+                while (left <= 0) { left += group_steps; ++gi; fresh = true; }
+            };
+            for (int st = 0; st < kstages; ++st) {
+                if (turn-- == 0) {
+                    turn = CONV_SETS - 1;
+                    if (!MULTI && zp_mode == 1) {
+                        open_group();
+                        advance(SPS);
+                    }
+                    if (!warp_wait(&w_full[sw], pw)) { ok = false; break; }
+                    const uint8_t *raw = smem + R_W_OFFSET + sw * W_BYTES;
+                    const uint32_t slot = tmem_base + ((uint32_t)(32 * q) << 16) + R_A_COL0 + s * A_SLOT_COLS;
 #pragma unroll
-                    for (int j = 0; j < NZ; ++j) { zz[j] = z0[j]; z0[j] = z1[j]; }
-                    fetch(st + 4, z1);
-                    if (!warp_wait(&w_full[s], ph)) { ok = false; break; }
-                    const uint8_t *raw = smem + R_W_OFFSET + s * W_BYTES;
-                    uint32_t w[4][4]; // [step][k-row], two bytes each
+                    for (int half = 0; half < 2; ++half) {
+                        uint32_t w[4][4]; // [step][k-row], two bytes each
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
+                        for (int k = 0; k < 4; ++k)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) w[k][i] = *reinterpret_cast<const unsigned short *>(raw + k * 1024 + off[i]);
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(&w_empty[s]);
-                    if (!MULTI && p.zp_mode == 1) set_offsets(zz[0]);
-                    uint32_t o[2][16];
+                            for (int i = 0; i < 4; ++i)
+                                w[k][i] = *reinterpret_cast<const unsigned short *>(raw + (4 * half + k) * 1024 + off[i]);
+                        if (half == 0) {
+                            if (!warp_wait(&ab_empty[s], ph)) { ok = false; break; }
+                            ptx::tc_fence_after_sync();
+                        } else {
+                            __syncwarp();
+                            if (lane == 0) ptx::mbar_arrive(&w_empty[sw]);
+                        }
+                        uint32_t oz[MULTI ? 4 : 1][4]; // the offsets of each step
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (MULTI && p.zp_mode == 1) set_offsets(zz[MULTI ? k : 0]);
+                        for (int k = 0; k < (MULTI ? 4 : 1); ++k) {
+                            if (MULTI) {
+                                open_group();
+                                advance(1);
+                            }
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) oz[k][c] = o2[c];
+                        }
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             const uint32_t sel = h ? 0x5511u : 0x4400u; // byte h of both rows
-                            const uint32_t x01 = perm(w[k][0], w[k][1], sel), x23 = perm(w[k][2], w[k][3], sel);
-                            if (F16) {
-                                o[h][4 * k + 0] = sub_f16x2(and_xor(x01, 0x000F000Fu, magic), o2[2 * h]);
-                                o[h][4 * k + 1] = fma_f16x2(and_xor(x01, 0x00F000F0u, magic_hi), 0x2C002C00u, o2[2 * h + 1]);
-                                o[h][4 * k + 2] = sub_f16x2(and_xor(x23, 0x000F000Fu, magic), o2[2 * h]);
-                                o[h][4 * k + 3] = fma_f16x2(and_xor(x23, 0x00F000F0u, magic_hi), 0x2C002C00u, o2[2 * h + 1]);
-                            } else {
-                                o[h][4 * k + 0] = sub_bf16x2(and_xor(x01, 0x000F000Fu, magic), o2[2 * h]);
-                                o[h][4 * k + 1] = sub_bf16x2(and_xor(x01 >> 4, 0x000F000Fu, magic), o2[2 * h + 1]);
-                                o[h][4 * k + 2] = sub_bf16x2(and_xor(x23, 0x000F000Fu, magic), o2[2 * h]);
-                                o[h][4 * k + 3] = sub_bf16x2(and_xor(x23 >> 4, 0x000F000Fu, magic), o2[2 * h + 1]);
+                            uint32_t o[16];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                const uint32_t ol = oz[MULTI ? k : 0][2 * h], oh = oz[MULTI ? k : 0][2 * h + 1];
+                                const uint32_t x01 = perm(w[k][0], w[k][1], sel), x23 = perm(w[k][2], w[k][3], sel);
+                                if (F16) {
+                                    o[4 * k + 0] = sub_f16x2(and_xor(x01, 0x000F000Fu, magic), ol);
+                                    o[4 * k + 1] = fma_f16x2(and_xor(x01, 0x00F000F0u, magic_hi), 0x2C002C00u, oh);
+                                    o[4 * k + 2] = sub_f16x2(and_xor(x23, 0x000F000Fu, magic), ol);
+                                    o[4 * k + 3] = fma_f16x2(and_xor(x23, 0x00F000F0u, magic_hi), 0x2C002C00u, oh);
+                                } else {
+                                    o[4 * k + 0] = sub_bf16x2(and_xor(x01, 0x000F000Fu, magic), ol);
+                                    o[4 * k + 1] = sub_bf16x2(and_xor(x01 >> 4, 0x000F000Fu, magic), oh);
+                                    o[4 * k + 2] = sub_bf16x2(and_xor(x23, 0x000F000Fu, magic), ol);
+                                    o[4 * k + 3] = sub_bf16x2(and_xor(x23 >> 4, 0x000F000Fu, magic), oh);
+                                }
                             }
+                            st_16x128b_x8(slot + ((uint32_t)(16 * h) << 16) + 32 * half, o);
                         }
                     }
-                    if (!warp_wait(&a_empty[sa], pa)) { ok = false; break; }
-                    ptx::tc_fence_after_sync();
-                    const uint32_t slot = tmem_base + ((uint32_t)(32 * q) << 16) + R_A_COL0 + sa * A_SLOT_COLS;
-                    st_16x128b_x8(slot, o[0]);
-                    st_16x128b_x8(slot + (16u << 16), o[1]);
+                    if (!ok) break;
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     ptx::tc_fence_before_sync();
                     __syncwarp(); // every lane's stores to tensor memory are done
-                    if (lane == 0) ptx::mbar_arrive(&a_full[sa]);
+                    if (lane == 0) ptx::mbar_arrive(&ab_full[s]);
+                } else if (zp_mode == 1) {
+                    advance(SPS);
                 }
-                if (++s == W_STAGES) { s = 0; ph ^= 1; }
-                if (++sa == A_SLOTS) { sa = 0; pa ^= 1; }
+                if (++sw == W_STAGES) { sw = 0; pw ^= 1; }
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
         if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp >= R_EPI0) {
         // ------------------------------------------------ epilogue: tot += scale * group sum, then the store
         const int q = warp & 3, h = (warp - R_EPI0) >> 2;
-        const int chunks = p.tile_rows / 16; // 16-row pieces of a tile: the first half of them to h = 0
-        const int c0 = h ? (chunks + 1) / 2 : 0, cn = h ? chunks / 2 : (chunks + 1) / 2;
+        // 16-row pieces of the tile, dealt to the warps of a lane quarter in turn
+        const int pieces = p.tile_rows / 16;
+        const int each = (pieces + R_EPI_WARPS / 4 - 1) / (R_EPI_WARPS / 4);
+        const int c0 = h * each, cn = in_reg(max(0, min(each, pieces - c0)));
         const int col = 32 * q + 4 * (lane & 7) + 2 * (lane >> 4) + ((lane >> 3) & 1);
-        const int groups = (p.ksteps + p.group_steps - 1) / p.group_steps;
+        const int groups = in_reg((p.ksteps + p.group_steps - 1) / p.group_steps);
+        const int sc_dt = in_reg(a.wei_scale.dt), N = in_reg((int)a.N);
+        const int sc_size = sc_dt == DT_F32 ? 4 : sc_dt == DT_BF16 || sc_dt == DT_F16 ? 2 : 1;
+        const int sc_pitch = in_reg((a.wei_scale.mask & 1) ? (int)a.wei_scale.ld * sc_size : 0); // N < 2^29 elements
         float ssc = 1.f;
         if (a.src_scale.ptr) ssc = load_float(a.src_scale.dt, a.src_scale.ptr, 0);
         else if (a.src_scale.on_host) ssc = a.src_scale.host_value;
@@ -409,61 +472,88 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         for (int t = blockIdx.x; t < p.num_tiles && ok && !*abort_flag; t += gridDim.x) {
             const int64_t n = (int64_t)(t / p.num_m_tiles) * RT_N + col;
             const int m0 = (t % p.num_m_tiles) * p.tile_rows;
-            float tot[4][16];
+            uint64_t tot[EPI_PIECES][8]; // pairs of rows: the packed FMA takes half the issue slots
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < EPI_PIECES; ++c)
 #pragma unroll
-                for (int j = 0; j < 16; ++j) tot[c][j] = 0.f;
-            auto scale_at = [&](int g) {
-                if (g >= groups || n >= a.N) return 0.f;
-                return load_float(a.wei_scale.dt, a.wei_scale.ptr, ((a.wei_scale.mask & 1) ? (int64_t)g * a.wei_scale.ld : 0) + n);
+                for (int j = 0; j < 8; ++j) tot[c][j] = 0ull;
+            // Scales of two groups at a time, loaded as raw bits while the two before are folded: a conversion
+            // beside the load would wait for it
+            const char *sc_ptr = (const char *)a.wei_scale.ptr + n * sc_size;
+            auto raw_scale = [&](int g) -> uint32_t {
+                if (g >= groups || n >= N) return 0u;
+                const char *e = sc_ptr + (int64_t)g * sc_pitch;
+                if (sc_dt == DT_F32) return ld_early_u32((const uint32_t *)e);
+                if (sc_size == 2) return ld_early_u16((const unsigned short *)e);
+                return __float_as_uint(load_float(sc_dt, e, 0));
             };
-            float nx[4]; // scales of the next groups, loaded ahead
+            auto scale_of = [&](uint32_t raw) {
+                return sc_dt == DT_BF16 ? __uint_as_float(raw << 16)
+                        : sc_dt == DT_F16 ? __half2float(__ushort_as_half((unsigned short)raw)) : __uint_as_float(raw);
+            };
+            uint32_t cur[2], nxt[2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) nx[i] = scale_at(i);
-            for (int g = 0; g < groups && ok; ++g) {
-                const float sc = nx[0];
-                nx[0] = nx[1]; nx[1] = nx[2]; nx[2] = nx[3];
-                nx[3] = scale_at(g + 4);
+            for (int i = 0; i < 2; ++i) nxt[i] = raw_scale(i);
+            for (int g0 = 0; g0 < groups && ok; g0 += 2) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) cur[i] = nxt[i];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) nxt[i] = raw_scale(g0 + 2 + i);
+#pragma unroll 1
+                for (int i = 0; i < 2 && g0 + i < groups; ++i) {
+                const float sc = scale_of(i == 0 ? cur[0] : cur[1]);
+                const uint64_t sc2 = pack2(__float_as_uint(sc), __float_as_uint(sc));
                 if (!warp_wait(&acc_full[buf], pacc)) { ok = false; break; }
                 ptx::tc_fence_after_sync();
                 const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + buf * RT_M + c0 * 16;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < EPI_PIECES; ++c) {
                     if (c < cn) {
                         uint32_t v[16];
                         ld_32x16(acc + 16 * c, v);
                         ptx::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) tot[c][j] = fmaf(sc, __uint_as_float(v[j]), tot[c][j]);
+                        for (int j = 0; j < 8; ++j) fma_f32x2(tot[c][j], sc2, v[2 * j], v[2 * j + 1]);
                     }
                 }
                 ptx::tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&acc_empty[buf]);
                 if (++buf == ACC_BUFS) { buf = 0; pacc ^= 1; }
+                }
             }
             if (!ok) break;
             if (n < a.N) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < EPI_PIECES; ++c) {
                     if (c >= cn) continue;
                     const int64_t mc = m0 + (c0 + c) * 16;
                     const int rows = (int)min((int64_t)16, min((int64_t)m0 + p.tile_rows, a.M) - mc);
+                    float d[16];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        if (j >= rows) continue;
-                        const int64_t m = mc + j;
-                        float d = tot[c][j] * ssc;
-                        if (a.bias) d = __fadd_rn(d, load_float(a.bias_dt, a.bias, m * a.bias_sm + n * a.bias_sn));
-                        if (p.fast_store) {
-                            const int64_t o = m * a.dst_sm + n * a.dst_sn;
-                            if (a.dst_dt == DT_BF16) ((unsigned short *)a.dst)[o] = f32_to_bf16_bits(d);
-                            else if (a.dst_dt == DT_F16) ((__half *)a.dst)[o] = __float2half_rn(d);
-                            else ((float *)a.dst)[o] = d;
+                    for (int j = 0; j < 16; ++j) d[j] = __uint_as_float((uint32_t)(tot[c][j >> 1] >> (32 * (j & 1)))) * ssc;
+                    if (p.fast_store && !a.bias) {
+                        const int64_t o = mc * a.dst_sm + n;
+                        if (a.dst_dt == DT_BF16) {
+                            unsigned short *dp = (unsigned short *)a.dst + o;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (j < rows) dp[j * a.dst_sm] = f32_to_bf16_bits(d[j]);
+                        } else if (a.dst_dt == DT_F16) {
+                            __half *dp = (__half *)a.dst + o;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (j < rows) dp[j * a.dst_sm] = __float2half_rn(d[j]);
                         } else {
-                            finish_store_general(a, d, m, n);
+                            float *dp = (float *)a.dst + o;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (j < rows) dp[j * a.dst_sm] = d[j];
                         }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (j < rows) finish_store_general(a, d[j], mc + j, n);
                     }
                 }
             }
@@ -547,7 +637,7 @@ int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     {
         cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M};
         cuuint64_t strides[1] = {(cuuint64_t)(a.src_sm * 2)};
-        cuuint32_t box[2] = {RK, (cuuint32_t)p.tile_rows};
+        cuuint32_t box[2] = {64, (cuuint32_t)p.tile_rows};
         cuuint32_t estr[2] = {1, 1};
         if (enc(&ts, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(a.src), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -564,12 +654,12 @@ int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     if (p.group_steps < 1 || p.group_steps > p.ksteps) p.group_steps = p.ksteps;
     p.sgn4 = a.wei_dt == DT_S4;
     p.zp_mode = !a.wei_zp.ptr ? 0 : (a.wei_zp.mask ? 1 : 2);
-    p.fast_store = a.n_po == 0 && !a.dst_scale.ptr && !a.dst_scale.on_host
+    p.fast_store = a.dst_sn == 1 && a.n_po == 0 && !a.dst_scale.ptr && !a.dst_scale.on_host
             && (a.dst_dt == DT_F32 || a.dst_dt == DT_BF16 || a.dst_dt == DT_F16);
     const bool f16 = a.src_dt == DT_F16;
     const uint32_t fmt = f16 ? ptx::FMT_F16 : ptx::FMT_BF16;
     p.idesc = ptx::make_idesc(ptx::CFMT_F32, fmt, fmt, false, false, RT_N, (uint32_t)p.tile_rows);
-    const bool multi = p.group_steps % 4 != 0 && p.zp_mode == 1;
+    const bool multi = p.group_steps % SPS != 0 && p.zp_mode == 1;
     if (f16) return multi ? rows_launch<true, true>(tw, ts, a, p, sm_count, st) : rows_launch<true, false>(tw, ts, a, p, sm_count, st);
     return multi ? rows_launch<false, true>(tw, ts, a, p, sm_count, st) : rows_launch<false, false>(tw, ts, a, p, sm_count, st);
 }
