@@ -10,34 +10,44 @@
 // from a small pre-kernel.
 //
 // tcgen05.mma takes its A operand from TENSOR MEMORY, so the widened weights
-// never pass through shared memory: TMA brings a raw [64 k x 128 n] s8 tile
+// never pass through shared memory: TMA brings raw [128 k x 128 n] s8 tiles
 // (128B-swizzled rows), converter warps read four k-rows of four columns per
-// lane and k16 step, pair the k-rows with one PRMT, widen them to bf16 (exact:
-// 8 significant bits) and write the stage's operand - 128 TMEM lanes x 32
-// columns, the fragment layout of `tcgen05.st.16x128b` - with two stores per
-// warp; `tcgen05.mma kind::f16` multiplies it with the src rows (K-major,
-// straight from TMA).  Shared memory carries the raw bytes once in, once out,
-// and the src rows; the bf16 copy (2 bytes per weight written and read again)
-// is gone from it.  As in the 8-bit GEMM the kernel computes dst^T: weights
-// are the A operand (128 dst columns = TMEM lanes), src rows the B operand, so
-// an epilogue lane owns one dst column, keeps its scale in a register and
-// stores coalesced rows.  Which column a TMEM lane holds is a permutation
-// inside each group of 32 (lane 16h + 8i + g <-> column 4g + 2h + i), chosen
-// so that a converter lane's four bytes go to the lanes its stores can reach.
+// lane and k16 step, pair the k-rows with PRMTs, widen them to bf16 (x / 64,
+// exact: 8 significant bits; see s8x2_to_bf16x2) and write a slot's operand -
+// 128 TMEM lanes x 32 columns, the fragment layout of `tcgen05.st.16x128b` -
+// with two stores per warp; `tcgen05.mma kind::f16` multiplies it with the src
+// rows (K-major, straight from TMA).  As in the 8-bit GEMM the kernel computes
+// dst^T: weights are the A operand (128 dst columns = TMEM lanes), src rows the
+// B operand, so an epilogue lane owns one dst column, keeps its scale in a
+// register and stores coalesced rows.  Which column a TMEM lane holds is a
+// permutation inside each group of 32 (lane 16h + 8i + g <-> column
+// 4g + 2h + i), chosen so that a converter lane's four bytes go to the lanes its
+// stores can reach.
 //
-// Tiles are (expert, 128 columns, up to 192 rows of that expert): two
-// accumulator buffers of 192 columns and four operand slots of 32 fill the 512
-// columns of tensor memory.  The MMA's N extent is the tile's row count
-// rounded up to 16, so small experts cost little tensor time.  Tile order:
-// expert, column block, row block fastest, so CTAs running together share
-// weight tiles through L2.  A small planning kernel turns the offsets
-// (cumulative END rows, validated like ref_grouped_gemm.cpp:164-213) into
-// per-expert tile ranges on the device: no host synchronisation.  One
-// persistent CTA per SM: warp 0 streams the raw weight tiles (ring of 8: they
-// come from HBM), the last warp the src rows (ring of 6), warps 2-9 convert
-// (two per lane quarter, alternating stages), warp 1 and the last three warps
-// issue the MMAs (stage by stage, in turn), four warps run the epilogue.  The issuing loops are warp-uniform code whose
-// tcgen05 / TMA instructions sit in a branch taken by one elected thread.  Every mbarrier wait is bounded.
+// Tiles are (expert, 128 columns, up to 208 rows of that expert): two
+// accumulator buffers of 208 columns and three operand slots of 32 fill the 512
+// columns of tensor memory.  An expert's rows are cut into blocks of equal size;
+// the MMA's N extent is the block's row count rounded up to 16, so small experts
+// cost little tensor time.  Tile order: expert, column block, row block fastest,
+// so CTAs running together share weight tiles through L2.  A small planning
+// kernel turns the offsets (cumulative END rows, validated like
+// ref_grouped_gemm.cpp:164-213) into per-expert tile ranges on the device: no
+// host synchronisation.
+//
+// One persistent CTA per SM: warp 0 streams the raw weight tiles (ring of 5), the
+// last warp the src rows (ring of 5), warp 1 issues all MMAs - one elected thread
+// each -, twelve warps convert (three per lane quarter, taking the slots in turn),
+// four run the epilogue.  Every mbarrier wait is bounded.
+//
+// What bounds it: for few rows the conversion (ALU pipe and the chain of waits of
+// a converter warp, about 400 cycles per 64 k x 128 columns against 320 of the HBM
+// stream); for full tiles what an SM can pull out of L2 (8 KB of weights and up to
+// 26 KB of src rows per 64 k).  Measured on a B200, us per call, before -> now, the
+// earlier form being four issuing warps that handed the stage order on, eight
+// converter warps with three LOP3 more per pair and blocks of up to 192 rows:
+// 8192 rows over 64 experts (Zipf), K = 4096, N = 14336: 1662 -> 1384; 37 rows over 8
+// experts: 162 -> 119; dense, 777 rows, K = N = 4096: 71 -> 42.  Four converter sets
+// with four slots and 192-row blocks, conversion unchanged: 1514 / 140 / 66.
 #include <cuda.h>
 
 #include "device_math.cuh"
@@ -52,18 +62,21 @@ namespace qmm {
 namespace {
 
 constexpr int GT_N = 128; // dst columns per tile = TMEM lanes = UMMA M
-constexpr int GT_M = 192; // most src rows per tile = UMMA N
-constexpr int GK = 64; // k per stage: one 128-byte swizzle row of bf16 src
-// Two shared-memory rings and one in tensor memory: the raw weights come from HBM (deep ring of small
-// tiles to cover its latency), the src rows from L2, and the widened operand is produced and consumed
-// on the SM (four slots of 32 columns beside the two accumulators).
-constexpr int RAW_STAGES = 8, A_SLOTS = 4, B_STAGES = 6;
-constexpr int RAW_BYTES = GK * GT_N; // s8 weights as loaded
+constexpr int GT_M = 208; // most src rows per tile = UMMA N
+constexpr int GK = 64; // k per operand slot: one 128-byte swizzle row of bf16 src
+// Two shared-memory rings and one in tensor memory: the raw weights come from HBM, the src rows from L2,
+// and the widened operand is produced and consumed on the SM (slots of 32 columns beside the two accumulators).
+// 208 rows per tile: what the two accumulators leave is three slots, which is what three converter sets fill;
+// 777 rows of a dense problem are then four blocks of 195 and 128 tiles - one wave - instead of 160 tiles.
+constexpr int RAW_STAGES = 5, A_SLOTS = 3, B_STAGES = 5;
+constexpr int LK = 2 * GK; // k per raw weight tile: a copy costs its thread about 500 cycles, whatever its size
+constexpr int RAW_BYTES = LK * GT_N; // s8 weights as loaded
 constexpr int B_BYTES = GT_M * GK * 2; // src rows, K-major
-constexpr int CONV_WARPS = 8, EPI_WARPS = 4;
-constexpr int MMA_WARPS = 4; // issuers: stage s belongs to issuer s % MMA_WARPS
-constexpr int G_THREADS = 32 * (3 + CONV_WARPS + EPI_WARPS + MMA_WARPS - 1);
-constexpr int MMA_WARP1 = 3 + CONV_WARPS + EPI_WARPS; // the issuers after the first are the last warps
+constexpr int CONV_SETS = 3; // sets of four converter warps (one per lane quarter), which take the stages in turn
+// a set that could run ahead of the others by more than the ring would take an older phase of a slot for its own
+static_assert(CONV_SETS <= A_SLOTS, "barrier parity");
+constexpr int CONV_WARPS = 4 * CONV_SETS, EPI_WARPS = 4;
+constexpr int G_THREADS = 32 * (3 + CONV_WARPS + EPI_WARPS);
 constexpr int ACC_STAGES = 2;
 constexpr int A_SLOT_COLS = GK / 2; // two k per 32-bit column
 constexpr int A_COL0 = ACC_STAGES * GT_M;
@@ -74,13 +87,6 @@ constexpr int PLAN_CACHE_GROUPS = 511; // records kept in shared memory (8 KB); 
 constexpr int G_PLAN_OFFSET = G_BAR_OFFSET + 512;
 constexpr int G_SMEM_BYTES = G_PLAN_OFFSET + (PLAN_CACHE_GROUPS + 1) * 16 + 1024;
 static_assert(G_SMEM_BYTES <= 227 * 1024, "shared memory");
-
-#ifdef QMM_PROFILE // builds with -DQMM_PROFILE stamp the SM clock of CTA 0 per role and stage; the shipped library has no such code
-__device__ unsigned long long *g_grouped_trace = nullptr;
-#define GT_TRACE(role, idx) do { if (g_grouped_trace && blockIdx.x == 0 && (idx) < 256) g_grouped_trace[(role) * 256 + (idx)] = (unsigned long long)clock64(); } while (0)
-#else
-#define GT_TRACE(role, idx) do { } while (0)
-#endif
 
 // plan[0] = {total tiles, groups, 0, 0}; plan[1 + g] = {first src row, first dst row, rows, first tile}
 struct Tile {
@@ -99,9 +105,11 @@ __device__ __forceinline__ Tile decode_tile(const int4 *plan, int groups, int nu
     const int mt = (e.z + GT_M - 1) / GT_M;
     Tile tl;
     tl.g = lo;
+    // row blocks of equal size (a multiple of 16): a short last block would pay a whole pass over the weights
+    const int per = ((e.z + mt - 1) / mt + 15) & ~15;
     tl.n0 = (r / mt) * GT_N;
-    tl.m0 = (r % mt) * GT_M;
-    tl.rows = min(GT_M, e.z - tl.m0);
+    tl.m0 = (r % mt) * per;
+    tl.rows = min(per, e.z - tl.m0);
     tl.src_row = e.x + tl.m0;
     tl.dst_row = e.y + tl.m0;
     return tl;
@@ -132,23 +140,22 @@ __global__ void grouped_plan_kernel(const __grid_constant__ MatmulArgs a, int4 *
     plan[0] = make_int4(tiles, a.group_count, 0, 0);
 }
 
-// four s8 -> four bf16 without a conversion instruction: with xx = x & 0x7f the bf16 0x43xx is
-// 128 + (x & 127), with xx = x & 0x80 it is 128 or 256; their difference is x, exactly
 __device__ __forceinline__ uint32_t prmt_(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t r;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
     return r;
 }
-__device__ __forceinline__ uint32_t bf16x2_sub(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+// Two s8 -> two bf16 of x / 64, exactly, with one LOP3 and one packed FMA.  A bf16 whose upper byte is zero is
+// u * 2^-133 for every lower byte u (the step from subnormal to normal numbers included), so with u = x + 128
+// (the sign bit flipped) u * 2^-133 * 2^127 - 2 = (u - 128) / 64.  The epilogue multiplies the sums by 64.
+// (Masks and a subtraction of 128 or 256 took three LOP3 and a subtraction per pair; the ALU pipe sets this
+// kernel's conversion rate.)
+constexpr float A_SCALE = 64.f;
+__device__ __forceinline__ uint32_t s8x2_to_bf16x2(uint32_t t) { // the bytes 0 and 2 of t
+    uint32_t u, d;
+    asm("lop3.b32 %0, %1, 0x00ff00ff, 0x00800080, 0x6a;" : "=r"(u) : "r"(t)); // (t & 0xff00ff) ^ 0x800080
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(u), "r"(0x7F007F00u), "r"(0xC000C000u));
     return d;
-}
-__device__ __forceinline__ void s8x4_to_bf16x4(uint32_t w, uint32_t &o0, uint32_t &o1) {
-    const uint32_t p0 = prmt_(w, 0x43434343u, 0x4140); // [x0, 0x43, x1, 0x43]
-    const uint32_t p1 = prmt_(w, 0x43434343u, 0x4342); // [x2, 0x43, x3, 0x43]
-    o0 = bf16x2_sub(p0 & 0xff7fff7fu, p0 & 0xff80ff80u);
-    o1 = bf16x2_sub(p1 & 0xff7fff7fu, p1 & 0xff80ff80u);
 }
 
 // 16 TMEM lanes x 32 columns (the four k16 steps of a stage): thread (g = lane / 4, t = lane % 4)
@@ -199,34 +206,31 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     uint64_t *raw_empty = raw_full + RAW_STAGES; // the converters have read it
     uint64_t *b_full = raw_empty + RAW_STAGES; // src rows have landed
     uint64_t *b_empty = b_full + B_STAGES; // the MMAs have read them
-    uint64_t *a_full = b_empty + B_STAGES; // the stage's operand is in tensor memory
+    uint64_t *a_full = b_empty + B_STAGES; // the slot's operand is in tensor memory
     uint64_t *a_empty = a_full + A_SLOTS; // the MMAs have read it
     uint64_t *tmem_full = a_empty + A_SLOTS;
     uint64_t *tmem_empty = tmem_full + ACC_STAGES;
-    // stages whose MMAs are in the pipe (written by the two issuers in turn, read by the other)
-    volatile uint32_t *stages_issued = (volatile uint32_t *)(tmem_empty + ACC_STAGES);
-    uint32_t *tmem_base_slot = (uint32_t *)(tmem_empty + ACC_STAGES + 1);
+    uint32_t *tmem_base_slot = (uint32_t *)(tmem_empty + ACC_STAGES);
     volatile int *abort_flag = (volatile int *)(tmem_base_slot + 1);
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     if (threadIdx.x == 0) {
         for (int s = 0; s < RAW_STAGES; ++s) {
             ptx::mbar_init(&raw_full[s], 1);
-            ptx::mbar_init(&raw_empty[s], CONV_WARPS / 2); // the stage's four converter warps
+            ptx::mbar_init(&raw_empty[s], 8); // four converter warps for each of its two halves
         }
         for (int s = 0; s < B_STAGES; ++s) {
             ptx::mbar_init(&b_full[s], 1);
             ptx::mbar_init(&b_empty[s], 1);
         }
         for (int s = 0; s < A_SLOTS; ++s) {
-            ptx::mbar_init(&a_full[s], CONV_WARPS / 2);
+            ptx::mbar_init(&a_full[s], 4); // the slot's four converter warps
             ptx::mbar_init(&a_empty[s], 1);
         }
         for (int s = 0; s < ACC_STAGES; ++s) {
-            ptx::mbar_init(&tmem_full[s], MMA_WARPS);
+            ptx::mbar_init(&tmem_full[s], 1);
             ptx::mbar_init(&tmem_empty[s], EPI_WARPS);
         }
-        *stages_issued = 0u;
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::prefetch_tensormap(&tmW);
@@ -252,126 +256,86 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         plan = cache;
     }
 
+    // The three single-thread roles: one elected thread runs the whole loop.
     if (warp == 0) {
         // ------------------------------------------------ TMA producer of the raw weight tiles
-        // (the whole warp walks the loop, one elected thread issues: the addresses stay warp-uniform values)
-        const bool issue = lane == 0;
-        int s = 0;
-        uint32_t ph = 1; // parity of the empty barrier's previous phase: a fresh barrier passes
-        [[maybe_unused]] uint32_t pit = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x) {
-            const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
-            for (int kb = 0; kb < num_k_blocks; ++kb) {
-                if (!__all_sync(0xffffffffu, ptx::mbar_wait(&raw_empty[s], ph))) { ok = false; break; }
-                if (ptx::elect_one()) {
+        if (ptx::elect_one()) {
+            int s = 0;
+            uint32_t ph = 1; // parity of the empty barrier's previous phase: a fresh barrier passes
+            bool ok = true;
+            for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x) {
+                const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
+                for (int kb = 0; kb < num_k_blocks; kb += 2) {
+                    if (!ptx::mbar_wait(&raw_empty[s], ph)) { ok = false; break; }
                     ptx::mbar_arrive_expect_tx(&raw_full[s], RAW_BYTES);
                     ptx::tma_load_3d(smem + RAW_OFFSET + s * RAW_BYTES, &tmW, &raw_full[s], tl.n0, kb * GK, tl.g);
+                    if (++s == RAW_STAGES) { s = 0; ph ^= 1; }
                 }
-                __syncwarp();
-                if (issue) GT_TRACE(0, pit);
-                ++pit;
-                if (++s == RAW_STAGES) { s = 0; ph ^= 1; }
             }
+            if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
-        if (!ok && issue) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp == 2 + CONV_WARPS + EPI_WARPS) {
         // ------------------------------------------------ TMA producer of the src rows
-        const bool issue = lane == 0;
-        int s = 0;
-        uint32_t ph = 1;
-        [[maybe_unused]] uint32_t bit = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x) {
-            const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
-            // one copy per stage (issuing a copy costs this thread about as much as the wait): a box of
-            // 64, 128 or 192 rows, whichever covers the tile's rows
-            const int nbox = (tl.rows + 63) / 64;
-            const CUtensorMap *tm = nbox == 1 ? &tmS : nbox == 2 ? &tmS2 : &tmS3;
-            for (int kb = 0; kb < num_k_blocks; ++kb) {
-                if (!__all_sync(0xffffffffu, ptx::mbar_wait(&b_empty[s], ph))) { ok = false; break; }
-                uint8_t *bt = smem + B_OFFSET + s * B_BYTES;
-                if (ptx::elect_one()) {
-                    ptx::mbar_arrive_expect_tx(&b_full[s], nbox * 64 * GK * 2);
-                    ptx::tma_load_2d(bt, tm, &b_full[s], kb * GK, tl.src_row);
+        if (ptx::elect_one()) {
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x) {
+                const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
+                // a box of 64, 128 or GT_M rows, whichever covers the tile's rows
+                const CUtensorMap *tm = tl.rows <= 64 ? &tmS : tl.rows <= 128 ? &tmS2 : &tmS3;
+                const uint32_t bytes = (tl.rows <= 64 ? 64 : tl.rows <= 128 ? 128 : GT_M) * GK * 2;
+                for (int kb = 0; kb < num_k_blocks; ++kb) {
+                    if (!ptx::mbar_wait(&b_empty[s], ph)) { ok = false; break; }
+                    ptx::mbar_arrive_expect_tx(&b_full[s], bytes);
+                    ptx::tma_load_2d(smem + B_OFFSET + s * B_BYTES, tm, &b_full[s], kb * GK, tl.src_row);
+                    if (++s == B_STAGES) { s = 0; ph ^= 1; }
                 }
-                __syncwarp();
-                if (issue) GT_TRACE(1, bit);
-                ++bit;
-                if (++s == B_STAGES) { s = 0; ph ^= 1; }
             }
+            if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
-        if (!ok && issue) { *abort_flag = 1; atomicExch(a.status, 5); }
-    } else if (warp == 1 || warp >= MMA_WARP1) {
-        // ------------------------------------------------ MMA issuers (warp-uniform loops, an elected thread issues)
-        // A warp issues an MMA every 40 to 65 cycles (twice that inside this kernel) and pays two waits
-        // and two commits per stage, more than the MMAs of a stage take: four warps share the work,
-        // stage by stage, waiting for their tiles and committing while another one issues.  The stages enter the pipe in their own order -
-        // each issuer tells the other when its stage is in (a fence and a released store) - so the sums
-        // are added in the same order every time and a second execution gives the same bits.
-        const int me = warp == 1 ? 0 : warp - MMA_WARP1 + 1;
-        const bool issue = lane == 0;
-        int sa = 0, sb = 0;
-        uint32_t pa = 0, pb = 0; // parities of the full barriers
-        uint32_t acc_it = 0, it = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x, ++acc_it) {
-            const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
-            const uint32_t n_mma = (uint32_t)max(16, (tl.rows + 15) & ~15);
-            const uint32_t idesc = ptx::make_idesc(ptx::CFMT_F32, ptx::FMT_BF16, ptx::FMT_BF16, false, false, GT_N, n_mma);
-            const int as = acc_it % ACC_STAGES;
-            const uint32_t aph = (acc_it / ACC_STAGES) & 1;
-            const uint32_t tmem_d = tmem_base + as * GT_M;
-            for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
-                if ((int)(it % MMA_WARPS) == me) {
-                    if (kb == 0) { // the tile's first stage overwrites the accumulator: the epilogue must have read it
-                        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&tmem_empty[as], aph ^ 1))) { ok = false; break; }
-                    }
-                    if (issue) GT_TRACE(2, it);
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&a_full[sa], pa))) { ok = false; break; }
-                    if (issue) GT_TRACE(3, it);
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&b_full[sb], pb))) { ok = false; break; }
-                    if (issue) GT_TRACE(4, it);
-                    // the stage before this one (the other issuer's) is in the pipe: a word in shared memory,
-                    // polled with plain loads (the hand-off is on the critical path of every stage, and a
-                    // woken mbarrier wait costs several hundred cycles more)
-                    {
-                        uint32_t seen = ptx::ld_acquire_shared(stages_issued);
-                        for (int spin = 0; seen < it && spin < (1 << 24); ++spin) seen = ptx::ld_acquire_shared(stages_issued);
-                        if (!__all_sync(0xffffffffu, seen >= it)) { ok = false; break; }
-                    }
+    } else if (warp == 1) {
+        // ------------------------------------------------ MMA issuer
+        // One elected thread runs the whole loop: it issues a tcgen05.mma about every 12 cycles, and the MMAs
+        // complete in the order of their issue, so the sums are added in the same order every time.  (Issuing
+        // by whole warps cost so much more that four of them shared the stages and handed the order on.)
+        if (ptx::elect_one()) {
+            int sa = 0, sb = 0;
+            uint32_t pa = 0, pb = 0, acc_it = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x, ++acc_it) {
+                const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
+                const uint32_t n_mma = (uint32_t)max(16, (tl.rows + 15) & ~15);
+                const uint32_t idesc = ptx::make_idesc(ptx::CFMT_F32, ptx::FMT_BF16, ptx::FMT_BF16, false, false, GT_N, n_mma);
+                const int as = acc_it % ACC_STAGES;
+                const uint32_t aph = (acc_it / ACC_STAGES) & 1;
+                const uint32_t tmem_d = tmem_base + as * GT_M;
+                if (!ptx::mbar_wait(&tmem_empty[as], aph ^ 1)) { ok = false; break; } // the epilogue has read the accumulator
+                ptx::tc_fence_after_sync();
+                for (int kb = 0; kb < num_k_blocks; ++kb) {
+                    if (!ptx::mbar_wait(&b_full[sb], pb)) { ok = false; break; }
+                    if (!ptx::mbar_wait(&a_full[sa], pa)) { ok = false; break; }
                     ptx::tc_fence_after_sync();
-                    if (issue) GT_TRACE(5, it);
-                    // src rows K-major: 32 bytes of the row per MMA; the descriptor is built once per stage
+                    // src rows K-major: 32 bytes of the row per MMA; the descriptor is built once per slot
                     // and advanced by a constant in its start-address field (16-byte units)
                     const uint64_t sd0 = ptx::smem_desc_sw128(ptx::smem_u32(smem + B_OFFSET + sb * B_BYTES), 0, 1024);
                     const uint32_t ta = tmem_base + A_COL0 + sa * A_SLOT_COLS;
-                    if (ptx::elect_one()) { // one elected thread: see elect_one
 #pragma unroll
-                        for (int kk = 0; kk < GK / 16; ++kk)
-                            mma_ts_bf16(tmem_d, ta + 8 * kk, sd0 + (uint64_t)(kk * (32 >> 4)), idesc, (kb | kk) != 0);
-                        ptx::tc_fence_before_sync();
-                        ptx::st_release_shared(stages_issued, it + 1);
-                        // the operand slot and the src tile are reusable once these MMAs have read them
-                        ptx::tc_commit(&a_empty[sa]);
-                        ptx::tc_commit(&b_empty[sb]);
-                    }
-                    __syncwarp();
-                    if (issue) GT_TRACE(6, it);
+                    for (int kk = 0; kk < GK / 16; ++kk)
+                        mma_ts_bf16(tmem_d, ta + 8 * kk, sd0 + (uint64_t)(kk * (32 >> 4)), idesc, (kb | kk) != 0);
+                    // the operand slot and the src tile are free once these MMAs have read them
+                    ptx::tc_commit(&a_empty[sa]);
+                    ptx::tc_commit(&b_empty[sb]);
+                    if (++sa == A_SLOTS) { sa = 0; pa ^= 1; }
+                    if (++sb == B_STAGES) { sb = 0; pb ^= 1; }
                 }
-                if (++sa == A_SLOTS) { sa = 0; pa ^= 1; }
-                if (++sb == B_STAGES) { sb = 0; pb ^= 1; }
+                if (ok) ptx::tc_commit(&tmem_full[as]); // accumulator complete
             }
-            if (!ok) break;
-            // this thread's share of the accumulator is complete (tcgen05.commit covers the MMAs of the
-            // thread that executes it: the elected lane is the same one, the lowest, every time)
-            if (ptx::elect_one()) ptx::tc_commit(&tmem_full[as]);
-            __syncwarp();
+            if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
-        if (!ok && issue) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp < 2 + CONV_WARPS) {
         // ------------------------------------------------ converters: s8 tile -> bf16 operand in tensor memory
-        // Warp (q = warp % 4, r): TMEM lanes 32q .. 32q+31, the stages of parity r.  Lane (g, t) reads,
+        // Warp (q = warp % 4, r): TMEM lanes 32q .. 32q+31, the stages of set r.  Lane (g, t) reads,
         // per k16 step, the four bytes of columns 32q + 4g .. +3 in the k-rows 2t, 2t+1, 2t+8, 2t+9; byte
         // 2h + i of those goes to TMEM lane 32q + 16h + 8i + g, so one 16-lane store per h carries the
         // stage's four steps.
@@ -385,16 +349,16 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             const uint32_t row = 2 * tq + (i & 1) + 8 * (i >> 1);
             off[i] = row * 128 + ((chunk ^ (row & 7)) << 4) + within;
         }
-        uint32_t it = 0;
+        int turn = r; // stages until this warp's next one
         int sr = 0, sa = 0;
         uint32_t pr = 0, pa = 1;
         bool ok = true;
         for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x) {
-            for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
-                if ((int)(it & 1) == r) {
+            for (int kb = 0; kb < num_k_blocks; ++kb) {
+                if (turn-- == 0) {
+                    turn = CONV_SETS - 1;
                     if (!__all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&raw_full[sr], pr))) { ok = false; break; }
-                    if (warp == 2 && lane == 0) GT_TRACE(7, it);
-                    const uint8_t *raw = smem + RAW_OFFSET + sr * RAW_BYTES;
+                    const uint8_t *raw = smem + RAW_OFFSET + sr * RAW_BYTES + (kb & 1) * (RAW_BYTES / 2);
                     uint32_t w[4][4]; // [step][k-row]
 #pragma unroll
                     for (int st = 0; st < 4; ++st)
@@ -405,16 +369,17 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                     if (lane == 0) ptx::mbar_arrive(&raw_empty[sr]);
                     if (!__all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&a_empty[sa], pa))) { ok = false; break; }
                     ptx::tc_fence_after_sync();
-                    if (warp == 2 && lane == 0) GT_TRACE(8, it);
                     const uint32_t slot = tmem_base + ((uint32_t)(32 * q) << 16) + A_COL0 + sa * A_SLOT_COLS;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const uint32_t sel = h ? 0x7362u : 0x5140u; // [a.b(2h), b.b(2h), a.b(2h+1), b.b(2h+1)]
+                        const uint32_t sel0 = h ? 0x7662u : 0x5440u, sel1 = h ? 0x7773u : 0x5551u; // byte 2h (2h + 1) of both rows
                         uint32_t o[16];
 #pragma unroll
                         for (int st = 0; st < 4; ++st) {
-                            s8x4_to_bf16x4(prmt_(w[st][0], w[st][1], sel), o[4 * st + 0], o[4 * st + 1]);
-                            s8x4_to_bf16x4(prmt_(w[st][2], w[st][3], sel), o[4 * st + 2], o[4 * st + 3]);
+                            o[4 * st + 0] = s8x2_to_bf16x2(prmt_(w[st][0], w[st][1], sel0));
+                            o[4 * st + 1] = s8x2_to_bf16x2(prmt_(w[st][0], w[st][1], sel1));
+                            o[4 * st + 2] = s8x2_to_bf16x2(prmt_(w[st][2], w[st][3], sel0));
+                            o[4 * st + 3] = s8x2_to_bf16x2(prmt_(w[st][2], w[st][3], sel1));
                         }
                         tmem_st_16x128b_x8(slot + ((uint32_t)(16 * h) << 16), o);
                     }
@@ -422,9 +387,8 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                     ptx::tc_fence_before_sync();
                     __syncwarp(); // every lane's stores to tensor memory are done
                     if (lane == 0) ptx::mbar_arrive(&a_full[sa]);
-                    if (warp == 2 && lane == 0) GT_TRACE(9, it);
                 }
-                if (++sr == RAW_STAGES) { sr = 0; pr ^= 1; }
+                if ((kb & 1) && ++sr == RAW_STAGES) { sr = 0; pr ^= 1; }
                 if (++sa == A_SLOTS) { sa = 0; pa ^= 1; }
             }
         }
@@ -469,7 +433,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                         for (int j = 0; j < 32; ++j) {
                             if (j >= m_hi) continue;
                             const int64_t m = row0 + j;
-                            float acc = __uint_as_float(r[j]);
+                            float acc = __uint_as_float(r[j]) * A_SCALE;
                             if (a.wei_zp.ptr) acc = fmaf(-zp, ptx::ld_dependent(rowsum + tl.src_row + cidx * 32 + j), acc);
                             float d = __fmul_rn(acc, scale);
                             if (a.bias)
@@ -484,12 +448,12 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                         unsigned short *d = (unsigned short *)a.dst + row0 * a.dst_sm + n;
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (j < m_hi) d[(int64_t)j * a.dst_sm] = f32_to_bf16_bits(__uint_as_float(r[j]) * scale);
+                            if (j < m_hi) d[(int64_t)j * a.dst_sm] = f32_to_bf16_bits(__uint_as_float(r[j]) * A_SCALE * scale);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
                             if (j < m_hi)
-                                store_float(a.dst_dt, __uint_as_float(r[j]) * scale, a.dst, (row0 + j) * a.dst_sm + n);
+                                store_float(a.dst_dt, __uint_as_float(r[j]) * A_SCALE * scale, a.dst, (row0 + j) * a.dst_sm + n);
                     }
                 }
             }
@@ -539,12 +503,12 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
     encode_tiled_fn enc = grouped_get_encode();
     if (!enc || !scratch) return 5;
     CUtensorMap tw, ts, ts2, ts3;
-    { // weights as bytes [G][K][N]: raw tile of 64 k x 128 n, 128B swizzle; a dense [K][N] matrix is one group
+    { // weights as bytes [G][K][N]: raw tile of 128 k x 128 n, 128B swizzle; a dense [K][N] matrix is one group
         const int64_t groups = a.group_count > 0 ? a.group_count : 1;
         const int64_t group_pitch = a.group_count > 0 ? a.wei_sg : a.K * a.wei_sk;
         cuuint64_t dims[3] = {(cuuint64_t)a.N, (cuuint64_t)a.K, (cuuint64_t)groups};
         cuuint64_t strides[2] = {(cuuint64_t)a.wei_sk, (cuuint64_t)group_pitch};
-        cuuint32_t box[3] = {GT_N, GK, 1};
+        cuuint32_t box[3] = {GT_N, LK, 1};
         cuuint32_t estr[3] = {1, 1, 1};
         if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(a.wei), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -552,12 +516,12 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
                 != CUDA_SUCCESS)
             return 5;
     }
-    // src as 16-bit words [M][K]: boxes of 64, 128 and 192 rows x 64 k, 128B swizzle
+    // src as 16-bit words [M][K]: boxes of 64, 128 and GT_M rows x 64 k, 128B swizzle
     CUtensorMap *src_maps[3] = {&ts, &ts2, &ts3};
     for (int i = 0; i < 3; ++i) {
         cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M};
         cuuint64_t strides[1] = {(cuuint64_t)(a.src_sm * 2)};
-        cuuint32_t box[2] = {GK, (cuuint32_t)(64 * (i + 1))};
+        cuuint32_t box[2] = {GK, (cuuint32_t)(i == 2 ? GT_M : 64 * (i + 1))};
         cuuint32_t estr[2] = {1, 1};
         if (enc(src_maps[i], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(a.src), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -566,7 +530,7 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
             return 5;
     }
     const int num_n_tiles = (int)((a.N + GT_N - 1) / GT_N);
-    const int num_k_blocks = (int)((a.K + GK - 1) / GK);
+    const int num_k_blocks = (int)((a.K + LK - 1) / LK) * 2; // in pairs: k beyond K reads as zeros
     int4 *plan = (int4 *)scratch;
     grouped_plan_kernel<<<1, 32, 0, st>>>(a, plan, num_n_tiles);
     count_launch();

@@ -4,11 +4,14 @@
 // scales per column or per (K-group, column), optional 4-bit zero-points (f16 src: 8-bit ones too) with the
 // same grouping or per tensor (fpmath apply_to_int; reference arithmetic: src/cpu/matmul/ref_matmul.cpp:193-233).
 //
-// w - zero_point is an integer that bf16 (f16) holds exactly, so the operand of the MMAs is exact: a nibble
-// becomes 128 + u (f16: 1024 + u) with one LOP3 per two weights and one packed subtraction takes off
-// 128 (+ 8 for s4) + zero_point.  The sums of a K-group are then exact products added in f32, and the group's
-// scale multiplies the finished group sum: tot += scale * sum, in f32 registers of the epilogue.  Nothing is
-// rounded to 16 bits before dst, and no correction by row sums is needed.
+// w - zero_point is an integer that bf16 (f16) holds exactly, so the operand of the MMAs is exact.  bf16: a lower
+// byte u under a zero upper byte is the number u * 2^-133 (the step from subnormal to normal numbers included), so
+// one LOP3 and one packed FMA make (w - zero_point) / 64 of two nibbles, low ones or high ones where they stand
+// (u * 2^-133 * 2^127, or * 2^123, less (8 for s4 + zero_point) / 64); the 64 rides on the scale.  f16: a nibble
+// under 0x64 is 1024 + u (or 1024 + 16 u), and a packed subtraction (or FMA) takes the rest off.  The sums of a
+// K-group are exact products added in f32, and the group's scale multiplies the finished group sum:
+// tot += scale * sum, in f32 registers of the epilogue.  Nothing is rounded to 16 bits before dst, and no
+// correction by row sums is needed.
 //
 // As in the other decompression kernels the weights are the A operand, in TENSOR MEMORY (128 dst columns = TMEM
 // lanes), and the src rows the B operand from shared memory, so an epilogue lane owns one dst column.  A tile is
@@ -23,8 +26,8 @@
 // Roles (28 warps): 0 weight tiles by TMA, 1 src tiles by TMA, 2 issues all MMAs, 4-11 converters (two per lane
 // quarter, taking the stages in turn), 12-27 epilogue (four per lane quarter, each a quarter of the rows).  Every mbarrier wait is bounded.
 //
-// Measured on a B200 at K = N = 4096, M = 300, groups of 128, u4 zero-points: 43 us a call (66 us with 64-k stages,
-// a warp-wide issuing loop and eight epilogue warps); the generic kernel,
+// Measured on a B200 at K = N = 4096, M = 300, groups of 128, u4 zero-points: 41 us a call (66 us with 64-k stages,
+// a warp-wide issuing loop and eight epilogue warps; 43 us with a shift and a subtraction per pair); the generic kernel,
 // which such calls took before, 54.3 ms.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -50,6 +53,8 @@ constexpr int ACC_BUFS = 2;
 constexpr int W_BYTES = RK * RT_N / 2; // nibbles as loaded: 64-byte rows
 constexpr int B_BYTES = RT_M * RK * 2; // src rows: two boxes of 64 k
 constexpr int CONV_SETS = 2; // sets of four converter warps, which take the stages in turn
+// a set that could run ahead of the other by more than the ring would take an older phase of a slot for its own
+static_assert(CONV_SETS <= STAGES, "barrier parity");
 constexpr int R_CONV_WARPS = 4 * CONV_SETS, R_EPI_WARPS = 16;
 constexpr int EPI_PIECES = RT_M / 16 / (R_EPI_WARPS / 4); // 16-row pieces of the accumulator per epilogue warp
 constexpr int R_CONV0 = 4, R_EPI0 = R_CONV0 + R_CONV_WARPS;
@@ -85,9 +90,9 @@ __device__ __forceinline__ uint32_t perm(uint32_t a, uint32_t b, uint32_t sel) {
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
     return r;
 }
-__device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
+__device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
 __device__ __forceinline__ uint32_t sub_f16x2(uint32_t a, uint32_t b) {
@@ -331,14 +336,14 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         }
         const int kstages = in_reg(p.kstages), ksteps = in_reg(p.ksteps), group_steps = in_reg(p.group_steps);
         const int zp_mode = in_reg(p.zp_mode), zp_dt = in_reg(a.wei_zp.dt);
-        const uint32_t magic = (uint32_t)in_reg(F16 ? (p.sgn4 ? 0x64086408 : 0x64006400) : (p.sgn4 ? 0x43084308 : 0x43004300));
-        const uint32_t magic_hi = (uint32_t)in_reg(p.sgn4 ? 0x64806480 : 0x64006400); // f16, nibble in place: 1024 + 16 u
+        const uint32_t magic = (uint32_t)in_reg(F16 ? (p.sgn4 ? 0x64086408 : 0x64006400) : (p.sgn4 ? 0x00080008 : 0));
+        const uint32_t magic_hi = (uint32_t)in_reg((F16 ? 0x64006400 : 0) | (p.sgn4 ? 0x00800080 : 0)); // the high nibble in its place
         const int base_off = in_reg(p.sgn4 ? 8 : 0);
         const int zt = zp_mode == 2 ? load_int(zp_dt, a.wei_zp.ptr, 0) : 0;
         // offsets of the four columns, as packed pairs: what the packed subtraction (or the f16 fma) takes
         uint32_t o2[4];
-        // (v = zero-point + 8 for s4 as a 16-bit float 2^e + v, in units of the last place, which halve below 2^e;
-        // 8-bit zero-points, f16 only, go through a conversion)
+        // v = zero-point + 8 for s4.  bf16: -v / 64.  f16: 1024 + v in units of the last place (half as large below
+        // 1024), or -(64 + v); 8-bit zero-points go through a conversion.
         const bool zp4 = zp_mode == 0 || zp_dt == DT_U4 || zp_dt == DT_S4;
         auto set_offsets = [&](uint32_t raw) {
 #pragma unroll
@@ -346,7 +351,7 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                 const int v = base_off + (zp_mode == 1 ? zp_of(zp_dt, raw, c) : zt);
                 const int u = v + min(v, 0);
                 uint32_t b;
-                if (!F16) b = 0x4300u + u;
+                if (!F16) b = __float_as_uint((float)v * -0.015625f) >> 16; // exact: at most six bits
                 else if (zp4) b = (c & 1) ? 0xD400u + 16 * u : 0x6400u + u;
                 else b = __half_as_ushort(__int2half_rn((c & 1) ? -(64 + v) : 1024 + v));
                 o2[c] = b * 0x10001u;
@@ -429,10 +434,10 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                                     o[4 * k + 2] = sub_f16x2(and_xor(x23, 0x000F000Fu, magic), ol);
                                     o[4 * k + 3] = fma_f16x2(and_xor(x23, 0x00F000F0u, magic_hi), 0x2C002C00u, oh);
                                 } else {
-                                    o[4 * k + 0] = sub_bf16x2(and_xor(x01, 0x000F000Fu, magic), ol);
-                                    o[4 * k + 1] = sub_bf16x2(and_xor(x01 >> 4, 0x000F000Fu, magic), oh);
-                                    o[4 * k + 2] = sub_bf16x2(and_xor(x23, 0x000F000Fu, magic), ol);
-                                    o[4 * k + 3] = sub_bf16x2(and_xor(x23 >> 4, 0x000F000Fu, magic), oh);
+                                    o[4 * k + 0] = fma_bf16x2(and_xor(x01, 0x000F000Fu, magic), 0x7F007F00u, ol);
+                                    o[4 * k + 1] = fma_bf16x2(and_xor(x01, 0x00F000F0u, magic_hi), 0x7D007D00u, oh);
+                                    o[4 * k + 2] = fma_bf16x2(and_xor(x23, 0x000F000Fu, magic), 0x7F007F00u, ol);
+                                    o[4 * k + 3] = fma_bf16x2(and_xor(x23, 0x00F000F0u, magic_hi), 0x7D007D00u, oh);
                                 }
                             }
                             st_16x128b_x8(slot + ((uint32_t)(16 * h) << 16) + 32 * half, o);
@@ -501,7 +506,7 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                 for (int i = 0; i < 2; ++i) nxt[i] = raw_scale(g0 + 2 + i);
 #pragma unroll 1
                 for (int i = 0; i < 2 && g0 + i < groups; ++i) {
-                const float sc = scale_of(i == 0 ? cur[0] : cur[1]);
+                const float sc = scale_of(i == 0 ? cur[0] : cur[1]) * (F16 ? 1.f : 64.f); // a power of two: exact
                 const uint64_t sc2 = pack2(__float_as_uint(sc), __float_as_uint(sc));
                 if (!warp_wait(&acc_full[buf], pacc)) { ok = false; break; }
                 ptx::tc_fence_after_sync();

@@ -204,6 +204,8 @@ GROUPED_TC_CASES = {
     "all_in_one": lambda: W.moe_grouped(70, 192, 256, 4, sizes=[0, 0, 70, 0]),
     "several_row_blocks": lambda: W.moe_grouped(700, 128, 256, 3, sizes=[513, 1, 186]),
     "tails_n_k": lambda: W.moe_grouped(50, 200, 176, 3, sizes=[16, 33, 1]),
+    "equal_row_blocks": lambda: W.moe_grouped(626, 640, 128, 3, sizes=[208, 209, 209]),
+    "odd_k_slots": lambda: W.moe_grouped(130, 1088, 256, 2, sizes=[129, 1]),
     "zipf": lambda: W.moe_grouped(1024, 512, 384, 16),
 }
 
