@@ -331,7 +331,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     // share a few weight column blocks and sweep the whole src once per block.
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < num_tiles && !*abort_flag; tile += gridDim.x) {
                 const int m0 = (tile % tp.num_m_tiles) * BT_M;
@@ -350,7 +350,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // (an elected thread: an MMA then takes about 12 cycles to issue; under a predicate computed from the lane
+        // index, which the hardware cannot know to be one lane, about 115 - nearly twice what a 128-row MMA runs)
+        if (ptx::elect_one()) {
             uint32_t it = 0, acc_it = 0;
             for (int tile = blockIdx.x; tile < num_tiles && !*abort_flag; tile += gridDim.x, ++acc_it) {
                 const int as = acc_it % ACC_STAGES;
@@ -681,10 +683,16 @@ int launch_gemm_tc(const MatmulArgs &a_in, void *scratch, int sm_count, cudaStre
     }
     tp.after_prekernel = tp.colsum != nullptr || tp.rowsum != nullptr;
 
-    // 256 dst rows per tile unless that leaves SMs without work
+    const bool chain = a.n_po > 0 || (a.bias && a.bias_sm != 0); // a bias varying along M rides the generic tail
+    // 256 dst rows per tile unless that leaves SMs without work; 64 when even tiles of 128 rows leave more than
+    // half of them idle, or for at most 64 rows (less src to load, and room for more stages in flight); kernels
+    // with a post-op chain, twelve of them, have no third tile size.  (int8, 17 rows, 4096 x 11008: 24.5 us with
+    // 128-row tiles and a lane-index predicate on the issuing thread, 20.5 with 64 rows and an elected one.)
     const int64_t tiles256 = (int64_t)tp.num_n_tiles * ((a.M + 255) / 256);
+    const int64_t tiles128 = (int64_t)tp.num_n_tiles * ((a.M + 127) / 128);
     const bool tall = a.M > 128 && tiles256 >= sm_count / 2;
-    const int BT_M = tall ? 256 : 128;
+    const bool flat = !tall && !chain && (a.M <= 64 || 2 * tiles128 <= sm_count);
+    const int BT_M = tall ? 256 : flat ? 64 : 128;
     tp.num_m_tiles = (int)((a.M + BT_M - 1) / BT_M);
 
     CUtensorMap mw, ms;
@@ -706,7 +714,6 @@ int launch_gemm_tc(const MatmulArgs &a_in, void *scratch, int sm_count, cudaStre
         cfmt = ptx::CFMT_F32;
     }
     tp.idesc = ptx::make_idesc(cfmt, wfmt, sfmt, !w_kmajor, false, BT_N, BT_M);
-    const bool chain = a.n_po > 0 || (a.bias && a.bias_sm != 0); // a bias varying along M rides the generic tail
     if (chain && a.peers.count) return 3; // refused when the replication is registered; not reached
     // kernels with a post-op chain are instantiated per dst data type
 #define QMM_TC_CHAIN(KIND, BTM, ST) \
@@ -718,6 +725,7 @@ int launch_gemm_tc(const MatmulArgs &a_in, void *scratch, int sm_count, cudaStre
                                           : launch_cfg<KIND, BTM, ST, true, DT_S32>(mw, ms, a, tp, sm_count, st))
 #define QMM_TC_LAUNCH(KIND) \
     (tall ? (chain ? QMM_TC_CHAIN(KIND, 256, 4) : launch_cfg<KIND, 256, 4, false>(mw, ms, a, tp, sm_count, st)) \
+    : flat ? launch_cfg<KIND, 64, 9, false>(mw, ms, a, tp, sm_count, st) \
           : (chain ? QMM_TC_CHAIN(KIND, 128, 6) : launch_cfg<KIND, 128, 6, false>(mw, ms, a, tp, sm_count, st)))
     return int_path ? QMM_TC_LAUNCH(1) : QMM_TC_LAUNCH(0);
 #undef QMM_TC_LAUNCH
