@@ -269,8 +269,36 @@ __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constan
                               : 0;
     }
     const bool has_ds = a.dst_scale.ptr != nullptr, has_zp = a.dst_zp != nullptr;
+    // s8 / u8 results need the quotient's integer only.  q = d * (1 / scale) lies within 2^-22 |q| of the divided
+    // value (a reciprocal in the normal range, rounded once, and one more rounding), so unless q is that close to
+    // half an integer both round alike; beyond the range both saturate alike.  Everything else (one warp pass in
+    // some twenty for uniform values, NaN, unusable reciprocals) divides.  The divisions of every element took
+    // 65 % of the issue slots while DRAM stood at 47 % (f32 4096 x 14336 -> s8: 71.4 us, now 66.9).
+    const bool by_rcp = (DDT == DT_S8 || DDT == DT_U8) && has_ds && !has_zp;
+    float rc[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        rc[e] = by_rcp ? __frcp_rn(ds[e]) : 0.f;
+        if (!(fabsf(rc[e]) >= 1.17549435e-38f && fabsf(rc[e]) <= 3.0e38f)) rc[e] = __int_as_float(0x7fffffff); // NaN
+    }
     auto convert = [&](const float (&f)[4], const int (&iv)[4], int64_t off) {
         float out[4];
+        if (by_rcp) {
+            float worst = 0.f; // largest distance of a quotient from its integer
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float diff = dt_is_int(SDT) ? (float)(iv[e] - zps[e]) : __fsub_rn(f[e], (float)zps[e]);
+                out[e] = __fmul_rn(__fmul_rn(ss[e], diff), rc[e]);
+                // (inside +-300 the sum with 1.5 * 2^23 leaves the nearest integer; results beyond saturate)
+                const float q = fminf(fmaxf(out[e], -300.f), 300.f);
+                const float t = fabsf(q - ((q + 12582912.f) - 12582912.f));
+                worst = out[e] == out[e] ? fmaxf(worst, t) : 1.f;
+            }
+            if (worst < 0.4998f) {
+                store4(DDT, out, a.dst, off);
+                return;
+            }
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float diff = dt_is_int(SDT) ? (float)(iv[e] - zps[e]) : __fsub_rn(f[e], (float)zps[e]);

@@ -56,6 +56,26 @@ def test_cuda_reorder_matches_oracle(gpu, name):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dst_dt", [W.S8, W.U8])
+def test_cuda_reorder_rounds_quotients_like_the_division(gpu, dst_dt):
+    """Columns whose scaled values lie on half integers and one unit beside them, saturate, or have a scale whose
+    reciprocal is not a normal number: the 8-bit results are those of the IEEE division (element-wise, no tolerance)."""
+    from onednn_b200.runner import run_reorder
+    eng, strm = gpu
+    r = np.random.Generator(np.random.PCG64(79))
+    sc = np.concatenate([r.uniform(1e-4, 1e-2, 56), [1.0, 3.0, 1e-30, 1e30, 1e38, 3e38, 1e-39, 2e-45]]).astype(np.float32)
+    half = (np.arange(-140, 140) + 0.5).astype(np.float32)
+    with np.errstate(over="ignore"):  # the largest scales: infinities are among the cases
+        x = (half[:, None] * sc[None, :]).astype(np.float32)
+    rows = [x, np.nextafter(x, np.float32(np.inf)), np.nextafter(x, np.float32(-np.inf)),
+            np.full((1, sc.size), 1e30, np.float32), np.full((1, sc.size), -np.inf, np.float32)]
+    x = np.concatenate(rows)
+    ro = W.Reorder("ties", W.QTensor(x, W.F32, x.shape), dst_dt, quant={"dst_scale": W.Quant(sc.reshape(1, -1), W.F32, 2)})
+    got, _ = run_reorder(ro, eng, strm)
+    assert np.array_equal(got, O.run_port_reorder(ro))
+
+
+@pytest.mark.gpu
 def test_cuda_reorder_feeds_the_matmul(gpu):
     """The canonical flow: quantize f32 weights to s8 with per-column scales by a reorder, then
     run the int8 matmul with the same scales; compared with the oracle run on the oracle's
