@@ -284,9 +284,9 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
 
     if (warp == PRODUCER_WARP) {
         // ------------------------------------------------ TMA producer
-        // (the whole warp walks the loop, one elected thread issues: see elect_one)
-        {
-            const bool issue = lane == 0;
+        // (one elected thread runs the whole loop: see elect_one)
+        if (ptx::elect_one()) {
+            constexpr bool issue = true;
             uint32_t it = 0;
             int s = 0;
             uint32_t ph = 1; // parity of the empty barrier's previous phase: a fresh barrier passes
@@ -295,15 +295,14 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                 const Segment sg = segment_at(L, L1, p.kstages);
                 const int xbyte = sg.tile * C::ROW_BYTES;
                 for (int st = sg.sb; st < sg.se; ++st, ++it) {
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty[s], ph))) { ok = false; break; }
+                    if (!(ptx::mbar_wait(&empty[s], ph))) { ok = false; break; }
                     uint8_t *sw = smem + s * W_STAGE_BYTES;
-                    if (ptx::elect_one()) {
+                    {
                         ptx::mbar_arrive_expect_tx(&full[s], W_STAGE_BYTES);
 #pragma unroll
                         for (int b = 0; b < C::W_BOXES; ++b)
                             ptx::tma_load_2d(sw + b * (C::KS * 128), &tmW, &full[s], xbyte + b * 128, st * C::KS);
                     }
-                    __syncwarp();
                     if (issue) WT_TRACE(0, it);
                     if (++s == C::STAGES) { s = 0; ph ^= 1; }
                 }
@@ -314,8 +313,8 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
     } else if (warp == PARAM_WARP) {
         // ------------------------------------------------ second producer: src tile, step sums and,
         // where a group piece can begin in the stage, the scale / zero-point rows of the stage's groups
-        {
-            const bool issue = lane == 0;
+        if (ptx::elect_one()) {
+            constexpr bool issue = true;
             int s = 0;
             uint32_t ph = 1;
             [[maybe_unused]] uint32_t pit = 0;
@@ -330,10 +329,10 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                 int first = sg.sb * C::SPS;
                 int gi0 = first / p.group_steps, r = first - gi0 * p.group_steps; // group of the stage's first step, steps into it
                 for (int st = sg.sb; st < sg.se; ++st) {
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&s_empty[s], ph))) { ok = false; break; }
+                    if (!(ptx::mbar_wait(&s_empty[s], ph))) { ok = false; break; }
                     uint8_t *ss = smem + C::S_RING_OFFSET + s * p.s_stage_bytes;
                     const bool params = st == sg.sb || r == 0 || p.group_steps - r < C::SPS;
-                    if (ptx::elect_one()) {
+                    {
                         ptx::mbar_arrive_expect_tx(&s_full[s], base_tx + (params ? par_tx : 0u));
 #pragma unroll
                         for (int b = 0; b < C::S_BOXES; ++b)
@@ -344,7 +343,6 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                             if (p.zp_mode == 1) ptx::tma_load_2d(ss + p.off_zp, &tmZp, &s_full[s], xpair, gi0);
                         }
                     }
-                    __syncwarp();
                     if (issue) WT_TRACE(12, pit);
                     ++pit;
                     first += C::SPS;
@@ -361,9 +359,10 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
         // [i * NBLK / MMA_WARPS, (i + 1) * NBLK / MMA_WARPS) of every k16 step; all walk the same barriers
         constexpr int JB = NBLK / C::MMA_WARPS;
         const int j0 = (warp - MMA_WARP0) * JB;
-        // (the whole warp walks the loop, one elected thread issues)
-        {
-            const bool issue = lane == 0;
+        // (one elected thread of the warp runs the whole loop; M = 1, 8192 x 28672: 50.8 us with warp-wide loops and
+        // an election per stage, 49.9 so)
+        if (ptx::elect_one()) {
+            constexpr bool issue = true;
             uint32_t it = 0, gc = 0;
             int s = 0, as = 0;
             uint32_t aph = 0; // parity of the operand-stage barriers
@@ -376,7 +375,7 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                 bool fresh = true; // the next MMA starts a group piece
                 for (int st = sg.sb; st < sg.se && !failed; ++st, ++it) {
                     // (the converters have seen the stage's src tile arrive before they arrive here)
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&a_full[as], aph))) { failed = true; break; }
+                    if (!(ptx::mbar_wait(&a_full[as], aph))) { failed = true; break; }
                     if (j0 == 0 && issue) WT_TRACE(5, it);
                     ptx::tc_fence_after_sync();
                     const uint32_t ss = ptx::smem_u32(smem + C::S_RING_OFFSET + s * p.s_stage_bytes);
@@ -388,7 +387,7 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                     if (nst == C::SPS && kpos + C::SPS <= gend && !WT_ABLATE(1)) {
                         const uint32_t buf = gc & 1;
                         if (fresh) {
-                            if (!__all_sync(0xffffffffu, ptx::mbar_wait(&acc_empty[buf], ((gc >> 1) & 1) ^ 1))) { failed = true; break; }
+                            if (!(ptx::mbar_wait(&acc_empty[buf], ((gc >> 1) & 1) ^ 1))) { failed = true; break; }
                             ptx::tc_fence_after_sync();
                         }
                         if (j0 == 0 && issue) WT_TRACE(6, it);
@@ -397,7 +396,7 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                         const uint64_t bd0 = ptx::smem_desc_sw128(ss, 0, 1024);
                         kpos += C::SPS;
                         const bool piece_done = kpos == gend;
-                        if (ptx::elect_one()) { // one elected thread issues (see elect_one)
+                        {
 #pragma unroll
                             for (int q = 0; q < C::SPS; ++q) {
                                 // the start-address field counts 16-byte units: later steps add a constant to it
@@ -410,7 +409,6 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                             ptx::tc_commit(&a_empty[as]); // the operand stage may be rewritten once these MMAs have read it
                             ptx::tc_commit(&s_empty[s]); // ... and the stage's src tile has been read
                         }
-                        __syncwarp();
                         fresh = false;
                         if (piece_done) {
                             ++gc;
@@ -422,7 +420,7 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                         for (int q = 0; q < nst; ++q, ++kpos) {
                             const uint32_t buf = gc & 1;
                             if (fresh) {
-                                if (!__all_sync(0xffffffffu, ptx::mbar_wait(&acc_empty[buf], ((gc >> 1) & 1) ^ 1))) { failed = true; break; }
+                                if (!(ptx::mbar_wait(&acc_empty[buf], ((gc >> 1) & 1) ^ 1))) { failed = true; break; }
                                 ptx::tc_fence_after_sync();
                             }
                             const uint64_t bd = ptx::smem_desc_sw128(ss + (q >> 2) * (C::MP * 128) + (q & 3) * 32, 0, 1024);
