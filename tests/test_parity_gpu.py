@@ -85,6 +85,9 @@ TC_CASES = {
     "fp8_wide": lambda: W.fp8_prefill(256, 256, 10240),
     "fp8_ba": lambda: _ba(W.fp8_prefill(128, 384, 256)),
     "fp8_e5m2": lambda: W.fp8_prefill(64, 256, 128, src_dt=W.F8_E5M2, wei_dt=W.F8_E5M2),
+    "int8_rows_64": lambda: W.int8_zp(64, 1296, 272),  # more stages than the ring of the 64-row tiles
+    "int8_rows_65": lambda: W.int8_zp(65, 1296, 272, per_n_scales=True),
+    "fp8_rows_63_wide": lambda: W.fp8_prefill(63, 256, 10240),
     "fp8_mixed": lambda: W.fp8_prefill(64, 256, 128, src_dt=W.F8_E4M3, wei_dt=W.F8_E5M2),
 }
 
