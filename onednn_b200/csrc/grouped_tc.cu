@@ -88,6 +88,18 @@ constexpr int G_PLAN_OFFSET = G_BAR_OFFSET + 512;
 constexpr int G_SMEM_BYTES = G_PLAN_OFFSET + (PLAN_CACHE_GROUPS + 1) * 16 + 1024;
 static_assert(G_SMEM_BYTES <= 227 * 1024, "shared memory");
 
+// Columns of the accumulator that the epilogue reads for a piece of up to 32 rows, `left` rows before the block's
+// end.  What lies past a full block's GT_M columns is live: the other accumulator, which the MMAs may be writing, or
+// an operand slot.  So the last 16 rows are read alone.
+constexpr int piece_columns(int left) { return left <= 16 ? 16 : 32; }
+constexpr bool pieces_stay_in_the_accumulator() {
+    for (int rows = 1; rows <= GT_M; ++rows)
+        for (int c = 0; c < rows; c += 32)
+            if (c + piece_columns(rows - c) > GT_M) return false;
+    return true;
+}
+static_assert(pieces_stay_in_the_accumulator(), "the epilogue reads tensor memory that other warps write");
+
 // plan[0] = {total tiles, groups, 0, 0}; plan[1 + g] = {first src row, first dst row, rows, first tile}
 struct Tile {
     int g, n0, m0, rows, src_row, dst_row;
@@ -416,7 +428,15 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 #pragma unroll 1
             for (int cidx = 0; cidx < chunks; ++cidx) {
                 uint32_t r[32];
-                ptx::tmem_ld_32x32(tmem_base + ((uint32_t)lane_base << 16) + as * GT_M + cidx * 32, r);
+                const uint32_t piece = tmem_base + ((uint32_t)lane_base << 16) + as * GT_M + cidx * 32;
+                if (piece_columns(tl.rows - cidx * 32) == 32) {
+                    ptx::tmem_ld_32x32(piece, r);
+                } else {
+                    uint32_t half[16];
+                    ptx::tmem_ld_32x16(piece, half);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = j < 16 ? half[j] : 0u;
+                }
                 ptx::tmem_ld_wait();
                 if (cidx == chunks - 1) { // accumulator fully read: hand the buffer back
                     ptx::tc_fence_before_sync();

@@ -113,15 +113,6 @@ __device__ __forceinline__ void st_16x128b_x8(uint32_t taddr, const uint32_t (&r
             "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
             : "memory");
 }
-__device__ __forceinline__ void ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr)
-            : "memory");
-}
 __device__ __forceinline__ void mma_ts_16bit(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, bool acc) {
     asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -515,7 +506,7 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                 for (int c = 0; c < EPI_PIECES; ++c) {
                     if (c < cn) {
                         uint32_t v[16];
-                        ld_32x16(acc + 16 * c, v);
+                        ptx::tmem_ld_32x16(acc + 16 * c, v);
                         ptx::tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 8; ++j) fma_f32x2(tot[c][j], sc2, v[2 * j], v[2 * j + 1]);

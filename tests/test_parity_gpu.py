@@ -210,6 +210,8 @@ GROUPED_TC_CASES = {
     "equal_row_blocks": lambda: W.moe_grouped(626, 640, 128, 3, sizes=[208, 209, 209]),
     "odd_k_slots": lambda: W.moe_grouped(130, 1088, 256, 2, sizes=[129, 1]),
     "zipf": lambda: W.moe_grouped(1024, 512, 384, 16),
+    # blocks that end in 16 rows or fewer of a 32-row epilogue piece, several tiles per CTA (both accumulators in use)
+    "full_blocks_both_accumulators": lambda: W.moe_grouped(609, 128, 19200, 3, sizes=[193, 208, 208]),
 }
 
 
@@ -270,9 +272,9 @@ def _moe_bias_gelu():
     return p
 
 
-def _moe_zero_points(zp_dt=W.S8):
+def _moe_zero_points(zp_dt=W.S8, sizes=(150, 0, 249, 1), N=176):
     """Grouped problem with one weight zero-point per (expert, column), several row blocks in one expert."""
-    p = W.moe_grouped(400, 192, 176, 4, sizes=[150, 0, 249, 1])
+    p = W.moe_grouped(sum(sizes), 192, N, len(sizes), sizes=list(sizes))
     r = np.random.Generator(np.random.PCG64(14))
     lo, hi = (0, 9) if zp_dt == W.U8 else (-8, 9)
     z = r.integers(lo, hi, (p.groups, 1, p.N)).astype({W.S8: np.int8, W.U8: np.uint8, W.S32: np.int32}[zp_dt])
@@ -294,6 +296,7 @@ GROUPED_TC_CHAIN_CASES = {
     "zero_points_s8": _moe_zero_points,
     "zero_points_u8": lambda: _moe_zero_points(W.U8),
     "zero_points_s32": lambda: _moe_zero_points(W.S32),
+    "zero_points_full_blocks": lambda: _moe_zero_points(W.S8, (208, 195, 17), 9600),
 }
 
 
