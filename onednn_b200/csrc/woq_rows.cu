@@ -7,7 +7,7 @@
 // w - zero_point is an integer that bf16 (f16) holds exactly, so the operand of the MMAs is exact.  bf16: a lower
 // byte u under a zero upper byte is the number u * 2^-133 (the step from subnormal to normal numbers included), so
 // one LOP3 and one packed FMA make (w - zero_point) / 64 of two nibbles, low ones or high ones where they stand
-// (u * 2^-133 * 2^127, or * 2^123, less (8 for s4 + zero_point) / 64); the 64 rides on the scale.  f16: a nibble
+// (u * 2^-133 * 2^127, or * 2^123, less (8 for s4 + zero_point) / 64); the group sum is multiplied by the 64.  f16: a nibble
 // under 0x64 is 1024 + u (or 1024 + 16 u), and a packed subtraction (or FMA) takes the rest off.  The sums of a
 // K-group are exact products added in f32, and the group's scale multiplies the finished group sum:
 // tot += scale * sum, in f32 registers of the epilogue.  Nothing is rounded to 16 bits before dst, and no
@@ -126,8 +126,13 @@ __device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
     return r;
 }
 // two fused multiply-adds: d = sc * {v0, v1} + d
-__device__ __forceinline__ void fma_f32x2(uint64_t &d, uint64_t sc, uint32_t v0, uint32_t v1) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(sc), "l"(pack2(v0, v1)));
+__device__ __forceinline__ void fma_f32x2(uint64_t &d, uint64_t sc, uint64_t v) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(sc), "l"(v));
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 // bias, post-ops, dst scale, any dst type: rare and large, out of line
 __device__ __noinline__ void finish_store_general(const MatmulArgs &a, float d, int64_t m, int64_t n) {
@@ -497,7 +502,7 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                 for (int i = 0; i < 2; ++i) nxt[i] = raw_scale(g0 + 2 + i);
 #pragma unroll 1
                 for (int i = 0; i < 2 && g0 + i < groups; ++i) {
-                const float sc = scale_of(i == 0 ? cur[0] : cur[1]) * (F16 ? 1.f : 64.f); // a power of two: exact
+                const float sc = scale_of(i == 0 ? cur[0] : cur[1]);
                 const uint64_t sc2 = pack2(__float_as_uint(sc), __float_as_uint(sc));
                 if (!warp_wait(&acc_full[buf], pacc)) { ok = false; break; }
                 ptx::tc_fence_after_sync();
@@ -509,7 +514,13 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                         ptx::tmem_ld_32x16(acc + 16 * c, v);
                         ptx::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) fma_f32x2(tot[c][j], sc2, v[2 * j], v[2 * j + 1]);
+                        for (int j = 0; j < 8; ++j) {
+                            uint64_t sum = pack2(v[2 * j], v[2 * j + 1]);
+                            // bf16: the operand was (w - zero_point) / 64; the 64 goes on the sum (a scale above
+                            // 2^122 would overflow), exactly
+                            if (!F16) sum = mul_f32x2(sum, 0x4280000042800000ull);
+                            fma_f32x2(tot[c][j], sc2, sum);
+                        }
                     }
                 }
                 ptx::tc_fence_before_sync();

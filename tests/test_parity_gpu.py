@@ -171,6 +171,16 @@ def test_woq_decode_matches_oracle(gpu, name, kernel):
     assert np.array_equal(got, got2)
 
 
+def _large_scales():
+    """f32 scales just below the type's range against src values as far below 1: all products and sums are finite."""
+    p = W.int4_decode(40, 256, 160, with_zp=False, dst_dt=W.F32)
+    r = np.random.Generator(np.random.PCG64(11))
+    p.src = W.QTensor(W.f32_to_bf16(W.bf16_to_f32(p.src.data) * np.float32(2.0 ** -100)), W.BF16, p.src.dims)
+    q = p.quant["wei_scale"]
+    p.quant["wei_scale"] = W.Quant((r.uniform(1.0, 1.99, q.data.shape) * 2.0 ** 123).astype(np.float32), W.F32, 3, q.groups)
+    return p
+
+
 WOQ_ROWS_CASES = {
     "m33_one_tile": lambda: W.int4_decode(33, 256, 128),
     "m129_two_tiles": lambda: W.int4_decode(129, 512, 288),
@@ -184,6 +194,7 @@ WOQ_ROWS_CASES = {
     "per_n_scale": lambda: _per_n_scale(W.int4_decode(36, 384, 256)),
     "bias_relu": lambda: _with_bias_relu(W.int4_decode(48, 512, 256)),
     "more_tiles_than_sms": lambda: W.int4_decode(140, 192, 9632, group=64),
+    "large_f32_scales": _large_scales,
 }
 
 
