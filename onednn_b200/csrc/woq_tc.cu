@@ -56,8 +56,8 @@ namespace qmm {
 
 namespace {
 
-// A warp issues a tcgen05.mma about every 40 to 65 cycles, whatever its size; issuing warps add up,
-// and the MMAs of this kernel are small (N = 16 or 32), so every 128-column block of a tile has an
+// A warp that walks its loop together issues a tcgen05.mma about every 40 to 65 cycles, whatever its size; issuing
+// warps add up, and the MMAs of this kernel are small (N = 16 or 32), so every 128-column block of a tile has an
 // issuer warp of its own where the registers allow it (WtCfg::MMA_WARPS).
 constexpr int CONV_WARPS = 8, EPI_WARPS = 4;
 // A thread issues a stage of TMA copies in a few hundred cycles (a wait, an expect-tx and about 70
@@ -76,6 +76,12 @@ struct WtCfg {
     // register file then gives 96 - enough for the 8-row epilogue only.
     static constexpr int MMA_WARPS = MR == 8 ? NBLK : 2;
     static constexpr int THREADS = 32 * (CONV_WARPS + EPI_WARPS + 2 + MMA_WARPS);
+    // An MMA issuer runs in one elected thread, or in its whole warp with an election per stage (elect_one picks the
+    // same lane every time, so a commit covers the MMAs of earlier elections).  K = 8192, N = 28672, groups of 128,
+    // bf16, us a call, whole warps -> one thread: M = 1 51.3 -> 50.0, M = 8 59.3 -> 58.4, M = 32 84.9 -> 84.8;
+    // M = 9 and 16, the other way round (why is not known): 65.9 -> 66.6, 73.6 -> 74.2.  Producers in single threads
+    // cost at every size (50.0 -> 51.3, 66.6 -> 67.9, 84.8 -> 88.3), so their whole warps walk the loops.
+    static constexpr bool SOLO_MMA = MR != 16;
     static constexpr int NB = 128 * NBLK; // dst columns per tile
     static constexpr int ROW_BYTES = NB / 2; // packed bytes per k-row of a tile: 256 or 128
     static constexpr int KS = W_STAGE_BYTES / ROW_BYTES; // k-rows per stage: 64 or 128
@@ -179,14 +185,19 @@ __device__ __forceinline__ void tmem_st_16x128b_steps(uint32_t taddr, const uint
     }
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] * B[smem], issued by the lane(s) with `issue` set
-__device__ __forceinline__ void mma_ts_f16(bool issue, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, bool acc) {
-    const uint32_t en = acc ? 1u : 0u;
+// D[tmem] (+)= A[tmem] * B[smem], issued by the calling thread
+__device__ __forceinline__ void mma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, bool acc) {
     asm volatile(
-            "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(en), "r"((uint32_t)issue)
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"((uint32_t)acc)
             : "memory");
+}
+// A wait of a role that runs in one thread (SOLO) or in its whole warp
+template <bool SOLO>
+__device__ __forceinline__ bool role_wait(uint64_t *bar, uint32_t parity) {
+    const bool ok = ptx::mbar_wait(bar, parity);
+    return SOLO ? ok : (bool)__all_sync(0xffffffffu, ok);
 }
 template <int N>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
@@ -284,86 +295,79 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
 
     if (warp == PRODUCER_WARP) {
         // ------------------------------------------------ TMA producer
-        // (one elected thread runs the whole loop: see elect_one)
-        if (ptx::elect_one()) {
-            constexpr bool issue = true;
-            uint32_t it = 0;
-            int s = 0;
-            uint32_t ph = 1; // parity of the empty barrier's previous phase: a fresh barrier passes
-            bool ok = true;
-            for (int64_t L = L0; L < L1 && ok && !*abort_flag;) {
-                const Segment sg = segment_at(L, L1, p.kstages);
-                const int xbyte = sg.tile * C::ROW_BYTES;
-                for (int st = sg.sb; st < sg.se; ++st, ++it) {
-                    if (!(ptx::mbar_wait(&empty[s], ph))) { ok = false; break; }
-                    uint8_t *sw = smem + s * W_STAGE_BYTES;
-                    {
-                        ptx::mbar_arrive_expect_tx(&full[s], W_STAGE_BYTES);
+        // (the whole warp walks the loop, one elected thread issues: see WtCfg::SOLO_MMA; so does the second producer's)
+        [[maybe_unused]] uint32_t it = 0;
+        int s = 0;
+        uint32_t ph = 1; // parity of the empty barrier's previous phase: a fresh barrier passes
+        bool ok = true;
+        for (int64_t L = L0; L < L1 && ok && !*abort_flag;) {
+            const Segment sg = segment_at(L, L1, p.kstages);
+            const int xbyte = sg.tile * C::ROW_BYTES;
+            for (int st = sg.sb; st < sg.se; ++st, ++it) {
+                if (!role_wait<false>(&empty[s], ph)) { ok = false; break; }
+                uint8_t *sw = smem + s * W_STAGE_BYTES;
+                if (ptx::elect_one()) {
+                    ptx::mbar_arrive_expect_tx(&full[s], W_STAGE_BYTES);
 #pragma unroll
-                        for (int b = 0; b < C::W_BOXES; ++b)
-                            ptx::tma_load_2d(sw + b * (C::KS * 128), &tmW, &full[s], xbyte + b * 128, st * C::KS);
-                    }
-                    if (issue) WT_TRACE(0, it);
-                    if (++s == C::STAGES) { s = 0; ph ^= 1; }
+                    for (int b = 0; b < C::W_BOXES; ++b)
+                        ptx::tma_load_2d(sw + b * (C::KS * 128), &tmW, &full[s], xbyte + b * 128, st * C::KS);
+                    WT_TRACE(0, it);
                 }
-                L += sg.se - sg.sb;
+                __syncwarp();
+                if (++s == C::STAGES) { s = 0; ph ^= 1; }
             }
-            if (!ok && issue) { *abort_flag = 1; atomicExch(a.status, 5); }
+            L += sg.se - sg.sb;
         }
+        if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp == PARAM_WARP) {
         // ------------------------------------------------ second producer: src tile, step sums and,
         // where a group piece can begin in the stage, the scale / zero-point rows of the stage's groups
-        if (ptx::elect_one()) {
-            constexpr bool issue = true;
-            int s = 0;
-            uint32_t ph = 1;
-            [[maybe_unused]] uint32_t pit = 0;
-            const uint32_t base_tx = C::S_BYTES + C::SUMS_BYTES;
-            const uint32_t par_tx = p.sc_box_bytes + (p.zp_mode == 1 ? p.zp_box_bytes : 0);
-            // the step sums come from the pre-kernel, of which this kernel is the programmatic dependent
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            bool ok = true;
-            for (int64_t L = L0; L < L1 && ok && !*abort_flag;) {
-                const Segment sg = segment_at(L, L1, p.kstages);
-                const int xpair = sg.tile * (C::NB / 2); // parameter maps count pairs of columns
-                int first = sg.sb * C::SPS;
-                int gi0 = first / p.group_steps, r = first - gi0 * p.group_steps; // group of the stage's first step, steps into it
-                for (int st = sg.sb; st < sg.se; ++st) {
-                    if (!(ptx::mbar_wait(&s_empty[s], ph))) { ok = false; break; }
-                    uint8_t *ss = smem + C::S_RING_OFFSET + s * p.s_stage_bytes;
-                    const bool params = st == sg.sb || r == 0 || p.group_steps - r < C::SPS;
-                    {
-                        ptx::mbar_arrive_expect_tx(&s_full[s], base_tx + (params ? par_tx : 0u));
+        int s = 0;
+        uint32_t ph = 1;
+        [[maybe_unused]] uint32_t pit = 0;
+        const uint32_t base_tx = C::S_BYTES + C::SUMS_BYTES;
+        const uint32_t par_tx = p.sc_box_bytes + (p.zp_mode == 1 ? p.zp_box_bytes : 0);
+        // the step sums come from the pre-kernel, of which this kernel is the programmatic dependent
+        ptx::grid_dependency_wait();
+        bool ok = true;
+        for (int64_t L = L0; L < L1 && ok && !*abort_flag;) {
+            const Segment sg = segment_at(L, L1, p.kstages);
+            const int xpair = sg.tile * (C::NB / 2); // parameter maps count pairs of columns
+            int first = sg.sb * C::SPS;
+            int gi0 = first / p.group_steps, r = first - gi0 * p.group_steps; // group of the stage's first step, steps into it
+            for (int st = sg.sb; st < sg.se; ++st, ++pit) {
+                if (!role_wait<false>(&s_empty[s], ph)) { ok = false; break; }
+                uint8_t *ss = smem + C::S_RING_OFFSET + s * p.s_stage_bytes;
+                const bool params = st == sg.sb || r == 0 || p.group_steps - r < C::SPS;
+                if (ptx::elect_one()) {
+                    ptx::mbar_arrive_expect_tx(&s_full[s], base_tx + (params ? par_tx : 0u));
 #pragma unroll
-                        for (int b = 0; b < C::S_BOXES; ++b)
-                            ptx::tma_load_2d(ss + b * (C::MP * 128), &tmS, &s_full[s], st * C::KS + b * 64, 0);
-                        ptx::tma_load_2d(ss + p.off_sums, &tmSums, &s_full[s], 0, first);
-                        if (params) {
-                            ptx::tma_load_2d(ss + p.off_sc, &tmSc, &s_full[s], xpair, gi0);
-                            if (p.zp_mode == 1) ptx::tma_load_2d(ss + p.off_zp, &tmZp, &s_full[s], xpair, gi0);
-                        }
+                    for (int b = 0; b < C::S_BOXES; ++b)
+                        ptx::tma_load_2d(ss + b * (C::MP * 128), &tmS, &s_full[s], st * C::KS + b * 64, 0);
+                    ptx::tma_load_2d(ss + p.off_sums, &tmSums, &s_full[s], 0, first);
+                    if (params) {
+                        ptx::tma_load_2d(ss + p.off_sc, &tmSc, &s_full[s], xpair, gi0);
+                        if (p.zp_mode == 1) ptx::tma_load_2d(ss + p.off_zp, &tmZp, &s_full[s], xpair, gi0);
                     }
-                    if (issue) WT_TRACE(12, pit);
-                    ++pit;
-                    first += C::SPS;
-                    r += C::SPS;
-                    while (r >= p.group_steps) { r -= p.group_steps; ++gi0; }
-                    if (++s == p.s_stages) { s = 0; ph ^= 1; }
+                    WT_TRACE(12, pit);
                 }
-                L += sg.se - sg.sb;
+                __syncwarp();
+                first += C::SPS;
+                r += C::SPS;
+                while (r >= p.group_steps) { r -= p.group_steps; ++gi0; }
+                if (++s == p.s_stages) { s = 0; ph ^= 1; }
             }
-            if (!ok && issue) { *abort_flag = 1; atomicExch(a.status, 5); }
+            L += sg.se - sg.sb;
         }
+        if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
     } else if (warp >= MMA_WARP0) {
         // ------------------------------------------------ MMA issuers: warp i takes the column blocks
         // [i * NBLK / MMA_WARPS, (i + 1) * NBLK / MMA_WARPS) of every k16 step; all walk the same barriers
         constexpr int JB = NBLK / C::MMA_WARPS;
         const int j0 = (warp - MMA_WARP0) * JB;
-        // (one elected thread of the warp runs the whole loop; M = 1, 8192 x 28672: 50.8 us with warp-wide loops and
-        // an election per stage, 49.9 so)
-        if (ptx::elect_one()) {
-            constexpr bool issue = true;
-            uint32_t it = 0, gc = 0;
+        if (!C::SOLO_MMA || ptx::elect_one()) {
+            [[maybe_unused]] uint32_t it = 0;
+            uint32_t gc = 0;
             int s = 0, as = 0;
             uint32_t aph = 0; // parity of the operand-stage barriers
             bool failed = false;
@@ -375,39 +379,37 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                 bool fresh = true; // the next MMA starts a group piece
                 for (int st = sg.sb; st < sg.se && !failed; ++st, ++it) {
                     // (the converters have seen the stage's src tile arrive before they arrive here)
-                    if (!(ptx::mbar_wait(&a_full[as], aph))) { failed = true; break; }
-                    if (j0 == 0 && issue) WT_TRACE(5, it);
+                    if (!role_wait<C::SOLO_MMA>(&a_full[as], aph)) { failed = true; break; }
                     ptx::tc_fence_after_sync();
                     const uint32_t ss = ptx::smem_u32(smem + C::S_RING_OFFSET + s * p.s_stage_bytes);
-                    const uint32_t ast = tmem_base + C::A_COL0 + as * C::A_STAGE_COLS;
+                    const uint32_t ast = tmem_base + C::A_COL0 + as * C::A_STAGE_COLS + j0 * (8 * C::SPS);
                     const int nst = min(C::SPS, kend - st * C::SPS);
-                    bool committed = false; // the straight-line path commits inside its elected branch
                     // The common stage - whole, inside one group piece - is straight-line code:
                     // descriptor and tensor-memory addresses are a base plus compile-time offsets.
                     if (nst == C::SPS && kpos + C::SPS <= gend && !WT_ABLATE(1)) {
                         const uint32_t buf = gc & 1;
                         if (fresh) {
-                            if (!(ptx::mbar_wait(&acc_empty[buf], ((gc >> 1) & 1) ^ 1))) { failed = true; break; }
+                            if (!role_wait<C::SOLO_MMA>(&acc_empty[buf], ((gc >> 1) & 1) ^ 1)) { failed = true; break; }
                             ptx::tc_fence_after_sync();
                         }
-                        if (j0 == 0 && issue) WT_TRACE(6, it);
                         const uint32_t accb = tmem_base + buf * C::ACC_COLS + j0 * C::MP;
-                        const uint32_t astb = ast + j0 * (8 * C::SPS);
                         const uint64_t bd0 = ptx::smem_desc_sw128(ss, 0, 1024);
                         kpos += C::SPS;
                         const bool piece_done = kpos == gend;
-                        {
+                        if (C::SOLO_MMA || ptx::elect_one()) {
+                            if (j0 == 0) WT_TRACE(6, it);
 #pragma unroll
                             for (int q = 0; q < C::SPS; ++q) {
                                 // the start-address field counts 16-byte units: later steps add a constant to it
                                 const uint64_t bd = bd0 + (uint64_t)(((q >> 2) * (C::MP * 128) + (q & 3) * 32) >> 4);
 #pragma unroll
                                 for (int j = 0; j < JB; ++j)
-                                    mma_ts_f16(true, accb + j * C::MP, astb + j * (8 * C::SPS) + 8 * q, bd, p.idesc, q > 0 || !fresh);
+                                    mma_ts_f16(accb + j * C::MP, ast + j * (8 * C::SPS) + 8 * q, bd, p.idesc, q > 0 || !fresh);
                             }
                             if (piece_done) ptx::tc_commit(&acc_full[buf]); // group piece complete
                             ptx::tc_commit(&a_empty[as]); // the operand stage may be rewritten once these MMAs have read it
                             ptx::tc_commit(&s_empty[s]); // ... and the stage's src tile has been read
+                            if (j0 == 0) WT_TRACE(1, it);
                         }
                         fresh = false;
                         if (piece_done) {
@@ -415,42 +417,44 @@ woq_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ C
                             fresh = true;
                             gend = min(kend, gend + p.group_steps);
                         }
-                        committed = true;
                     } else {
                         for (int q = 0; q < nst; ++q, ++kpos) {
                             const uint32_t buf = gc & 1;
                             if (fresh) {
-                                if (!(ptx::mbar_wait(&acc_empty[buf], ((gc >> 1) & 1) ^ 1))) { failed = true; break; }
+                                if (!role_wait<C::SOLO_MMA>(&acc_empty[buf], ((gc >> 1) & 1) ^ 1)) { failed = true; break; }
                                 ptx::tc_fence_after_sync();
                             }
                             const uint64_t bd = ptx::smem_desc_sw128(ss + (q >> 2) * (C::MP * 128) + (q & 3) * 32, 0, 1024);
-                            const uint32_t acc = tmem_base + buf * C::ACC_COLS;
-                            if (!WT_ABLATE(1)) {
+                            const uint32_t accb = tmem_base + buf * C::ACC_COLS + j0 * C::MP;
+                            const bool piece_done = kpos + 1 == gend;
+                            if (C::SOLO_MMA || ptx::elect_one()) {
+                                if (!WT_ABLATE(1)) {
 #pragma unroll
-                                for (int j = 0; j < JB; ++j)
-                                    mma_ts_f16(issue, acc + (j0 + j) * C::MP, ast + (j0 + j) * (8 * C::SPS) + 8 * q, bd, p.idesc, !fresh);
+                                    for (int j = 0; j < JB; ++j)
+                                        mma_ts_f16(accb + j * C::MP, ast + j * (8 * C::SPS) + 8 * q, bd, p.idesc, !fresh);
+                                }
+                                if (piece_done) ptx::tc_commit(&acc_full[buf]);
                             }
                             fresh = false;
-                            if (kpos + 1 == gend) { // group piece complete
-                                ptx::tc_commit_if(issue, &acc_full[buf]);
+                            if (piece_done) {
                                 ++gc;
                                 fresh = true;
                                 gend = min(kend, gend + p.group_steps);
                             }
                         }
+                        if (failed) break;
+                        if (C::SOLO_MMA || ptx::elect_one()) {
+                            ptx::tc_commit(&a_empty[as]);
+                            ptx::tc_commit(&s_empty[s]);
+                        }
                     }
-                    if (failed) break;
-                    if (!committed) {
-                        ptx::tc_commit_if(issue, &a_empty[as]); // the operand stage may be rewritten once these MMAs have read it
-                        ptx::tc_commit_if(issue, &s_empty[s]); // ... and the stage's src tile has been read
-                    }
-                    if (j0 == 0 && issue) WT_TRACE(1, it);
+                    if (!C::SOLO_MMA) __syncwarp();
                     if (++s == p.s_stages) s = 0;
                     if (++as == A_STAGES) { as = 0; aph ^= 1; }
                 }
                 L += sg.se - sg.sb;
             }
-            if (failed && issue) { *abort_flag = 1; atomicExch(a.status, 5); }
+            if (failed) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
     } else if (warp < CONV_WARPS) {
         // ------------------------------------------------ converters
