@@ -248,7 +248,8 @@ __global__ void __launch_bounds__(256) reorder_dense4_kernel(const __grid_consta
 // along the contiguous dim and that have no sum: four rows in flight per thread, conversions
 // without run-time type switches.  This is the quantization / dequantization of a weight or
 // activation matrix with per-tensor or per-column parameters.
-template <int SDT, int DDT>
+// RCP: s8 / u8 results by a reciprocal per column instead of a division per element, see there.
+template <int SDT, int DDT, bool RCP = false>
 __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constant__ ReorderArgs a) {
     const int dst_zp = a.dst_zp ? __ldg(a.dst_zp) : 0;
     const int d0 = a.order[0];
@@ -273,17 +274,18 @@ __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constan
     // value (a reciprocal in the normal range, rounded once, and one more rounding), so unless q is that close to
     // half an integer both round alike; beyond the range both saturate alike.  Everything else (one warp pass in
     // some twenty for uniform values, NaN, unusable reciprocals) divides.  The divisions of every element took
-    // 65 % of the issue slots while DRAM stood at 47 % (f32 4096 x 14336 -> s8: 71.4 us, now 66.9).
-    const bool by_rcp = (DDT == DT_S8 || DDT == DT_U8) && has_ds && !has_zp;
+    // 65 % of the issue slots while DRAM stood at 47 %; the launch says where this form is taken.
     float rc[4];
+    if constexpr (RCP) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        rc[e] = by_rcp ? __frcp_rn(ds[e]) : 0.f;
-        if (!(fabsf(rc[e]) >= 1.17549435e-38f && fabsf(rc[e]) <= 3.0e38f)) rc[e] = __int_as_float(0x7fffffff); // NaN
+        for (int e = 0; e < 4; ++e) {
+            rc[e] = __frcp_rn(ds[e]);
+            if (!(fabsf(rc[e]) >= 1.17549435e-38f && fabsf(rc[e]) <= 3.0e38f)) rc[e] = __int_as_float(0x7fffffff); // NaN
+        }
     }
     auto convert = [&](const float (&f)[4], const int (&iv)[4], int64_t off) {
         float out[4];
-        if (by_rcp) {
+        if constexpr (RCP) {
             float worst = 0.f; // largest distance of a quotient from its integer
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -390,7 +392,8 @@ reorder_kernel_fn cols4_for_dst(int ddt) {
         default: return nullptr;
     }
 }
-reorder_kernel_fn cols4_kernel(int sdt, int ddt) {
+reorder_kernel_fn cols4_kernel(int sdt, int ddt, bool rcp) {
+    if (rcp) return ddt == DT_S8 ? reorder_cols4_kernel<DT_F32, DT_S8, true> : reorder_cols4_kernel<DT_F32, DT_U8, true>;
     switch (sdt) {
         case DT_F32: return cols4_for_dst<DT_F32>(ddt);
         case DT_BF16: return cols4_for_dst<DT_BF16>(ddt);
@@ -634,7 +637,13 @@ dnnl_status_t qmm::execute_reorder(const dnnl_primitive_desc &pd, dnnl_stream_t 
             const int d = a.order[k];
             outer |= a.src_scale.str[d] != 0 || a.dst_scale.str[d] != 0 || a.src_zp.str[d] != 0;
         }
-        reorder_kernel_fn typed = (!outer && a.beta == 0.f) ? cols4_kernel(a.src_dt, a.dst_dt) : nullptr;
+        // Reciprocals cost four divisions of their own and the check of every quotient, so a thread has to walk
+        // enough rows, and there is nothing to gain where the src is not f32.  us a call, division -> reciprocal, f32 to
+        // s8: 2048 x 2048 (3 rows a thread) 12.8 -> 14.3, 2048 x 4096 (7) 17.7 -> 18.4, 4096 x 4096 (14) 24.7 both,
+        // 4096 x 8192 (28) 41.2 -> 39.4, 4096 x 14336 (48) 71.8 -> 67.6; bf16: 41.1 -> 42.3 and 69.9 -> 70.5 at the last two.
+        const bool rcp = a.src_dt == DT_F32 && (a.dst_dt == DT_S8 || a.dst_dt == DT_U8) && a.dst_scale.ptr && !a.dst_zp
+                && rows >= 16 * gy * ty;
+        reorder_kernel_fn typed = (!outer && a.beta == 0.f) ? cols4_kernel(a.src_dt, a.dst_dt, rcp) : nullptr;
         if (typed) typed<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, stream->stream>>>(a);
         else reorder_dense4_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, stream->stream>>>(a);
     } else {

@@ -57,8 +57,10 @@ def test_cuda_reorder_matches_oracle(gpu, name):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dst_dt", [W.S8, W.U8])
-def test_cuda_reorder_rounds_quotients_like_the_division(gpu, dst_dt):
-    """Columns whose scaled values lie on half integers and one unit beside them, saturate, or have a scale whose
+@pytest.mark.parametrize("tiles", [(1, 1), (2, 224)], ids=["few_rows_a_thread", "many_rows_a_thread"])
+def test_cuda_reorder_rounds_quotients_like_the_division(gpu, dst_dt, tiles):
+    """Small matrices divide, large ones (16 rows a thread or more) multiply with reciprocals where that is safe.
+    Columns whose scaled values lie on half integers and one unit beside them, saturate, or have a scale whose
     reciprocal is not a normal number: the 8-bit results are those of the IEEE division (element-wise, no tolerance)."""
     from onednn_b200.runner import run_reorder
     eng, strm = gpu
@@ -69,7 +71,7 @@ def test_cuda_reorder_rounds_quotients_like_the_division(gpu, dst_dt):
         x = (half[:, None] * sc[None, :]).astype(np.float32)
     rows = [x, np.nextafter(x, np.float32(np.inf)), np.nextafter(x, np.float32(-np.inf)),
             np.full((1, sc.size), 1e30, np.float32), np.full((1, sc.size), -np.inf, np.float32)]
-    x = np.concatenate(rows)
+    x, sc = np.tile(np.concatenate(rows), tiles), np.tile(sc, tiles[1])
     ro = W.Reorder("ties", W.QTensor(x, W.F32, x.shape), dst_dt, quant={"dst_scale": W.Quant(sc.reshape(1, -1), W.F32, 2)})
     got, _ = run_reorder(ro, eng, strm)
     assert np.array_equal(got, O.run_port_reorder(ro))
