@@ -411,7 +411,8 @@ def build(settings, desc, seed=None, max_macs=None):
     p = W.Problem(name or desc, M, N, K, src, wei, ddt, bias, quant, post_ops, apply_to_int, fpmath)
     p.dst_init = dst_init
     if s_st is not None or w_st is not None:  # the same problem with dense tensors, for the allowance formulas
-        dense = [W.QTensor(np.ascontiguousarray(_gather(t.data, t.dims, t.strides)), t.dt, t.dims) for t in (src, wei)]
+        dense = [t if st is None else W.QTensor(np.ascontiguousarray(_gather(t.data, t.dims, t.strides)), t.dt, t.dims)
+                 for t, st in ((src, s_st), (wei, w_st))]
         opts["dense"] = W.Problem(p.name, M, N, K, dense[0], dense[1], ddt, bias, quant, post_ops, apply_to_int, fpmath)
         opts["dense"].dst_init = dst_init
     return p, opts

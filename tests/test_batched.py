@@ -61,6 +61,8 @@ BATCHED = {
     "int8_f32_per_n_scales": (lambda s: W.int8_zp(33, 128, 64, per_n_scales=True, seed=s), 2, 2),
     "fp8_bias": (lambda s: W.fp8_prefill(40, 256, 128, seed=s), 2, 1),
     "int4_decode": (lambda s: W.int4_decode(4, 512, 256, seed=s), 3, 3),
+    "int4_rows": (lambda s: W.int4_decode(45, 256, 96, seed=s), 3, 3),
+    "int4_rows_unaligned_matrices": (lambda s: W.int4_decode(33, 272, 32, group=16, src_dt=W.F16, dst_dt=W.F16, seed=s), 3, 1),
 }
 
 

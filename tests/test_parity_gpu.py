@@ -171,6 +171,33 @@ def test_woq_decode_matches_oracle(gpu, name, kernel):
     assert np.array_equal(got, got2)
 
 
+def _scales_as(p, dt):
+    """The same problem with its weight scales in another data type."""
+    q = p.quant["wei_scale"]
+    p.quant["wei_scale"] = W.Quant(W.to_storage(W.to_f32(q.data, q.dt), dt), dt, q.mask, q.groups)
+    return p
+
+
+def _common_wei_zp(p, value, dt):
+    """One 8-bit weight zero-point for the whole tensor (4-bit ones have to vary along a dim)."""
+    p.quant["wei_zp"] = W.Quant(W.to_storage(np.array([value]), dt), dt, 0)
+    return p
+
+
+def _src_scale(p):
+    p.quant["src_scale"] = W.Quant(np.array([0.37], np.float32), W.F32, 0)
+    return p
+
+
+def _requantized(p):
+    """sum, relu and an s8 dst with a dst scale."""
+    r = np.random.Generator(np.random.PCG64(10))
+    p.post_ops += [W.PostOp(W.PO_SUM, scale=0.5), W.PostOp(W.PO_ELTWISE, W.ELTWISE["relu"], 0.0, 0.0, 1.0)]
+    p.quant["dst_scale"] = W.Quant(np.array([0.25], np.float32), W.F32, 0)
+    p.dst_init = r.integers(-100, 100, (p.M, p.N)).astype(np.int8)
+    return p
+
+
 def _large_scales():
     """f32 scales just below the type's range against src values as far below 1: all products and sums are finite."""
     p = W.int4_decode(40, 256, 160, with_zp=False, dst_dt=W.F32)
@@ -195,6 +222,22 @@ WOQ_ROWS_CASES = {
     "bias_relu": lambda: _with_bias_relu(W.int4_decode(48, 512, 256)),
     "more_tiles_than_sms": lambda: W.int4_decode(140, 192, 9632, group=64),
     "large_f32_scales": _large_scales,
+    # more than two turns of the ten-stage weight ring, batches of zero-points in rotation
+    "long_k_32_groups": lambda: W.int4_decode(70, 4096, 256),
+    "long_k_tail": lambda: W.int4_decode(50, 2896, 160, group=16),
+    "long_k_group64": lambda: W.int4_decode(129, 3072, 160, group=64, wei_dt=W.U4, zp_dt=W.S4),
+    "long_k_group256": lambda: W.int4_decode(48, 4096, 128, group=256),
+    "long_k_f16_u8zp": lambda: W.int4_decode(80, 2944, 256, zp_dt=W.U8, src_dt=W.F16, dst_dt=W.F32),
+    "long_k_two_tiles_per_cta": lambda: W.int4_decode(33, 2944, 19072),
+    "f32_scales": lambda: _scales_as(W.int4_decode(60, 640, 160), W.F32),
+    "f16_scales_f16": lambda: _scales_as(W.int4_decode(45, 512, 96, src_dt=W.F16, dst_dt=W.F16), W.F16),
+    "f8_scales": lambda: _scales_as(W.int4_decode(38, 512, 160, with_zp=False), W.F8_E4M3),
+    "f32_scales_group32": lambda: _scales_as(W.int4_decode(90, 512, 160, group=32), W.F32),
+    "common_zp_f16_s8": lambda: _common_wei_zp(W.int4_decode(64, 512, 160, src_dt=W.F16, dst_dt=W.F32), -128, W.S8),
+    "common_zp_f16_u8_per_n": lambda: _common_wei_zp(_per_n_scale(W.int4_decode(40, 512, 160, src_dt=W.F16, dst_dt=W.F16)), 255, W.U8),
+    "f16_u4_s8zp": lambda: W.int4_decode(44, 384, 160, wei_dt=W.U4, zp_dt=W.S8, src_dt=W.F16, dst_dt=W.F16),
+    "src_scale": lambda: _src_scale(W.int4_decode(72, 384, 160)),
+    "requantized_s8": lambda: _requantized(W.int4_decode(55, 256, 160, dst_dt=W.S8)),
 }
 
 
@@ -210,6 +253,34 @@ def test_woq_rows_matches_oracle(gpu, name):
     assert_parity(got, want, p.dst_dt, name, slack_for(p, impl))
     got2, _ = run_problem(p, eng, strm)
     assert np.array_equal(got, got2)
+
+
+@pytest.mark.parametrize("which,shift", [("src", 2), ("wei", 1), ("wei_zp", 2)])
+def test_woq_rows_misaligned_pointers_take_the_generic_kernel(gpu, which, shift):
+    """Buffers that TMA (16 bytes) or the zero-point loads (4 bytes) cannot read: the same results, from the generic
+    kernel, through the same primitive."""
+    import torch
+    from onednn_b200.runner import Prepared
+    eng, strm = gpu
+    p = W.int4_decode(40, 256, 96)
+    dev, keep, ptrs = torch.device("cuda:0"), [], {}
+    for name, a in [("src", p.src.data), ("wei", p.wei.data)] + [(k, q.data) for k, q in p.quant.items()]:
+        raw = torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1).copy())
+        t = torch.zeros(raw.numel() + 256, dtype=torch.uint8, device=dev)
+        at = shift if name == which else 0
+        t[at:at + raw.numel()].copy_(raw)
+        keep.append(t)
+        ptrs[name] = t.data_ptr() + at
+    dst = torch.zeros(p.M * p.N, dtype=torch.int16, device=dev)
+    ptrs["dst"] = dst.data_ptr()
+    prep = Prepared(p, eng)
+    assert prep.impl == "cuda:tcgen05:woq4_rows"
+    prep.bind_device(ptrs)
+    torch.cuda.synchronize()  # torch's copies run on its own stream
+    prep.execute(strm)
+    strm.wait()
+    got = dst.cpu().numpy().view(np.uint16).reshape(p.M, p.N)
+    assert_parity(got, O.run_port(p), p.dst_dt, which)
 
 
 GROUPED_TC_CASES = {
@@ -400,8 +471,6 @@ def test_runtime_m_matches_oracle(gpu, name):
     eng, strm = gpu
     for M in (1, 24, 100):
         p = RUNTIME_M_CASES[name](M)
-        if p.M > 32 and name == "int4_decode":
-            continue
         r = Prepared(p, eng, runtime_m=True).upload()
         r.execute(strm)
         strm.wait()
@@ -409,6 +478,21 @@ def test_runtime_m_matches_oracle(gpu, name):
         fixed, impl = run_problem(p, eng, strm)
         assert np.array_equal(got, fixed), "%s M=%d: runtime-M result differs from the fixed-M primitive (%s)" % (name, M, impl)
         assert_parity(got, O.run_port(p), p.dst_dt, "%s M=%d" % (name, M), slack_for(p, impl))
+
+
+def test_one_int4_primitive_goes_from_decode_to_rows_and_back(gpu):
+    """A primitive with open M takes the decode kernel (partial sums and arrival counters in the scratchpad) or the
+    kernel for more rows (no scratchpad), by the M of each call."""
+    from onednn_b200.runner import Prepared
+    eng, strm = gpu
+    prim = None
+    for M in (1, 24, 100, 33, 32, 40, 1):
+        p = W.int4_decode(M, 2048, 1024)
+        r = Prepared(p, eng, runtime_m=True).upload()
+        prim = prim or r.prim
+        prim.execute(strm, r.args)
+        strm.wait()
+        assert_parity(r.download(), O.run_port(p), p.dst_dt, "M = %d" % M, summation_slack(p))
 
 
 @pytest.mark.gpu
