@@ -63,11 +63,12 @@ namespace {
 
 constexpr int GT_N = 128; // dst columns per tile = TMEM lanes = UMMA M
 constexpr int GT_M = 208; // most src rows per tile = UMMA N
+constexpr int GT_M_LOW = 192; // ... where that costs no wave of tiles, see grouped_plan_kernel
 constexpr int GK = 64; // k per operand slot: one 128-byte swizzle row of bf16 src
 // Two shared-memory rings and one in tensor memory: the raw weights come from HBM, the src rows from L2,
 // and the widened operand is produced and consumed on the SM (slots of 32 columns beside the two accumulators).
 // 208 rows per tile: what the two accumulators leave is three slots, which is what three converter sets fill;
-// 777 rows of a dense problem are then four blocks of 195 and 128 tiles - one wave - instead of 160 tiles.
+// 777 rows of a dense problem are then four blocks and, for 4096 columns, 128 tiles - one wave - instead of 160.
 constexpr int RAW_STAGES = 5, A_SLOTS = 3, B_STAGES = 5;
 constexpr int LK = 2 * GK; // k per raw weight tile: a copy costs its thread about 500 cycles, whatever its size
 constexpr int RAW_BYTES = LK * GT_N; // s8 weights as loaded
@@ -100,13 +101,20 @@ constexpr bool pieces_stay_in_the_accumulator() {
 }
 static_assert(pieces_stay_in_the_accumulator(), "the epilogue reads tensor memory that other warps write");
 
-// plan[0] = {total tiles, groups, 0, 0}; plan[1 + g] = {first src row, first dst row, rows, first tile}
+// plan[0] = {total tiles, groups, blocks of up to GT_M_LOW rows (else GT_M), 0}; plan[1 + g] = {first src row, first dst row, rows, first tile}
 struct Tile {
     int g, n0, m0, rows, src_row, dst_row;
 };
+// ceil(rows / limit), limit = 208 or 192, in the three instructions of a constant divisor (every role does this once a
+// tile): x / 16 < 2^27, for which ceil(2^32 / 13) and ceil(2^32 / 12) as multipliers give the exact quotient.
+__device__ __forceinline__ int row_blocks(int rows, bool low) {
+    const uint32_t x = (uint32_t)rows + (low ? GT_M_LOW - 1u : GT_M - 1u);
+    return (int)__umulhi(x >> 4, low ? 357913942u : 330382100u);
+}
+static_assert(GT_M == 13 * 16 && GT_M_LOW == 12 * 16, "row_blocks");
 // (`plan` is the kernel's copy of the records in shared memory when they fit: every role looks a tile
 // up when it begins it, and six dependent loads from global memory there cost microseconds per tile)
-__device__ __forceinline__ Tile decode_tile(const int4 *plan, int groups, int num_n_tiles, int t) {
+__device__ __forceinline__ Tile decode_tile(const int4 *plan, int groups, bool low, int t) {
     int lo = 0, hi = groups; // last group whose first tile is <= t, skipping empty groups behind it
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -114,7 +122,7 @@ __device__ __forceinline__ Tile decode_tile(const int4 *plan, int groups, int nu
     }
     const int4 e = plan[1 + lo];
     const int r = t - e.w;
-    const int mt = (e.z + GT_M - 1) / GT_M;
+    const int mt = row_blocks(e.z, low);
     Tile tl;
     tl.g = lo;
     // row blocks of equal size (a multiple of 16): a short last block would pay a whole pass over the weights
@@ -127,29 +135,62 @@ __device__ __forceinline__ Tile decode_tile(const int4 *plan, int groups, int nu
     return tl;
 }
 
-__global__ void grouped_plan_kernel(const __grid_constant__ MatmulArgs a, int4 *plan, int num_n_tiles) {
+// Blocks of up to GT_M rows, unless blocks of up to 192 take the tiles through the SMs in the same number of waves:
+// the busiest SM then works through fewer rows, and a short K takes its time for rows (the epilogue's stores).  us a
+// call, 208 -> 192: dense, 4096 rows, K = N = 1024 48.3 -> 45.2; 1940 rows, K = 592, N = 4400 65.7 -> 61.5;
+// 8 experts, 8192 rows, K = N = 1024 69.8 -> 65.3 (the last with the scale and the 64 in one product).
+//
+// One warp, a lane per group, in two walks over the groups: counts, then records.  (One thread that walked the groups
+// with both counts took 1.8 us longer for 32 groups and 6 us for 64 than with one; its loads wait for one another.)
+__global__ void grouped_plan_kernel(const __grid_constant__ MatmulArgs a, int4 *plan, int num_n_tiles, int sms) {
     asm volatile("griddepcontrol.launch_dependents;"); // the main kernel may set itself up meanwhile; it waits before it reads the plan
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const int lane = threadIdx.x;
+    auto waves = [&](int total) { return (total + sms - 1) / sms; };
     if (a.group_count == 0) { // a dense problem: one group that owns every row
+        if (lane != 0) return;
+        const int tall = row_blocks((int)a.M, false) * num_n_tiles, low = row_blocks((int)a.M, true) * num_n_tiles;
+        const bool use_low = waves(low) == waves(tall);
         plan[1] = make_int4(0, 0, (int)a.M, 0);
-        plan[0] = make_int4((int)((a.M + GT_M - 1) / GT_M) * num_n_tiles, 1, 0, 0);
+        plan[0] = make_int4(use_low ? low : tall, 1, use_low, 0);
         return;
     }
     bool bad = false;
-    int tiles = 0;
-    for (int g = 0; g < a.group_count; ++g) {
+    // {first src row, first dst row, rows} of group g; an invalid group owns no rows
+    auto group = [&](int g) {
         const int64_t b = g == 0 ? 0 : a.offsets[g - 1], e = a.offsets[g];
         const int64_t db = g == 0 ? 0 : a.dst_offsets[g - 1], de = a.dst_offsets[g];
-        if (b < 0 || e > a.M || e < b || db < 0 || de > a.M || de < db || de - db != e - b) bad = true;
-        const int rows = bad ? 0 : (int)(e - b);
-        plan[1 + g] = make_int4((int)b, (int)db, rows, tiles);
-        tiles += ((rows + GT_M - 1) / GT_M) * num_n_tiles;
+        const bool wrong = b < 0 || e > a.M || e < b || db < 0 || de > a.M || de < db || de - db != e - b;
+        bad |= wrong;
+        return make_int3((int)b, (int)db, wrong ? 0 : (int)(e - b));
+    };
+    int tall = 0, low = 0;
+    for (int g = lane; g < a.group_count; g += 32) {
+        const int rows = group(g).z;
+        tall += row_blocks(rows, false);
+        low += row_blocks(rows, true);
     }
-    if (bad) {
-        atomicExch(a.status, 2); // invalid_arguments, reported when the stream is waited on
-        tiles = 0;
+    tall = __reduce_add_sync(0xffffffffu, tall) * num_n_tiles;
+    low = __reduce_add_sync(0xffffffffu, low) * num_n_tiles;
+    const bool use_low = waves(low) == waves(tall);
+    int first = 0; // tiles of the 32s of groups before this one
+    for (int g0 = 0; g0 < a.group_count; g0 += 32) {
+        const int g = g0 + lane;
+        const int3 r = g < a.group_count ? group(g) : make_int3(0, 0, 0);
+        const int own = row_blocks(r.z, use_low) * num_n_tiles;
+        int upto = own; // inclusive sum over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= d) upto += x;
+        }
+        if (g < a.group_count) plan[1 + g] = make_int4(r.x, r.y, r.z, first + upto - own);
+        first += __shfl_sync(0xffffffffu, upto, 31);
     }
-    plan[0] = make_int4(tiles, a.group_count, 0, 0);
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        if (bad) atomicExch(a.status, 2); // invalid_arguments, reported when the stream is waited on
+        plan[0] = make_int4(bad ? 0 : first, a.group_count, use_low, 0);
+    }
 }
 
 __device__ __forceinline__ uint32_t prmt_(uint32_t a, uint32_t b, uint32_t sel) {
@@ -209,7 +250,7 @@ template <bool EPI_CHAIN>
 __global__ void __launch_bounds__(G_THREADS, 1)
 grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
         const __grid_constant__ CUtensorMap tmS2, const __grid_constant__ CUtensorMap tmS3,
-        const __grid_constant__ MatmulArgs a, const int4 *plan_global, const float *rowsum, int num_n_tiles,
+        const __grid_constant__ MatmulArgs a, const int4 *plan_global, const float *rowsum,
         int num_k_blocks) {
     constexpr uint32_t TMEM_COLS = 512;
     extern __shared__ uint8_t smem_raw[];
@@ -260,6 +301,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     ptx::grid_dependency_wait();
     const int4 head = ptx::ld_dependent_int4(&plan_global[0]);
     const int num_tiles = head.x, groups = head.y;
+    const bool low_blocks = head.z != 0;
     const int4 *plan = plan_global;
     if (groups <= PLAN_CACHE_GROUPS) {
         int4 *cache = reinterpret_cast<int4 *>(smem + G_PLAN_OFFSET);
@@ -276,7 +318,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             uint32_t ph = 1; // parity of the empty barrier's previous phase: a fresh barrier passes
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x) {
-                const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
+                const Tile tl = decode_tile(plan, groups, low_blocks, t);
                 for (int kb = 0; kb < num_k_blocks; kb += 2) {
                     if (!ptx::mbar_wait(&raw_empty[s], ph)) { ok = false; break; }
                     ptx::mbar_arrive_expect_tx(&raw_full[s], RAW_BYTES);
@@ -293,7 +335,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             uint32_t ph = 1;
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x) {
-                const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
+                const Tile tl = decode_tile(plan, groups, low_blocks, t);
                 // a box of 64, 128 or GT_M rows, whichever covers the tile's rows
                 const CUtensorMap *tm = tl.rows <= 64 ? &tmS : tl.rows <= 128 ? &tmS2 : &tmS3;
                 const uint32_t bytes = (tl.rows <= 64 ? 64 : tl.rows <= 128 ? 128 : GT_M) * GK * 2;
@@ -316,7 +358,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             uint32_t pa = 0, pb = 0, acc_it = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok && !*abort_flag; t += gridDim.x, ++acc_it) {
-                const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
+                const Tile tl = decode_tile(plan, groups, low_blocks, t);
                 const uint32_t n_mma = (uint32_t)max(16, (tl.rows + 15) & ~15);
                 const uint32_t idesc = ptx::make_idesc(ptx::CFMT_F32, ptx::FMT_BF16, ptx::FMT_BF16, false, false, GT_N, n_mma);
                 const int as = acc_it % ACC_STAGES;
@@ -410,7 +452,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         const int lane_base = (warp % 4) * 32; // TMEM lanes (dst columns) this warp may read
         uint32_t acc_it = 0;
         for (int t = blockIdx.x; t < num_tiles && !*abort_flag; t += gridDim.x, ++acc_it) {
-            const Tile tl = decode_tile(plan, groups, num_n_tiles, t);
+            const Tile tl = decode_tile(plan, groups, low_blocks, t);
             const int as = acc_it % ACC_STAGES;
             const uint32_t aph = (acc_it / ACC_STAGES) & 1;
             const int64_t n = tl.n0 + lane_base + lane_column(lane);
@@ -418,6 +460,10 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             if (a.wei_scale.ptr && n < a.N)
                 scale = load_float(a.wei_scale.dt, a.wei_scale.ptr,
                         (int64_t)tl.g * a.wei_scale.gstride + ((a.wei_scale.mask & 2) ? n : 0));
+            // the sums times 64 times the scale: in one product unless 64 * scale overflows in some lane (1940 rows,
+            // K = 592, N = 4400: 61.5 us with two, 59.7 with one)
+            const float scale64 = scale * A_SCALE;
+            const bool plain = a.dst_dt == DT_BF16 && __all_sync(0xffffffffu, !(fabsf(scale) >= 0x1p120f));
             float zp = 0.f; // weight zero-point of this column (chain epilogue only)
             if (EPI_CHAIN && a.wei_zp.ptr && n < a.N)
                 zp = (float)load_int(a.wei_zp.dt, a.wei_zp.ptr,
@@ -464,11 +510,11 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                             d = apply_post_ops(a, d, 0.f, m, n, tl.g);
                             store_float(a.dst_dt, d, a.dst, m * a.dst_sm + n);
                         }
-                    } else if (a.dst_dt == DT_BF16) {
+                    } else if (plain) {
                         unsigned short *d = (unsigned short *)a.dst + row0 * a.dst_sm + n;
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (j < m_hi) d[(int64_t)j * a.dst_sm] = f32_to_bf16_bits(__uint_as_float(r[j]) * A_SCALE * scale);
+                            if (j < m_hi) d[(int64_t)j * a.dst_sm] = f32_to_bf16_bits(__uint_as_float(r[j]) * scale64);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
@@ -551,8 +597,9 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
     }
     const int num_n_tiles = (int)((a.N + GT_N - 1) / GT_N);
     const int num_k_blocks = (int)((a.K + LK - 1) / LK) * 2; // in pairs: k beyond K reads as zeros
+    const int sms = sm_count > 0 ? sm_count : 148;
     int4 *plan = (int4 *)scratch;
-    grouped_plan_kernel<<<1, 32, 0, st>>>(a, plan, num_n_tiles);
+    grouped_plan_kernel<<<1, 32, 0, st>>>(a, plan, num_n_tiles, sms);
     count_launch();
     float *rowsum = (float *)((char *)scratch + plan_bytes(a.group_count > 0 ? a.group_count : 1));
     if (a.wei_zp.ptr) {
@@ -566,7 +613,7 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
     if (!opt_in_dynamic_smem(kern, G_SMEM_BYTES, configured[chain])) return 5;
     {
         cudaLaunchConfig_t cfg {};
-        cfg.gridDim = dim3((unsigned)(sm_count > 0 ? sm_count : 148));
+        cfg.gridDim = dim3((unsigned)sms);
         cfg.blockDim = dim3((unsigned)G_THREADS);
         cfg.dynamicSmemBytes = (size_t)G_SMEM_BYTES;
         cfg.stream = st;
@@ -577,9 +624,9 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
         cfg.numAttrs = 1;
         const int4 *plan_c = plan;
         const float *rowsum_c = rowsum;
-        if (cudaLaunchKernelEx(&cfg, kern, tw, ts, ts2, ts3, a, plan_c, rowsum_c, num_n_tiles, num_k_blocks) != cudaSuccess) {
+        if (cudaLaunchKernelEx(&cfg, kern, tw, ts, ts2, ts3, a, plan_c, rowsum_c, num_k_blocks) != cudaSuccess) {
             (void)cudaGetLastError(); // the attribute was refused: an ordinary launch
-            kern<<<sm_count > 0 ? sm_count : 148, G_THREADS, G_SMEM_BYTES, st>>>(tw, ts, ts2, ts3, a, plan, rowsum, num_n_tiles, num_k_blocks);
+            kern<<<sms, G_THREADS, G_SMEM_BYTES, st>>>(tw, ts, ts2, ts3, a, plan, rowsum, num_k_blocks);
         }
     }
     count_launch();

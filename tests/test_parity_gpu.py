@@ -293,6 +293,10 @@ GROUPED_TC_CASES = {
     "odd_k_slots": lambda: W.moe_grouped(130, 1088, 256, 2, sizes=[129, 1]),
     "zipf": lambda: W.moe_grouped(1024, 512, 384, 16),
     # blocks that end in 16 rows or fewer of a 32-row epilogue piece, several tiles per CTA (both accumulators in use)
+    # more groups than the planning warp has lanes, none of their numbers a multiple of 32
+    "70_groups": lambda: W.moe_grouped(300, 128, 64, 70),
+    "33_groups_empty_ends": lambda: W.moe_grouped(450, 128, 160, 33, sizes=[0, 0, 209] + [0] * 28 + [241, 0]),
+    "low_blocks": lambda: W.moe_grouped(594, 128, 256, 4, sizes=[400, 0, 193, 1]),  # blocks of up to 192 rows: no more waves
     "full_blocks_both_accumulators": lambda: W.moe_grouped(609, 128, 19200, 3, sizes=[193, 208, 208]),
 }
 
@@ -334,6 +338,16 @@ def _woq8(M, K, N, per_n=True, dst_dt=W.BF16, seed=31):
     return W.Problem("woq8", M, N, K, W.QTensor(W.f32_to_bf16(r.standard_normal((M, K), dtype=np.float32)), W.BF16, (M, K)),
                      W.QTensor(r.integers(-127, 128, (K, N), dtype=np.int8), W.S8, (K, N)), dst_dt, quant=q,
                      apply_to_int=True, fpmath=1)
+
+
+def _woq8_large_scales():
+    """Scales beyond which the kernel no longer multiplies them by 64 beforehand (a few in every warp's columns),
+    against src values as far below 1; scale * weight is finite, as the reference's order of products needs."""
+    p = _woq8(70, 128, 256, dst_dt=W.BF16)
+    p.src = W.QTensor(W.f32_to_bf16(W.bf16_to_f32(p.src.data) * np.float32(2.0 ** -100)), W.BF16, p.src.dims)
+    q = p.quant["wei_scale"].data
+    q[:, ::3] = 2.0 ** 120 * np.linspace(1.0, 1.8, q[:, ::3].shape[1])
+    return p
 
 
 def _woq8_bias_chain():
@@ -400,6 +414,9 @@ WOQ8_CASES = {
     "zero_point_common_s32": lambda: _woq8_zp(False, W.S32),
     "prefill": lambda: _woq8(300, 512, 384),
     "tails": lambda: _woq8(77, 200, 176),
+    "full_blocks": lambda: _woq8(208, 128, 9600),  # one wave of 208-row blocks, two of 192-row ones
+    "low_blocks": lambda: _woq8(400, 128, 9600),  # two waves either way
+    "large_scales": lambda: _woq8_large_scales(),
     "one_row": lambda: _woq8(1, 256, 128),
     "common_scale_f32": lambda: _woq8(130, 128, 256, per_n=False, dst_dt=W.F32),
 }
