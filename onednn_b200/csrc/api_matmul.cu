@@ -430,7 +430,8 @@ dnnl_status_t woq_accepts(const dnnl_primitive_desc &pd) {
 }
 
 // More rows than the decode kernels take: src rows by TMA, and weights less zero-points that stay exact
-// in the src's type - bf16 holds every integer up to 256, w - zp with 4-bit zero-points; f16 up to 2048
+// in the src's type: f16 holds every integer up to 2048; bf16 every one up to 256, which s4 - u8 can leave (-263).
+// With a bf16 src all 8-bit zero-points go to the generic kernel, those that would stay exact too.
 dnnl_status_t woq_rows_accepts(const dnnl_primitive_desc &pd) {
     if (woq4_accepts(pd) != dnnl_success) return dnnl_unimplemented;
     UNIMPL_IF(pd.M() <= 32 || pd.M() >= (1LL << 31) || pd.N() >= (1LL << 29) || pd.src.strides[0] % 8 != 0 || pd.src.strides[0] < pd.K());

@@ -294,7 +294,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     using L = SmemLayout<BT_M, STAGES>;
     constexpr bool INT = KIND == 1;
     constexpr int ACC_STAGES = 2;
-    constexpr uint32_t TMEM_COLS = ACC_STAGES * BT_M; // 256 or 512, a power of two
+    constexpr uint32_t TMEM_COLS = ACC_STAGES * BT_M; // 128, 256 or 512, a power of two
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full_bar = (uint64_t *)(smem + L::BAR_OFFSET);
@@ -686,8 +686,10 @@ int launch_gemm_tc(const MatmulArgs &a_in, void *scratch, int sm_count, cudaStre
     const bool chain = a.n_po > 0 || (a.bias && a.bias_sm != 0); // a bias varying along M rides the generic tail
     // 256 dst rows per tile unless that leaves SMs without work; 64 when even tiles of 128 rows leave more than
     // half of them idle, or for at most 64 rows (less src to load, and room for more stages in flight); kernels
-    // with a post-op chain, twelve of them, have no third tile size.  (int8, 17 rows, 4096 x 11008: 24.5 us with
-    // 128-row tiles and a lane-index predicate on the issuing thread, 20.5 with 64 rows and an elected one.)
+    // with a post-op chain, twelve of them, have no third tile size.  us a call, 128-row tiles -> 64: int8 17 x 4096 x
+    // 11008 24.4 -> 20.6, fp8 64 x 4096 x 11008 16.5 -> 14.5; above 64 rows fp8 128 x 4096 x 4096 14.6 -> 12.4,
+    // 300 x 8192 x 1024 20.6 -> 16.5; where 128-row tiles occupy more than half of the SMs (65 x 4096 x 11008) 64 rows
+    // would make two waves.
     const int64_t tiles256 = (int64_t)tp.num_n_tiles * ((a.M + 255) / 256);
     const int64_t tiles128 = (int64_t)tp.num_n_tiles * ((a.M + 127) / 128);
     const bool tall = a.M > 128 && tiles256 >= sm_count / 2;

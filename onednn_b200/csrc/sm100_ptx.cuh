@@ -18,9 +18,10 @@ __device__ __forceinline__ uint64_t globaltimer() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// True in exactly one lane of a converged warp.  tcgen05.mma issued under this predicate (a branch or
-// a guard) takes about 70 cycles per instruction; under a predicate computed from the lane index, which
-// the hardware cannot know to be one lane, about 115.
+// True in exactly one lane of a converged warp, the same one every time.  A tcgen05.mma takes about 12 cycles to
+// issue where the elected thread runs the role's whole loop, about 70 in a branch on this predicate inside a loop that
+// the whole warp walks, and about 115 under a predicate computed from the lane index, which the hardware cannot know
+// to be one lane.
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(
@@ -107,28 +108,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
         if (globaltimer() - t0 > limit_ns) return false;
     }
 }
-// A 32-bit word in shared memory handed from one warp to another
-__device__ __forceinline__ uint32_t ld_acquire_shared(const volatile uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(const_cast<uint32_t *>(p))) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_shared(volatile uint32_t *p, uint32_t v) {
-    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t *>(p))), "r"(v) : "memory");
-}
-
-// A commit under a lane predicate, for the rarely taken paths of warp-uniform issuing code (whole
-// warps walk the loops, so that loop counters, addresses and descriptors stay warp-uniform values).
-// The hot paths put a stage's tcgen05 / TMA instructions in a branch taken by the thread elect_one()
-// picks instead: an instruction guarded by a predicate computed from the lane index costs nearly twice
-// as much to issue.
-__device__ __forceinline__ void tc_commit_if(bool issue, uint64_t *bar) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"((uint32_t)issue)
-                 : "memory");
-}
-
-// The same for a whole warp that may wait long: between polls the warp sleeps a few dozen
+// mbar_wait for a whole warp that may wait long: between polls the warp sleeps a few dozen
 // nanoseconds, so that a dozen waiting warps do not fill the SM's shared-memory instruction queue
 // with polls that the working warps' loads, arrives and tensor-memory stores then queue behind.
 __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t *bar, uint32_t parity, uint64_t limit_ns = 2000000000ull) {

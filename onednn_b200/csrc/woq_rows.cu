@@ -26,9 +26,15 @@
 // Roles (28 warps): 0 weight tiles by TMA, 1 src tiles by TMA, 2 issues all MMAs, 4-11 converters (two per lane
 // quarter, taking the stages in turn), 12-27 epilogue (four per lane quarter, each a quarter of the rows).  Every mbarrier wait is bounded.
 //
-// Measured on a B200 at K = N = 4096, M = 300, groups of 128, u4 zero-points: 41 us a call (66 us with 64-k stages,
-// a warp-wide issuing loop and eight epilogue warps; 43 us with a shift and a subtraction per pair); the generic kernel,
-// which such calls took before, 54.3 ms.
+// Measured on a B200, us a call at K = N = 4096, bf16, zero-points per group, by the group size (every group costs a
+// fold of the whole accumulator and two hand-offs):
+//   group            32    64   128   256
+//   M = 64          118    66    40    33
+//   M = 128         136    76    43    35
+//   M = 300         116    70    43    36
+//   M = 512         137    77    44    37
+// 32 tiles and 96 at M = 64 and 300 leave SMs idle: K is not split.  300 rows in groups of 128 without zero-points 37;
+// the generic kernel takes 54.3 ms for them.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -347,7 +353,7 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                 const int v = base_off + (zp_mode == 1 ? zp_of(zp_dt, raw, c) : zt);
                 const int u = v + min(v, 0);
                 uint32_t b;
-                if (!F16) b = __float_as_uint((float)v * -0.015625f) >> 16; // exact: at most six bits
+                if (!F16) b = __float_as_uint((float)v * -0.015625f) >> 16; // exact for 4-bit zero-points
                 else if (zp4) b = (c & 1) ? 0xD400u + 16 * u : 0x6400u + u;
                 else b = __half_as_ushort(__int2half_rn((c & 1) ? -(64 + v) : 1024 + v));
                 o2[c] = b * 0x10001u;
