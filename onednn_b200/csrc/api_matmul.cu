@@ -441,17 +441,16 @@ dnnl_status_t woq_rows_accepts(const dnnl_primitive_desc &pd) {
     return dnnl_success;
 }
 
-// int4 decompression through tensor memory: what the skinny GEMM accepts, with
-// the src rows reachable by TMA (16-byte row pitch unless there is one row)
+// int4 decompression for few rows: what the skinny GEMM accepts, with the src rows reachable by TMA (16-byte row pitch unless there is one row)
 dnnl_status_t woq_tc_accepts(const dnnl_primitive_desc &pd) {
     if (woq_accepts(pd) != dnnl_success) return dnnl_unimplemented;
     UNIMPL_IF(pd.M() > 1 && pd.src.strides[0] % 8 != 0);
     UNIMPL_IF(pd.wei.strides[0] % 32 != 0);
-    // the scale / zero-point rows of a stage's groups must fit in the kernel's shared-memory ring
+    // wide scale / zero-point rows of small groups: see woq_decode_fits
     const auto &ws = pd.attr.scale(DNNL_ARG_WEIGHTS);
     const auto &wz = pd.attr.zp(DNNL_ARG_WEIGHTS);
     const dnnl_dim_t group = ws.mask == 3 ? ws.groups[0] : pd.K();
-    UNIMPL_IF(!woq_tc_fits(pd.M(), pd.K(), group, (int)ws.dt, (wz.set && wz.mask == 3) ? (int)wz.dt : -1));
+    UNIMPL_IF(!woq_decode_fits(pd.M(), pd.K(), group, (int)ws.dt, (wz.set && wz.mask == 3) ? (int)wz.dt : -1));
     return dnnl_success;
 }
 
@@ -520,7 +519,7 @@ dnnl_status_t impl_accepts(const dnnl_primitive_desc &pd, int impl, std::string 
             return grouped_tc_accepts(pd);
         case IMPL_WOQ_TC:
             if (pd.grouped) return dnnl_unimplemented;
-            name = "cuda:tcgen05:woq4";
+            name = "cuda:tcgen05:woq4"; // the name programs know this entry by; its kernel is woq_decode.cu
             return woq_tc_accepts(pd);
         case IMPL_WOQ_GEMV:
             if (pd.grouped) return dnnl_unimplemented;
@@ -553,9 +552,9 @@ dnnl_status_t select_impl(dnnl_primitive_desc &pd, int first) {
             if (i == IMPL_TCGEN05_GEMM && (pd.attr.zp(DNNL_ARG_SRC).set || pd.attr.zp(DNNL_ARG_WEIGHTS).set))
                 pd.scratch_bytes = gemm_tc_scratch_bytes(pd.M(), pd.N());
             // the skinny GEMM keeps split-K partial sums and arrival counters there
-            if (i == IMPL_WOQ_TC)
-                pd.scratch_bytes = woq_tc_scratch_bytes(
-                        pd.M(), pd.N(), pd.K(), pd.engine->sm_count > 0 ? pd.engine->sm_count : 148);
+            // the decode kernel adds its split sums through shared memory; a program that brings the scratchpad
+            // itself goes on being asked for one (it need not be cleared)
+            if (i == IMPL_WOQ_TC && pd.attr.scratchpad_mode == dnnl_scratchpad_mode_user) pd.scratch_bytes = 256;
             if (i == IMPL_WOQ_GEMV)
                 pd.scratch_bytes = woq_skinny_scratch_bytes(
                         pd.N(), pd.K(), pd.engine->sm_count > 0 ? pd.engine->sm_count : 148);
@@ -1155,13 +1154,8 @@ static dnnl_status_t execute_matmul_2d(const_dnnl_primitive_t primitive, const d
     switch (pd.impl) {
         case IMPL_REF: rc = launch_ref(a, stream->stream); break;
         case IMPL_WOQ_TC:
-            if (!woq_tc_pointers_ok(a)) {
-                rc = launch_ref(a, stream->stream); // misaligned user pointers: generic kernel
-            } else {
-                if (pd.attr.scratchpad_mode == dnnl_scratchpad_mode_user) // counters of a user buffer
-                    cudaMemsetAsync(scratch, 0, ((pd.N() + 255) / 256) * sizeof(int), stream->stream);
-                rc = launch_woq_tc(a, scratch, pd.engine->sm_count, stream->stream);
-            }
+            if (!woq_decode_pointers_ok(a)) rc = launch_ref(a, stream->stream); // misaligned user pointers: generic kernel
+            else rc = launch_woq_decode(a, pd.engine->sm_count, stream->stream);
             break;
         case IMPL_WOQ_GEMV:
             if ((uintptr_t)a.wei % 16 || (uintptr_t)a.src % 4 || (uintptr_t)a.wei_scale.ptr % 16

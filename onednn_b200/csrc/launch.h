@@ -47,14 +47,10 @@ bool gemm_tc_pointers_ok(const MatmulArgs &a);
 int launch_woq_skinny(const MatmulArgs &a, void *scratch, int sm_count, cudaStream_t st);
 size_t woq_skinny_scratch_bytes(int64_t N, int64_t K, int sm_count);
 
-// int4 weight-decompression GEMM for M <= 32 on tcgen05 with the rebuilt
-// weights as a tensor-memory operand (woq_tc.cu).  `scratch`:
-// woq_tc_scratch_bytes(...) bytes, zero-initialised once (arrival counters
-// and split-K partial sums).
-int launch_woq_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStream_t st);
-size_t woq_tc_scratch_bytes(int64_t M, int64_t N, int64_t K, int sm_count);
-bool woq_tc_pointers_ok(const MatmulArgs &a);
-bool woq_tc_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_dt);
+// int4 weight-decompression GEMM for M <= 32 (woq_decode.cu)
+int launch_woq_decode(const MatmulArgs &a, int sm_count, cudaStream_t st);
+bool woq_decode_pointers_ok(const MatmulArgs &a);
+bool woq_decode_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_dt);
 
 // int4 weight-decompression GEMM for M > 32 on tcgen05 (woq_rows.cu)
 int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st);

@@ -137,7 +137,7 @@ struct dnnl_primitive_attr {
 // One entry of the implementation list walked by primitive_desc_next_impl.
 enum impl_id_t : int {
     IMPL_TCGEN05_GEMM = 0, // tensor-core int8 / fp8 GEMM
-    IMPL_WOQ_TC, // int4 weight decompression through tensor memory (M <= 32)
+    IMPL_WOQ_TC, // int4 weight decompression, few rows (M <= 32)
     IMPL_WOQ_GEMV, // weight-decompression skinny GEMM (M <= 32), mma.sync
     IMPL_WOQ_ROWS, // int4 weight decompression through tensor memory, M > 32
     IMPL_GROUPED_TC, // grouped (MoE) tensor-core GEMM

@@ -1,0 +1,110 @@
+"""int4 weight decompression for at most 32 rows: the edges of the kernel's row blocks, column tiles, K stages and groups."""
+import numpy as np
+import pytest
+
+from onednn_b200 import workloads as W
+from onednn_b200.runner import run_problem
+from oracle import oracle as O
+from util import assert_parity, summation_slack
+
+pytestmark = pytest.mark.gpu
+
+
+def _scales(p, dt):
+    q = p.quant["wei_scale"]
+    p.quant["wei_scale"] = W.Quant(W.to_storage(W.to_f32(q.data, q.dt), dt), dt, q.mask, q.groups)
+    return p
+
+
+def _common_zp(p, value, dt):
+    p.quant["wei_zp"] = W.Quant(W.to_storage(np.array([value]), dt), dt, 0)
+    return p
+
+
+def _one_scale_row(p):
+    q = p.quant["wei_scale"]
+    p.quant["wei_scale"] = W.Quant(np.ascontiguousarray(q.data.reshape(-1, p.N)[:1]), q.dt, 2)
+    p.quant.pop("wei_zp", None)
+    return p
+
+
+def _large_scales():
+    """f32 scales just below the type's range against src values as far below 1: all products and sums are finite."""
+    p = W.int4_decode(6, 256, 160, with_zp=False, dst_dt=W.F32)
+    r = np.random.Generator(np.random.PCG64(11))
+    p.src = W.QTensor(W.f32_to_bf16(W.bf16_to_f32(p.src.data) * np.float32(2.0 ** -100)), W.BF16, p.src.dims)
+    q = p.quant["wei_scale"]
+    p.quant["wei_scale"] = W.Quant((r.uniform(1.0, 1.99, q.data.shape) * 2.0 ** 123).astype(np.float32), W.F32, 3, q.groups)
+    return p
+
+
+CASES = {
+    "one_step_one_column_piece": lambda: W.int4_decode(1, 16, 32, group=16),
+    "m9_two_blocks": lambda: W.int4_decode(9, 512, 288),
+    "m24_three_blocks": lambda: W.int4_decode(24, 1024, 544, group=64),
+    "m25_four_blocks_f16": lambda: W.int4_decode(25, 768, 256, wei_dt=W.U4, src_dt=W.F16, dst_dt=W.F16, with_zp=False, group=64),
+    "m17_group32": lambda: W.int4_decode(17, 416, 320, group=32),
+    "m16_group48_across_stages": lambda: W.int4_decode(16, 1104, 256, group=48),
+    "m32_group16": lambda: W.int4_decode(32, 272, 160, group=16, zp_dt=W.S4),
+    "k_tail_group16": lambda: W.int4_decode(3, 1040, 96, group=16, wei_dt=W.U4),
+    "k_tail_one_group": lambda: _one_scale_row(W.int4_decode(11, 1072, 288, group=16)),
+    "shares_cut_groups": lambda: W.int4_decode(2, 4096, 256, group=512),
+    "eight_shares_ring_turns": lambda: W.int4_decode(5, 8192, 256),
+    "many_tiles": lambda: W.int4_decode(1, 256, 40992),
+    "f16_s4_s4zp": lambda: W.int4_decode(13, 1024, 288, zp_dt=W.S4, src_dt=W.F16, dst_dt=W.F32),
+    "u8_zp_m20": lambda: W.int4_decode(20, 512, 288, zp_dt=W.U8),
+    "s8_zp_f16_m30": lambda: W.int4_decode(30, 512, 288, wei_dt=W.U4, zp_dt=W.S8, src_dt=W.F16, dst_dt=W.F16),
+    "common_zp": lambda: _common_zp(W.int4_decode(7, 512, 160), -77, W.S8),
+    "f32_scales_u4_zp": lambda: _scales(W.int4_decode(12, 640, 160, group=64), W.F32),
+    "f16_scales": lambda: _scales(W.int4_decode(8, 640, 160), W.F16),
+    "f8_scales": lambda: _scales(W.int4_decode(3, 512, 160, with_zp=False), W.F8_E4M3),
+    "large_f32_scales": _large_scales,
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_matches_oracle(gpu, name):
+    eng, strm = gpu
+    p = CASES[name]()
+    got, impl = run_problem(p, eng, strm)
+    assert impl == "cuda:tcgen05:woq4"
+    assert_parity(got, O.run_port(p), p.dst_dt, name, summation_slack(p))
+    got2, _ = run_problem(p, eng, strm)  # the shares are added in the same order every time
+    assert np.array_equal(got, got2)
+
+
+def test_calls_in_a_row_see_each_other_s_results(gpu):
+    """The kernel starts before its predecessor on the stream has ended: a chain of calls, each reading what the one
+    before it wrote, gives what the calls give one at a time."""
+    import torch
+    from onednn_b200.runner import Prepared
+    eng, strm = gpu
+    n = 1024
+    p = W.int4_decode(4, n, n)
+    first = Prepared(p, eng)
+    dev = torch.device("cuda:0")
+    put = lambda a: torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1).copy()).to(dev)
+    fixed = {"wei": put(p.wei.data), **{k: put(q.data) for k, q in p.quant.items()}}
+    # small weights keep the values of the chain in range
+    bufs = [put(p.src.data)] + [torch.zeros(4 * n * 2, dtype=torch.uint8, device=dev) for _ in range(6)]
+
+    def bound(i):
+        r = first if i == 0 else Prepared(p, eng)
+        r.bind_device({"src": bufs[i].data_ptr(), "dst": bufs[i + 1].data_ptr(), **{k: t.data_ptr() for k, t in fixed.items()}})
+        return r
+
+    calls = [bound(i) for i in range(6)]
+    torch.cuda.synchronize()
+    for r in calls:
+        r.execute(strm)
+        strm.wait()
+    want = [b.cpu().numpy().copy() for b in bufs[1:]]
+    for _ in range(5):
+        for b in bufs[1:]:
+            b.zero_()
+        torch.cuda.synchronize()
+        for r in calls:
+            r.execute(strm)
+        strm.wait()
+        for b, w in zip(bufs[1:], want):
+            assert np.array_equal(b.cpu().numpy(), w)
