@@ -13,6 +13,7 @@
 // dim order (the quantization of weights and activations before a matmul) a
 // thread takes four neighbours with 16-byte loads and one packed store.
 #include <cstdio>
+#include <type_traits>
 
 #include "device_math.cuh"
 #include "launch.h"
@@ -45,6 +46,7 @@ struct ReorderArgs {
     float beta;
 };
 
+__device__ __forceinline__ void ptx_grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ bool dt_is_int(int dt) { return dt == DT_S32 || dt == DT_S8 || dt == DT_U8; }
 
 __device__ __forceinline__ unsigned quantize_nibble(float v, bool sgn) {
@@ -248,8 +250,7 @@ __global__ void __launch_bounds__(256) reorder_dense4_kernel(const __grid_consta
 // along the contiguous dim and that have no sum: four rows in flight per thread, conversions
 // without run-time type switches.  This is the quantization / dequantization of a weight or
 // activation matrix with per-tensor or per-column parameters.
-// RCP: s8 / u8 results by a reciprocal per column instead of a division per element, see there.
-template <int SDT, int DDT, bool RCP = false>
+template <int SDT, int DDT>
 __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constant__ ReorderArgs a) {
     const int dst_zp = a.dst_zp ? __ldg(a.dst_zp) : 0;
     const int d0 = a.order[0];
@@ -270,37 +271,8 @@ __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constan
                               : 0;
     }
     const bool has_ds = a.dst_scale.ptr != nullptr, has_zp = a.dst_zp != nullptr;
-    // s8 / u8 results need the quotient's integer only.  q = d * (1 / scale) lies within 2^-22 |q| of the divided
-    // value (a reciprocal in the normal range, rounded once, and one more rounding), so unless q is that close to
-    // half an integer both round alike; beyond the range both saturate alike.  Everything else (one warp pass in
-    // some twenty for uniform values, NaN, unusable reciprocals) divides.  The divisions of every element took
-    // 65 % of the issue slots while DRAM stood at 47 %; the launch says where this form is taken.
-    float rc[4];
-    if constexpr (RCP) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            rc[e] = __frcp_rn(ds[e]);
-            if (!(fabsf(rc[e]) >= 1.17549435e-38f && fabsf(rc[e]) <= 3.0e38f)) rc[e] = __int_as_float(0x7fffffff); // NaN
-        }
-    }
     auto convert = [&](const float (&f)[4], const int (&iv)[4], int64_t off) {
         float out[4];
-        if constexpr (RCP) {
-            float worst = 0.f; // largest distance of a quotient from its integer
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float diff = dt_is_int(SDT) ? (float)(iv[e] - zps[e]) : __fsub_rn(f[e], (float)zps[e]);
-                out[e] = __fmul_rn(__fmul_rn(ss[e], diff), rc[e]);
-                // (inside +-300 the sum with 1.5 * 2^23 leaves the nearest integer; results beyond saturate)
-                const float q = fminf(fmaxf(out[e], -300.f), 300.f);
-                const float t = fabsf(q - ((q + 12582912.f) - 12582912.f));
-                worst = out[e] == out[e] ? fmaxf(worst, t) : 1.f;
-            }
-            if (worst < 0.4998f) {
-                store4(DDT, out, a.dst, off);
-                return;
-            }
-        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float diff = dt_is_int(SDT) ? (float)(iv[e] - zps[e]) : __fsub_rn(f[e], (float)zps[e]);
@@ -325,6 +297,96 @@ __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constan
         int iv[4];
         load4(SDT, a.src, r * cols + i0, f, iv);
         convert(f, iv, r * cols + i0);
+    }
+}
+
+// Quantization proper: f32 / bf16 / f16 to s8 / u8 with dst scales that vary along the contiguous dim at most, no sum and no
+// dst zero-point.  The result needs the integer next to the IEEE quotient d / scale.  d is first cut to what saturates
+// (products of the scale with the type's ends; a NaN becomes the lower one, as the general kernels' clamp makes it), so
+// that product by a reciprocal taken once, exact remainder and correction (Markstein) neither over- nor underflow: the
+// correctly rounded quotient in three operations.  (Checked against the division for every significand of the scale and the
+// dividends around every half-integer up to 255.5: no difference.)  Adding 1.5 * 2^23 rounds it to the integer in the low
+// byte.  Scales outside [2^-100, 2^100], negative ones and NaN divide.
+// Bound by the stream: 4 rows of 16 bytes (f32) or 8 of 8 in flight per thread, one wave of CTAs, equal shares, a ragged end
+// read four (eight) rows at a time too.  us a call, division or reciprocal and check -> now: f32 4096 x 14336 67.6 -> 48.1
+// (6.1 of 6.56 TB/s measured copy bandwidth), 2936 x 7192 30.8 -> 20.7, 904 x 968 8.2 -> 4.1;
+// bf16 5646 x 8896 63.5 -> 37.3, 826 x 7696 12.6 -> 7.2.
+constexpr int quantize_ctas(int sdt, bool ss) { return sdt == DT_F32 && !ss ? 5 : 4; } // per SM: what the registers allow
+template <int SDT, int DDT, bool SS>
+__global__ void __launch_bounds__(256, quantize_ctas(SDT, SS)) reorder_quantize_kernel(const __grid_constant__ ReorderArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    constexpr float LO = DDT == DT_S8 ? -128.f : 0.f, HI = DDT == DT_S8 ? 127.f : 255.f;
+    constexpr int U = SDT == DT_F32 ? 4 : 8; // rows in flight
+    const int d0 = a.order[0];
+    const int64_t cols = a.dims[d0], rows = a.work * 4 / cols;
+    const int tx = a.tx, ty = 256 / tx;
+    const int64_t i0 = ((int64_t)blockIdx.x * tx + threadIdx.x % tx) * 4;
+    const int64_t walkers = (int64_t)gridDim.y * ty;
+    int64_t r = (int64_t)blockIdx.y * ty + threadIdx.x / tx;
+    ptx_grid_dependency_wait();
+    if (i0 >= cols) return;
+    float ss[SS ? 4 : 1], ds[4], rc[4], lo[4], hi[4];
+    bool usual = true;
+    if (a.dst_scale.str[d0] == 1 && (uintptr_t)a.dst_scale.ptr % 16 == 0) { // one per column, dense
+        const float4 v = __ldg((const float4 *)a.dst_scale.ptr + (i0 >> 2));
+        ds[0] = v.x; ds[1] = v.y; ds[2] = v.z; ds[3] = v.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ds[e] = __ldg((const float *)a.dst_scale.ptr + (i0 + e) * a.dst_scale.str[d0]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (SS) ss[SS ? e : 0] = load_float(a.src_scale.dt, a.src_scale.ptr, ((i0 + e) / a.src_scale.grp[d0]) * a.src_scale.str[d0]);
+        usual &= ds[e] >= 7.8886091e-31f && ds[e] <= 1.2676506e30f; // 2^-100, 2^100
+        rc[e] = __frcp_rn(ds[e]);
+        lo[e] = LO * ds[e];
+        hi[e] = HI * ds[e];
+    }
+    auto convert = [&](float (&f)[4]) -> unsigned {
+        unsigned t[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (SS) f[e] = __fmul_rn(ss[SS ? e : 0], f[e]);
+            const float d = fminf(fmaxf(f[e], lo[e]), hi[e]);
+            const float q = d * rc[e];
+            const float rem = fmaf(-q, ds[e], d);
+            t[e] = __float_as_uint(fmaf(rem, rc[e], q) + 12582912.f);
+        }
+        return __byte_perm(__byte_perm(t[0], t[1], 0x0040), __byte_perm(t[2], t[3], 0x0040), 0x5410);
+    };
+    auto divide = [&](float (&f)[4]) -> unsigned {
+        unsigned w = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (SS) f[e] = __fmul_rn(ss[SS ? e : 0], f[e]);
+            const float v = fminf(fmaxf(__fdiv_rn(f[e], ds[e]), LO), HI);
+            w |= ((unsigned)__float2int_rn(v) & 0xffu) << (8 * e);
+        }
+        return w;
+    };
+    // (kept as read until they are converted: 16-bit rows take half the registers, and twice as many are in flight)
+    using raw_t = typename std::conditional<SDT == DT_F32, uint4, uint2>::type;
+    for (; r < rows; r += U * walkers) {
+        raw_t raw[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (r + u * walkers < rows) raw[u] = __ldg((const raw_t *)a.src + (((r + u * walkers) * cols + i0) >> 2));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            float f[4];
+            if constexpr (SDT == DT_F32) {
+                f[0] = __uint_as_float(raw[u].x); f[1] = __uint_as_float(raw[u].y);
+                f[2] = __uint_as_float(raw[u].z); f[3] = __uint_as_float(raw[u].w);
+            } else if constexpr (SDT == DT_BF16) {
+                f[0] = __uint_as_float(raw[u].x << 16); f[1] = __uint_as_float(raw[u].x & 0xffff0000u);
+                f[2] = __uint_as_float(raw[u].y << 16); f[3] = __uint_as_float(raw[u].y & 0xffff0000u);
+            } else {
+                const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(&raw[u].x)), w = __half22float2(*reinterpret_cast<const __half2 *>(&raw[u].y));
+                f[0] = v.x; f[1] = v.y; f[2] = w.x; f[3] = w.y;
+            }
+            if (r + u * walkers < rows)
+                ((unsigned *)a.dst)[((r + u * walkers) * cols + i0) >> 2] = usual ? convert(f) : divide(f);
+        }
     }
 }
 
@@ -392,8 +454,15 @@ reorder_kernel_fn cols4_for_dst(int ddt) {
         default: return nullptr;
     }
 }
-reorder_kernel_fn cols4_kernel(int sdt, int ddt, bool rcp) {
-    if (rcp) return ddt == DT_S8 ? reorder_cols4_kernel<DT_F32, DT_S8, true> : reorder_cols4_kernel<DT_F32, DT_U8, true>;
+template <int SDT>
+reorder_kernel_fn quantize_for_dst(int ddt, bool ss) {
+    if (ddt == DT_S8) return ss ? reorder_quantize_kernel<SDT, DT_S8, true> : reorder_quantize_kernel<SDT, DT_S8, false>;
+    return ss ? reorder_quantize_kernel<SDT, DT_U8, true> : reorder_quantize_kernel<SDT, DT_U8, false>;
+}
+reorder_kernel_fn quantize_kernel(int sdt, int ddt, bool ss) {
+    return sdt == DT_F32 ? quantize_for_dst<DT_F32>(ddt, ss) : sdt == DT_BF16 ? quantize_for_dst<DT_BF16>(ddt, ss) : quantize_for_dst<DT_F16>(ddt, ss);
+}
+reorder_kernel_fn cols4_kernel(int sdt, int ddt) {
     switch (sdt) {
         case DT_F32: return cols4_for_dst<DT_F32>(ddt);
         case DT_BF16: return cols4_for_dst<DT_BF16>(ddt);
@@ -637,15 +706,37 @@ dnnl_status_t qmm::execute_reorder(const dnnl_primitive_desc &pd, dnnl_stream_t 
             const int d = a.order[k];
             outer |= a.src_scale.str[d] != 0 || a.dst_scale.str[d] != 0 || a.src_zp.str[d] != 0;
         }
-        // Reciprocals cost four divisions of their own and the check of every quotient, so a thread has to walk
-        // enough rows, and there is nothing to gain where the src is not f32.  us a call, division -> reciprocal, f32 to
-        // s8: 2048 x 2048 (3 rows a thread) 12.8 -> 14.3, 2048 x 4096 (7) 17.7 -> 18.4, 4096 x 4096 (14) 24.7 both,
-        // 4096 x 8192 (28) 41.2 -> 39.4, 4096 x 14336 (48) 71.8 -> 67.6; bf16: 41.1 -> 42.3 and 69.9 -> 70.5 at the last two.
-        const bool rcp = a.src_dt == DT_F32 && (a.dst_dt == DT_S8 || a.dst_dt == DT_U8) && a.dst_scale.ptr && !a.dst_zp
-                && rows >= 16 * gy * ty;
-        reorder_kernel_fn typed = (!outer && a.beta == 0.f) ? cols4_kernel(a.src_dt, a.dst_dt, rcp) : nullptr;
-        if (typed) typed<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, stream->stream>>>(a);
-        else reorder_dense4_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, stream->stream>>>(a);
+        const bool plain_params = !outer && a.beta == 0.f;
+        reorder_kernel_fn typed = nullptr;
+        if (plain_params && (a.src_dt == DT_F32 || a.src_dt == DT_BF16 || a.src_dt == DT_F16) && (a.dst_dt == DT_S8 || a.dst_dt == DT_U8)
+                && a.dst_scale.ptr && !a.dst_zp && !a.src_zp.ptr) {
+            // the widest row of threads that wastes the fewest lanes beyond the columns, then one wave of equal shares
+            int64_t best = INT64_MAX;
+            for (int t = 256; t >= 32; t /= 2) {
+                const int64_t lanes = (cols / 4 + t - 1) / t * t;
+                if (lanes < best) { best = lanes; a.tx = t; }
+            }
+            const int64_t tyq = 256 / a.tx, gxq = (cols / 4 + a.tx - 1) / a.tx;
+            int64_t gyq = (int64_t)sms * quantize_ctas(a.src_dt, a.src_scale.ptr != nullptr) / gxq;
+            if (gyq > (rows + tyq - 1) / tyq) gyq = (rows + tyq - 1) / tyq;
+            if (gyq > 65535) gyq = 65535;
+            if (gyq < 1) gyq = 1;
+            cudaLaunchConfig_t cfg {};
+            cfg.gridDim = dim3((unsigned)gxq, (unsigned)gyq);
+            cfg.blockDim = dim3(256);
+            cfg.stream = stream->stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            void *kargs[] = {&a};
+            cudaLaunchKernelExC(&cfg, (const void *)quantize_kernel(a.src_dt, a.dst_dt, a.src_scale.ptr != nullptr), kargs);
+        } else if (plain_params && (typed = cols4_kernel(a.src_dt, a.dst_dt))) {
+            typed<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, stream->stream>>>(a);
+        } else {
+            reorder_dense4_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, stream->stream>>>(a);
+        }
     } else {
         // a matrix (or a batch of matrices) whose contiguous dim changes: the tiled kernel
         int dr = -1, dc = -1;
