@@ -1,4 +1,5 @@
-// int4 weight-decompression matmul for few rows (token generation, M <= 32):
+// int4 weight-decompression matmul for few rows (token generation; more rows where woq_rows.cu would leave SMs idle or
+// pay for small groups):
 //   dst[M,N] = src[M,K] (bf16/f16) x dequant(weights[K,N] s4/u4 `ab`),
 // scales per column or per (K-group, column), optional zero-points (fpmath
 // apply_to_int; reference arithmetic: src/cpu/matmul/ref_matmul.cpp:193-233).
@@ -67,6 +68,7 @@ struct WdCfg {
 struct WdParams {
     int ksteps; // K / 16
     int kstages; // ceil(K / 64)
+    int rows; // src rows per CTA (at most 32)
     int group_steps; // k16 steps per quantization group (ksteps when not grouped along K)
     int sc_grouped; // scales have a row per group (else one row)
     int split_log; // log2 of the CTAs per tile = cluster size
@@ -227,7 +229,7 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     uint64_t *empty = full + MAX_STAGES, *sums_bar = empty + MAX_STAGES;
     const int warp = threadIdx.x / 32, lane = in_reg(threadIdx.x % 32);
     const int split_log = p.split_log, splits = 1 << split_log, rank = (int)blockIdx.x & (splits - 1), tile = (int)blockIdx.x >> split_log;
-    const int M = (int)a.M;
+    const int m0 = (int)blockIdx.y * p.rows, M = min(p.rows, (int)a.M - m0); // this CTA's rows
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
             ptx::mbar_init(&full[s], 1);
@@ -276,7 +278,7 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                     rows = r + (last - first) <= group_steps ? 1 : (r + (last - first) + group_steps - 1) / group_steps;
                 arrive_expect_tx(bar, W_BYTES + C::S_BYTES + rows * (sc_bytes + zp_bytes));
                 tma_load(sw, map_w, bar, n0 / 2, st * KS);
-                tma_load(sw + W_BYTES, map_s, bar, st * KS, 0);
+                tma_load(sw + W_BYTES, map_s, bar, st * KS, m0);
                 const char *sc = sc_row, *zp = zp_row;
                 for (int i = 0; i < rows; ++i) {
                     bulk_load(sw + off_sc + i * sc_pitch, sc, sc_bytes, bar);
@@ -547,9 +549,9 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             if (a.bias) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    d[e] = __fadd_rn(d[e], load_float(a.bias_dt, a.bias, m * a.bias_sm + (n + e) * a.bias_sn));
+                    d[e] = __fadd_rn(d[e], load_float(a.bias_dt, a.bias, (m0 + m) * a.bias_sm + (n + e) * a.bias_sn));
             }
-            const int64_t o = (int64_t)m * a.dst_sm + n;
+            const int64_t o = (int64_t)(m0 + m) * a.dst_sm + n;
             if (a.dst_dt == DT_F32) {
                 *reinterpret_cast<float4 *>((float *)a.dst + o) = make_float4(d[0], d[1], d[2], d[3]);
             } else if (a.dst_dt == DT_BF16) {
@@ -565,7 +567,7 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             }
         } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) finish_store_cold(a, d[e], m, n + e);
+            for (int e = 0; e < 4; ++e) finish_store_cold(a, d[e], m0 + m, n + e);
         }
     }
 }
@@ -606,11 +608,11 @@ int wd_rows_per_stage(int group_steps) {
 // CTA's start and end count as 2 + mt stages, and a stage that has the SM to itself takes as long as 2.75 - mt / 4 that
 // share it.  us a call with 1 / 2 / 4 / 8 CTAs per tile: K = 8192, N = 28672, M = 1: 50.4 / 39.4 / 36.8 / 35.1 (8 chosen),
 // M = 32: 106 / 82.4 / 87.2 / 91.0 (2); M = 13, 4096 x 11008: - / 17.5 / 16.3 / 11.7 (8); M = 8, 1280 x 7008: - / 7.2 / 5.9 / 6.2 (8).
-int wd_split_log(int ntiles, int kstages, int mt, int sm_count) {
+int wd_split_log(int64_t ntiles, int kstages, int mt, int sm_count) {
     int best = 0;
     int64_t cost = INT64_MAX;
     for (int l = 0; 1 << l <= MAX_CLUSTER && 1 << l <= kstages; ++l) {
-        const int64_t busiest = (((int64_t)ntiles << l) + sm_count - 1) / sm_count;
+        const int64_t busiest = ((ntiles << l) + sm_count - 1) / sm_count;
         const int64_t share = 4 * busiest > 11 - mt ? 4 * busiest : 11 - mt; // in quarters
         const int64_t c = share * (((kstages + (1 << l) - 1) >> l) + 2 + mt);
         if (c < cost) { cost = c; best = l; }
@@ -627,7 +629,7 @@ int wd_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a,
     p.off_sc = W_BYTES + C::S_BYTES;
     p.off_zp = p.off_sc + up128(rb * NB * p.sc_bits / 8);
     p.stage_bytes = (p.off_zp + up128(rb * NB * p.zp_bits / 8) + 1023) / 1024 * 1024;
-    const int sums_bytes = (int)a.M * NB * 4;
+    const int sums_bytes = p.rows * NB * 4;
     // as many stages as the CTA's share of the SM holds; four where wide parameter rows leave fewer (then fewer CTAs fit an SM)
     p.stages = (C::SMEM - BAR_BYTES - sums_bytes) / p.stage_bytes;
     p.stages = p.stages > MAX_STAGES ? MAX_STAGES : p.stages < 4 ? 4 : p.stages;
@@ -637,7 +639,7 @@ int wd_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a,
     static std::atomic<unsigned long long> configured;
     if (!opt_in_dynamic_smem(kern, SMEM_PER_SM, configured)) return 5;
     cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3((unsigned)ntiles << p.split_log);
+    cfg.gridDim = dim3((unsigned)ntiles << p.split_log, (unsigned)((a.M + p.rows - 1) / p.rows));
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = (size_t)smem_bytes;
     cfg.stream = st;
@@ -688,12 +690,23 @@ bool woq_decode_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_d
     return M <= 16 || rb * NB * (wd_bits(scale_dt) + (zp_dt < 0 ? 0 : wd_bits(zp_dt))) / 8 < W_BYTES;
 }
 
+// Microseconds that a problem takes here, for the choice between this kernel and the one whose operand lies in tensor
+// memory (woq_rows.cu) when there are more than 32 rows: a stage costs an SM 0.82 for blocks of 32 rows (0.65 for 24), more
+// with small groups (a fold of the sums at each end), and the launch about 4.
+float woq_decode_us(int64_t M, int64_t N, int64_t K, int64_t group, int sm_count) {
+    const int64_t blocks = (M + 31) / 32, rows = (M + blocks - 1) / blocks;
+    const float stage = (rows > 24 ? 0.82f : 0.65f) * (group < 64 ? 1.35f : group < 128 ? 1.1f : 1.f);
+    const int64_t stages = blocks * ((N + NB - 1) / NB) * ((K + KS - 1) / KS);
+    const float share = (float)stages / (float)(sm_count > 0 ? sm_count : 148), alone = (float)((K + KS - 1) / KS) / MAX_CLUSTER * 1.3f;
+    return 4.f + stage * (share > alone ? share : alone);
+}
+
 int launch_woq_decode(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     if (a.M == 0 || a.N == 0) return 0;
-    if (a.M > 32) return 3;
     encode_tiled_fn enc = wd_get_encode();
     if (!enc) return 5;
-    const int mt = (int)(a.M + 7) / 8;
+    // more than 32 rows: equal blocks of them, each with CTAs of its own that read the weights again (from L2)
+    const int blocks = (int)((a.M + 31) / 32), rows = (int)((a.M + blocks - 1) / blocks), mt = (rows + 7) / 8;
     CUtensorMap tw, ts;
     {
         cuuint64_t dims[2] = {(cuuint64_t)(a.N / 2), (cuuint64_t)a.K};
@@ -721,6 +734,7 @@ int launch_woq_decode(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     WdParams p {};
     p.ksteps = (int)((a.K + 15) / 16);
     p.kstages = (int)((a.K + KS - 1) / KS);
+    p.rows = rows;
     p.sc_grouped = a.wei_scale.mask & 1;
     const bool zp_rows = a.wei_zp.ptr && a.wei_zp.mask;
     const int64_t group = p.sc_grouped ? a.wei_scale.g0 : (zp_rows && (a.wei_zp.mask & 1)) ? a.wei_zp.g0 : a.K;
@@ -740,7 +754,7 @@ int launch_woq_decode(const MatmulArgs &a, int sm_count, cudaStream_t st) {
                 && (a.M == 1 || a.dst_sm % 4 == 0) && (uintptr_t)a.dst % (4 * es) == 0;
     }
     const int ntiles = (int)((a.N + NB - 1) / NB);
-    p.split_log = wd_split_log(ntiles, p.kstages, mt, sm_count > 0 ? sm_count : 148);
+    p.split_log = wd_split_log(ntiles * blocks, p.kstages, mt, sm_count > 0 ? sm_count : 148);
     const bool f16 = a.src_dt == DT_F16;
 #define QMM_WD(MT) (f16 ? wd_choose<MT, true>(tw, ts, a, p, zpm, ntiles, st) : wd_choose<MT, false>(tw, ts, a, p, zpm, ntiles, st))
     return mt == 1 ? QMM_WD(1) : mt == 2 ? QMM_WD(2) : mt == 3 ? QMM_WD(3) : QMM_WD(4);

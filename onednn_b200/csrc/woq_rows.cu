@@ -33,7 +33,7 @@
 //   M = 128         136    76    43    35
 //   M = 300         116    70    43    36
 //   M = 512         137    77    44    37
-// 32 tiles and 96 at M = 64 and 300 leave SMs idle: K is not split.  300 rows in groups of 128 without zero-points 37;
+// 32 tiles and 96 at M = 64 and 300 leave SMs idle: K is not split (launch_woq_rows says what goes to woq_decode.cu).  300 rows in groups of 128 without zero-points 37;
 // the generic kernel takes 54.3 ms for them.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -628,6 +628,21 @@ int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     encode_tiled_fn enc = rows_get_encode();
     if (!enc) return 5;
     if (sm_count < 1) sm_count = 148;
+    const int64_t group = (a.wei_scale.ptr && (a.wei_scale.mask & 1)) ? a.wei_scale.g0
+            : (a.wei_zp.ptr && (a.wei_zp.mask & 1))                    ? a.wei_zp.g0
+                                                                       : a.K;
+    {
+        // The decode kernel in blocks of up to 32 rows, where it is the faster one.  This kernel takes 0.45 us a stage of a wave
+        // of tiles, and 0.8 more for every group end in it; nothing splits its K.
+        // us a call, this kernel -> that one: 64 x 4096 x 4096 in groups of 128 37.9 -> 18.7, of 32 104 -> 29.3; 128 rows, f16, groups of
+        // 64 71.7 -> 29.2; 300 rows, groups of 32 99 -> 87; 40 x 8192 x 1024 66.6 -> 11.8; 48 x 8192 x 28672 139 -> 105;
+        // 300 x 4096 x 4096 in groups of 128 stays here (40.6).
+        const int64_t waves = ((a.M + RT_M - 1) / RT_M * ((a.N + RT_N - 1) / RT_N) + sm_count - 1) / sm_count;
+        const float here = 4.f + (float)(waves * ((a.K + RK - 1) / RK)) * (0.45f + 102.f / (float)(group < 4 * RK ? group : 4 * RK));
+        if (a.M <= 65536 && woq_decode_pointers_ok(a) && woq_decode_fits(a.M, a.K, group, a.wei_scale.dt, a.wei_zp.ptr && a.wei_zp.mask ? a.wei_zp.dt : -1)
+                && woq_decode_us(a.M, a.N, a.K, group, sm_count) < here)
+            return launch_woq_decode(a, sm_count, st);
+    }
     RowsParams p {};
     // as few row tiles as cover M, of equal size
     p.num_m_tiles = (int)((a.M + RT_M - 1) / RT_M);
@@ -660,9 +675,6 @@ int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     }
     p.ksteps = (int)(a.K / 16);
     p.kstages = (int)((a.K + RK - 1) / RK);
-    const int64_t group = (a.wei_scale.ptr && (a.wei_scale.mask & 1)) ? a.wei_scale.g0
-            : (a.wei_zp.ptr && (a.wei_zp.mask & 1))                    ? a.wei_zp.g0
-                                                                       : a.K;
     p.group_steps = (int)(group / 16);
     if (p.group_steps < 1 || p.group_steps > p.ksteps) p.group_steps = p.ksteps;
     p.sgn4 = a.wei_dt == DT_S4;

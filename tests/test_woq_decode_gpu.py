@@ -73,6 +73,33 @@ def test_matches_oracle(gpu, name):
     assert np.array_equal(got, got2)
 
 
+ROWS_CASES = {
+    # blocks of rows of the decode kernel: 2 x 17, 2 x 32, 3 x 22 with a short last one, ...
+    "m33": lambda: W.int4_decode(33, 1024, 288),
+    "m64_group32": lambda: W.int4_decode(64, 512, 160, group=32),
+    "m65_f16": lambda: W.int4_decode(65, 768, 544, wei_dt=W.U4, src_dt=W.F16, dst_dt=W.F16, group=64),
+    "m97_k_tail": lambda: W.int4_decode(97, 1104, 96, group=16),
+    # enough tiles and short K for the kernel with the operand in tensor memory
+    "m1000_group128": lambda: W.int4_decode(1000, 512, 1056),
+    "m2040_group64": lambda: W.int4_decode(2040, 256, 1024, group=64),
+    "m2048_group32_u4": lambda: W.int4_decode(2048, 256, 1024, group=32, wei_dt=W.U4),
+    "m2000_group48": lambda: W.int4_decode(2000, 288, 1024, group=48),
+    "m1024_f16_u8zp": lambda: W.int4_decode(1024, 512, 1024, group=256, zp_dt=W.U8, src_dt=W.F16, dst_dt=W.F16),
+    "m1024_no_zp": lambda: W.int4_decode(1024, 528, 1024, group=528, with_zp=False, dst_dt=W.F32),
+}
+
+
+@pytest.mark.parametrize("name", sorted(ROWS_CASES))
+def test_more_rows_match_oracle(gpu, name):
+    eng, strm = gpu
+    p = ROWS_CASES[name]()
+    got, impl = run_problem(p, eng, strm)
+    assert impl == "cuda:tcgen05:woq4_rows"
+    assert_parity(got, O.run_port(p), p.dst_dt, name, summation_slack(p))
+    got2, _ = run_problem(p, eng, strm)
+    assert np.array_equal(got, got2)
+
+
 def test_calls_in_a_row_see_each_other_s_results(gpu):
     """The kernel starts before its predecessor on the stream has ended: a chain of calls, each reading what the one
     before it wrote, gives what the calls give one at a time."""
