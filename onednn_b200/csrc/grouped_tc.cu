@@ -566,6 +566,7 @@ bool grouped_tc_pointers_ok(const MatmulArgs &a) {
 // weight scales, bf16 / f16 / f32 dst.  `scratch`: grouped_tc_scratch_bytes(group_count) bytes.
 int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStream_t st) {
     if (a.M == 0 || a.N == 0) return 0;
+    if (woq8_decode_wins(a, sm_count)) return launch_woq8_decode(a, sm_count, st); // few rows
     encode_tiled_fn enc = grouped_get_encode();
     if (!enc || !scratch) return 5;
     CUtensorMap tw, ts, ts2, ts3;

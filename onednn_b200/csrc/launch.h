@@ -57,6 +57,10 @@ bool woq_decode_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_d
 int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st);
 bool woq_rows_pointers_ok(const MatmulArgs &a);
 
+// s8 weight decompression for few rows, dense and grouped (woq8_decode.cu)
+int launch_woq8_decode(const MatmulArgs &a, int sm_count, cudaStream_t st);
+bool woq8_decode_wins(const MatmulArgs &a, int sm_count);
+
 // tcgen05 grouped (MoE) GEMM, bf16 src x s8 weights (grouped_tc.cu).
 // `scratch`: grouped_tc_scratch_bytes(group_count, M) bytes, no initialisation
 // (tile ranges per group, and the src row sums that weight zero-points need).

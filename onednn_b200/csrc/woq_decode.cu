@@ -40,7 +40,7 @@
 #include "device_math.cuh"
 #include "launch.h"
 #include "objects.hpp"
-#include "sm100_ptx.cuh"
+#include "decode_ptx.cuh"
 
 namespace qmm {
 
@@ -80,135 +80,6 @@ struct WdParams {
     int off_bars;
 };
 
-__device__ __forceinline__ uint32_t and_xor(uint32_t x, uint32_t mask, uint32_t magic) { // (x & mask) ^ magic
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(r) : "r"(x), "r"(mask), "r"(magic));
-    return r;
-}
-__device__ __forceinline__ uint32_t perm(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
-template <bool F16>
-__device__ __forceinline__ uint32_t fma2(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    if (F16) asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    else asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-template <bool F16>
-__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    if (F16)
-        asm volatile(
-                "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-    else
-        asm volatile(
-                "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// src fragments of a k16 step, two words per block of 8 rows
-__device__ __forceinline__ void ldsm_x4(uint32_t *r, uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr)
-                 : "memory");
-}
-__device__ __forceinline__ void ldsm_x2(uint32_t *r, uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-    uint32_t r;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(addr) : "memory");
-    return r;
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-// a kernel parameter held in a register: the parameter block is 3 KB and the constant cache small
-__device__ __forceinline__ int in_reg(int v) {
-    int r;
-    asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(v));
-    return r;
-}
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, int rank) { // the same place in another CTA of the cluster
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w, uint32_t bar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(x),
-                 "r"(y), "r"(z), "r"(w), "r"(bar)
-                 : "memory");
-}
-// The loops keep shared-memory addresses in registers: one taken from a pointer is made from a special register
-// (the CTA's place in its cluster) each time, which is slow to read.
-__device__ __forceinline__ uint32_t try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-    return ok;
-}
-// Bounded by 2 s, as ptx::mbar_wait.  Between polls the warp sleeps: the producers of an SM wait for most of the time
-// (their rings are full), and without it their polls were a third of the instructions issued.
-template <int NS>
-__device__ __noinline__ bool wait_long(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < 1024; ++i) {
-        if (try_wait(bar, parity)) return true;
-        __nanosleep(NS);
-    }
-    const uint64_t t0 = ptx::globaltimer();
-    while (!try_wait(bar, parity)) {
-        __nanosleep(NS);
-        if (ptx::globaltimer() - t0 > 2000000000ull) return false;
-    }
-    return true;
-}
-template <int NS>
-__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity) { return try_wait(bar, parity) || wait_long<NS>(bar, parity); }
-__device__ __forceinline__ void arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load(uint32_t dst, uint64_t map, uint32_t bar, int x, int y) {
-    asm volatile(
-            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
-            "r"(bar), "r"(x), "r"(y)
-            : "memory");
-}
-// global -> shared, 16-byte multiples
-__device__ __forceinline__ void bulk_load(uint32_t dst, const char *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
-                 "r"(bar)
-                 : "memory");
-}
 __device__ __noinline__ void finish_store_cold(const MatmulArgs &a, float d, int64_t m, int64_t n) {
     if (a.bias) d = __fadd_rn(d, load_float(a.bias_dt, a.bias, m * a.bias_sm + n * a.bias_sn));
     finish_store(a, d, m, n, false);
