@@ -140,20 +140,12 @@ __device__ __forceinline__ Tile decode_tile(const int4 *plan, int groups, bool l
 // call, 208 -> 192: dense, 4096 rows, K = N = 1024 48.3 -> 45.2; 1940 rows, K = 592, N = 4400 65.7 -> 61.5;
 // 8 experts, 8192 rows, K = N = 1024 69.8 -> 65.3 (the last with the scale and the 64 in one product).
 //
-// One warp, a lane per group, in two walks over the groups: counts, then records.  (One thread that walked the groups
+// Grouped calls (dense ones: see launch_grouped_tc).  One warp, a lane per group, in two walks over the groups: counts, then records.  (One thread that walked the groups
 // with both counts took 1.8 us longer for 32 groups and 6 us for 64 than with one; its loads wait for one another.)
 __global__ void grouped_plan_kernel(const __grid_constant__ MatmulArgs a, int4 *plan, int num_n_tiles, int sms) {
     asm volatile("griddepcontrol.launch_dependents;"); // the main kernel may set itself up meanwhile; it waits before it reads the plan
     const int lane = threadIdx.x;
     auto waves = [&](int total) { return (total + sms - 1) / sms; };
-    if (a.group_count == 0) { // a dense problem: one group that owns every row
-        if (lane != 0) return;
-        const int tall = row_blocks((int)a.M, false) * num_n_tiles, low = row_blocks((int)a.M, true) * num_n_tiles;
-        const bool use_low = waves(low) == waves(tall);
-        plan[1] = make_int4(0, 0, (int)a.M, 0);
-        plan[0] = make_int4(use_low ? low : tall, 1, use_low, 0);
-        return;
-    }
     bool bad = false;
     // {first src row, first dst row, rows} of group g; an invalid group owns no rows
     auto group = [&](int g) {
@@ -246,12 +238,17 @@ __global__ void grouped_rowsum_kernel(const __grid_constant__ MatmulArgs a, floa
     if (threadIdx.x % 32 == 0) rowsum[m] = s;
 }
 
-template <bool EPI_CHAIN>
+// A dense problem is one group that owns every row: its plan comes from the host, without a planning kernel.
+struct DensePlan {
+    int4 head, group;
+};
+
+template <bool EPI_CHAIN, bool DENSE>
 __global__ void __launch_bounds__(G_THREADS, 1)
 grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
         const __grid_constant__ CUtensorMap tmS2, const __grid_constant__ CUtensorMap tmS3,
         const __grid_constant__ MatmulArgs a, const int4 *plan_global, const float *rowsum,
-        int num_k_blocks) {
+        int num_k_blocks, const __grid_constant__ DensePlan dense) {
     constexpr uint32_t TMEM_COLS = 512;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -296,16 +293,20 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     __syncthreads();
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_base_slot;
-    // launched as the programmatic dependent of the planning (or row-sum) kernel: everything above ran
-    // beside it; the plan and the row sums are read from here on
+    // launched as the programmatic dependent of the planning (or row-sum) kernel, or, dense, of whatever precedes it on the
+    // stream: everything above ran beside it; inputs, the plan and the row sums are read from here on
     ptx::grid_dependency_wait();
-    const int4 head = ptx::ld_dependent_int4(&plan_global[0]);
+    const int4 head = DENSE ? dense.head : ptx::ld_dependent_int4(&plan_global[0]);
     const int num_tiles = head.x, groups = head.y;
     const bool low_blocks = head.z != 0;
     const int4 *plan = plan_global;
     if (groups <= PLAN_CACHE_GROUPS) {
         int4 *cache = reinterpret_cast<int4 *>(smem + G_PLAN_OFFSET);
-        for (int i = threadIdx.x; i <= groups; i += blockDim.x) cache[i] = ptx::ld_dependent_int4(&plan_global[i]);
+        if constexpr (DENSE) {
+            if (threadIdx.x == 0) cache[1] = dense.group;
+        } else {
+            for (int i = threadIdx.x; i <= groups; i += blockDim.x) cache[i] = ptx::ld_dependent_int4(&plan_global[i]);
+        }
         __syncthreads();
         plan = cache;
     }
@@ -327,6 +328,10 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                 }
             }
             if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
+        }
+        if constexpr (DENSE) { // the successor may start (its set-up allocates tensor memory: every CTA of this grid has its own by now)
+            __syncwarp();
+            asm volatile("griddepcontrol.launch_dependents;");
         }
     } else if (warp == 2 + CONV_WARPS + EPI_WARPS) {
         // ------------------------------------------------ TMA producer of the src rows
@@ -600,8 +605,18 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
     const int num_k_blocks = (int)((a.K + LK - 1) / LK) * 2; // in pairs: k beyond K reads as zeros
     const int sms = sm_count > 0 ? sm_count : 148;
     int4 *plan = (int4 *)scratch;
-    grouped_plan_kernel<<<1, 32, 0, st>>>(a, plan, num_n_tiles, sms);
-    count_launch();
+    DensePlan dense {};
+    if (a.group_count > 0) {
+        grouped_plan_kernel<<<1, 32, 0, st>>>(a, plan, num_n_tiles, sms);
+        count_launch();
+    } else {
+        auto blocks = [&](int limit) { return (a.M + limit - 1) / limit * num_n_tiles; };
+        auto waves = [&](int64_t tiles) { return (tiles + sms - 1) / sms; };
+        const int64_t tall = blocks(GT_M), low = blocks(GT_M_LOW);
+        const bool use_low = waves(low) == waves(tall);
+        dense.head = make_int4((int)(use_low ? low : tall), 1, use_low, 0);
+        dense.group = make_int4(0, 0, (int)a.M, 0);
+    }
     float *rowsum = (float *)((char *)scratch + plan_bytes(a.group_count > 0 ? a.group_count : 1));
     if (a.wei_zp.ptr) {
         grouped_rowsum_kernel<<<(unsigned)((a.M + 7) / 8), 256, 0, st>>>(a, rowsum);
@@ -609,9 +624,11 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
     }
     // epilogue with zero-points / bias / post-ops: its own instantiation
     const bool chain = a.bias != nullptr || a.n_po > 0 || a.wei_zp.ptr != nullptr;
-    auto kern = chain ? grouped_tc_kernel<true> : grouped_tc_kernel<false>;
-    static std::atomic<unsigned long long> configured[2];
-    if (!opt_in_dynamic_smem(kern, G_SMEM_BYTES, configured[chain])) return 5;
+    const bool is_dense = a.group_count == 0;
+    auto kern = is_dense ? (chain ? grouped_tc_kernel<true, true> : grouped_tc_kernel<false, true>)
+                         : (chain ? grouped_tc_kernel<true, false> : grouped_tc_kernel<false, false>);
+    static std::atomic<unsigned long long> configured[4];
+    if (!opt_in_dynamic_smem(kern, G_SMEM_BYTES, configured[2 * is_dense + chain])) return 5;
     {
         cudaLaunchConfig_t cfg {};
         cfg.gridDim = dim3((unsigned)sms);
@@ -625,9 +642,9 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
         cfg.numAttrs = 1;
         const int4 *plan_c = plan;
         const float *rowsum_c = rowsum;
-        if (cudaLaunchKernelEx(&cfg, kern, tw, ts, ts2, ts3, a, plan_c, rowsum_c, num_k_blocks) != cudaSuccess) {
+        if (cudaLaunchKernelEx(&cfg, kern, tw, ts, ts2, ts3, a, plan_c, rowsum_c, num_k_blocks, dense) != cudaSuccess) {
             (void)cudaGetLastError(); // the attribute was refused: an ordinary launch
-            kern<<<sms, G_THREADS, G_SMEM_BYTES, st>>>(tw, ts, ts2, ts3, a, plan, rowsum, num_k_blocks);
+            kern<<<sms, G_THREADS, G_SMEM_BYTES, st>>>(tw, ts, ts2, ts3, a, plan, rowsum, num_k_blocks, dense);
         }
     }
     count_launch();
