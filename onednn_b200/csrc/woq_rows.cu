@@ -224,6 +224,8 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     __syncthreads();
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    // a programmatic dependent of whatever precedes it on the stream: what is above runs under the predecessor's end
+    ptx::grid_dependency_wait();
 
     // The three single-thread roles: one elected thread runs the whole loop.  A role's time per stage is its
     // chain of dependent instructions (about five cycles each), so these loops are kept short.
@@ -245,6 +247,9 @@ woq_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
             }
             if (!ok) { *abort_flag = 1; atomicExch(a.status, 5); }
         }
+        __syncwarp();
+        // the successor may start (its set-up allocates tensor memory: every CTA of this grid has its own by now)
+        asm volatile("griddepcontrol.launch_dependents;");
     } else if (warp == 1) {
         // ------------------------------------------------ TMA producer of the src tiles
         if (ptx::elect_one()) {
@@ -606,10 +611,20 @@ int rows_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &
     auto kern = woq_rows_kernel<F16, MULTI>;
     static std::atomic<unsigned long long> configured;
     if (!opt_in_dynamic_smem(kern, R_SMEM_BYTES, configured)) return 5;
-    kern<<<p.num_tiles < sm_count ? p.num_tiles : sm_count, R_THREADS, R_SMEM_BYTES, st>>>(tw, ts, a, p);
+    cudaLaunchConfig_t cfg {};
+    cfg.gridDim = dim3((unsigned)(p.num_tiles < sm_count ? p.num_tiles : sm_count));
+    cfg.blockDim = dim3((unsigned)R_THREADS);
+    cfg.dynamicSmemBytes = (size_t)R_SMEM_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, ts, a, p);
     count_launch();
-    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();
         set_last_error(std::string("cuda:tcgen05:woq4_rows launch: ") + cudaGetErrorString(e));
         return 5;
     }
