@@ -18,6 +18,7 @@
 #include "device_math.cuh"
 #include "launch.h"
 #include "objects.hpp"
+#include "sm100_ptx.cuh"
 
 using namespace qmm;
 
@@ -46,7 +47,6 @@ struct ReorderArgs {
     float beta;
 };
 
-__device__ __forceinline__ void ptx_grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ bool dt_is_int(int dt) { return dt == DT_S32 || dt == DT_S8 || dt == DT_U8; }
 
 __device__ __forceinline__ unsigned quantize_nibble(float v, bool sgn) {
@@ -311,6 +311,8 @@ __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constan
 // read four (eight) rows at a time too.  us a call, division or reciprocal and check -> now: f32 4096 x 14336 67.6 -> 48.1
 // (6.1 of 6.56 TB/s measured copy bandwidth), 2936 x 7192 30.8 -> 20.7, 904 x 968 8.2 -> 4.1;
 // bf16 5646 x 8896 63.5 -> 37.3, 826 x 7696 12.6 -> 7.2.
+// It starts before its predecessor on the stream has ended, which may be what writes the matrix and its scales: both are read
+// behind the wait, by loads that stay there (the other kernels of this file are ordinary launches and may use __ldg).
 constexpr int quantize_ctas(int sdt, bool ss) { return sdt == DT_F32 && !ss ? 5 : 4; } // per SM: what the registers allow
 template <int SDT, int DDT, bool SS>
 __global__ void __launch_bounds__(256, quantize_ctas(SDT, SS)) reorder_quantize_kernel(const __grid_constant__ ReorderArgs a) {
@@ -323,16 +325,16 @@ __global__ void __launch_bounds__(256, quantize_ctas(SDT, SS)) reorder_quantize_
     const int64_t i0 = ((int64_t)blockIdx.x * tx + threadIdx.x % tx) * 4;
     const int64_t walkers = (int64_t)gridDim.y * ty;
     int64_t r = (int64_t)blockIdx.y * ty + threadIdx.x / tx;
-    ptx_grid_dependency_wait();
+    ptx::grid_dependency_wait();
     if (i0 >= cols) return;
     float ss[SS ? 4 : 1], ds[4], rc[4], lo[4], hi[4];
     bool usual = true;
     if (a.dst_scale.str[d0] == 1 && (uintptr_t)a.dst_scale.ptr % 16 == 0) { // one per column, dense
-        const float4 v = __ldg((const float4 *)a.dst_scale.ptr + (i0 >> 2));
+        const float4 v = ptx::ld_dependent((const float4 *)a.dst_scale.ptr + (i0 >> 2));
         ds[0] = v.x; ds[1] = v.y; ds[2] = v.z; ds[3] = v.w;
     } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ds[e] = __ldg((const float *)a.dst_scale.ptr + (i0 + e) * a.dst_scale.str[d0]);
+        for (int e = 0; e < 4; ++e) ds[e] = ptx::ld_dependent((const float *)a.dst_scale.ptr + (i0 + e) * a.dst_scale.str[d0]);
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(256, quantize_ctas(SDT, SS)) reorder_quantize_
         raw_t raw[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (r + u * walkers < rows) raw[u] = __ldg((const raw_t *)a.src + (((r + u * walkers) * cols + i0) >> 2));
+            if (r + u * walkers < rows) raw[u] = ptx::ld_dependent((const raw_t *)a.src + (((r + u * walkers) * cols + i0) >> 2));
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             float f[4];

@@ -33,9 +33,11 @@ __device__ __forceinline__ bool elect_one() {
 // ---- programmatic dependent launch ----------------------------------------
 // Waits until the grids this one depends on have completed and their writes are visible.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Loads of what such a grid has written.  An ordinary or __ldg load may become a non-coherent one, which
-// the compiler is free to move above the wait (it takes the memory for constant while the kernel runs):
-// a planning kernel's output was then read before it existed, on a primitive's first execution.
+// What such a grid may have written - every tensor, scale, zero-point and offset that a caller passes, where a kernel is
+// a dependent of whatever precedes it on the stream - is read behind the wait with coherent loads: these, or ordinary ones,
+// which the wait's memory clobber holds back.  Never with __ldg, ld.global.nc or through a __restrict__ pointer, which say
+// that the memory is constant while the kernel runs: the compiler may move such a load above the wait (a planning
+// kernel's output was read before it existed, on a primitive's first execution), and the non-coherent path may serve old data.
 __device__ __forceinline__ int4 ld_dependent_int4(const int4 *p) {
     int4 v;
     asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
@@ -49,6 +51,22 @@ __device__ __forceinline__ int ld_dependent(const int *p) {
 __device__ __forceinline__ float ld_dependent(const float *p) {
     float v;
     asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+// (streams: volatile keeps them behind the wait and in order, and leaves the compiler's view of other memory alone)
+__device__ __forceinline__ float4 ld_dependent(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_dependent(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_dependent(const uint2 *p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
     return v;
 }
 

@@ -1,0 +1,152 @@
+"""Kernels that start before their predecessor on the stream has ended (programmatic dependent launch).
+
+They wait for that end (griddepcontrol.wait) before they read anything, and what they read then may be what the
+predecessor wrote: tensors, scales, zero-points, offsets.  A load that says its memory is constant while the kernel runs
+(__ldg, ld.global.nc, a __restrict__ pointer) may be moved above the wait by the compiler or served from a path that is
+not coherent, so no such load may stand in these kernels or in the functions they use.  Whether a given compiler moves
+one cannot be seen from results, so the CPU test reads the sources; the GPU tests chain calls in which every kind of
+input is written by the call before."""
+import os
+import re
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "onednn_b200", "csrc")
+NON_COHERENT = re.compile(r"__ldg|\.global\.nc|__restrict__|__ldcs|__ldlu")
+
+
+def _source(name):
+    text = open(os.path.join(CSRC, name)).read()
+    text = re.sub(r"/\*.*?\*/", "", text, flags=re.S)
+    text = re.sub(r"//[^\n]*", "", text)
+    return re.sub(r"__launch_bounds__\((?:[^()]|\([^()]*\))*\)", "", text)
+
+
+def _functions(text):
+    """{name: body} of every function of a source (the definitions' braces matched), overloads joined."""
+    out = {}
+    for m in re.finditer(r"(\w+)\s*\((?:[^;{}()]|\([^;{}()]*\))*\)\s*(?:const\s*)?\{", text):
+        at, depth = m.end(), 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        if m.group(1) not in ("if", "for", "while", "switch"):
+            out[m.group(1)] = out.get(m.group(1), "") + text[m.end():at]
+    return out
+
+
+def _reachable(file):
+    """{kernel: text} of the dependent kernels of a file: their bodies and those of every function reached from them."""
+    names, todo = set(), [file]
+    while todo:
+        f = todo.pop()
+        if f in names or not os.path.exists(os.path.join(CSRC, f)):
+            continue
+        names.add(f)
+        todo += re.findall(r'#include "([^"]+)"', open(os.path.join(CSRC, f)).read())
+    functions = {}
+    for f in names:
+        for n, b in _functions(_source(f)).items():
+            functions[n] = functions.get(n, "") + b
+    kernels = {n: b for n, b in _functions(_source(file)).items()
+               if n.endswith("_kernel") and "grid_dependency_wait()" in b}
+    out = {}
+    for k in kernels:
+        seen, queue = {k}, [k]
+        while queue:
+            for n in set(re.findall(r"\b(\w+)\s*(?:<[^<>;]*>)?\s*\(", functions[queue.pop()])):
+                if n in functions and n not in seen:
+                    seen.add(n)
+                    queue.append(n)
+        out[k] = "".join(functions[n] for n in seen)
+    return out
+
+
+@pytest.mark.parametrize("file", ["reorder.cu"])
+def test_dependent_kernels_read_with_coherent_loads(file):
+    kernels = _reachable(file)
+    assert kernels, "no kernel with a wait in " + file
+    for name, text in kernels.items():
+        assert not NON_COHERENT.findall(text), "%s: %s" % (name, sorted(set(NON_COHERENT.findall(text))))
+
+
+class _Device:
+    """Device buffers (torch tensors) behind memory objects of this library, and a stream of its own for the calls."""
+
+    def __init__(self, eng):
+        import torch
+        self.torch, self.eng, self.keep = torch, eng, []
+
+    def put(self, a):
+        t = self.torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1).copy()).to("cuda:0")
+        self.keep.append(t)
+        return t
+
+    def empty(self, nbytes):
+        t = self.torch.zeros(nbytes, dtype=self.torch.uint8, device="cuda:0")
+        self.keep.append(t)
+        return t
+
+    def mem(self, dims, dt, t):
+        from onednn_b200 import api
+        return api.memory(api.memory.desc(dims, dt, api.tag.a if len(dims) == 1 else api.tag.ab), self.eng, t.data_ptr())
+
+
+def _in_a_row(dev, strm, calls, outputs, repeats=8):
+    """Runs the calls one at a time, then all of them without a wait between, the outputs cleared each time: same bits."""
+    dev.torch.cuda.synchronize()
+    for prim, args in calls:
+        prim.execute(strm, args)
+        strm.wait()
+    want = [t.cpu().numpy().copy() for t in outputs]
+    for _ in range(repeats):
+        for t in outputs:
+            t.zero_()
+        dev.torch.cuda.synchronize()
+        for prim, args in calls:
+            prim.execute(strm, args)
+        strm.wait()
+        for t, w in zip(outputs, want):
+            assert np.array_equal(t.cpu().numpy(), w)
+    return want
+
+
+def _reorder(eng, dims, src_dt, dst_dt, **scales):
+    from onednn_b200 import api, workloads as W
+    attr = api.primitive_attr()
+    for arg, mask in scales.items():
+        attr.set_scales(api.ARG_DST if arg == "dst" else api.ARG_SRC, mask, (), W.F32)
+    md = lambda dt: api.memory.desc(dims, dt, api.tag.ab)
+    return api.reorder(api.reorder.primitive_desc(eng, md(src_dt), eng, md(dst_dt), attr))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(8, 128), (512, 1024), (300, 4100)])
+def test_reorders_of_a_matrix_and_scales_that_the_calls_before_wrote(gpu, shape):
+    """bf16 -> f32 matrix, f32 scales brought over from another place, then the quantization of the one by the others, to s8
+    and, from the 16-bit matrix that a third call wrote, to u8: each call's inputs are the outputs of those before."""
+    from onednn_b200 import api, workloads as W
+    eng, strm = gpu
+    M, N = shape
+    r = np.random.Generator(np.random.PCG64(31))
+    d = _Device(eng)
+    x16 = W.f32_to_bf16(r.standard_normal((M, N), dtype=np.float32))
+    src, sc0 = d.put(x16), d.put(r.uniform(0.01, 0.05, (1, N)).astype(np.float32))
+    x32, h16, sc, q8, qu = d.empty(4 * M * N), d.empty(2 * M * N), d.empty(4 * N), d.empty(M * N), d.empty(M * N)
+    quant = api.ARG_ATTR_SCALES | api.ARG_DST
+    calls = [
+        (_reorder(eng, (M, N), W.BF16, W.F32), {api.ARG_FROM: d.mem((M, N), W.BF16, src), api.ARG_TO: d.mem((M, N), W.F32, x32)}),
+        (_reorder(eng, (1, N), W.F32, W.F32), {api.ARG_FROM: d.mem((1, N), W.F32, sc0), api.ARG_TO: d.mem((1, N), W.F32, sc)}),
+        (_reorder(eng, (M, N), W.F32, W.S8, dst=2), {api.ARG_FROM: d.mem((M, N), W.F32, x32), api.ARG_TO: d.mem((M, N), W.S8, q8),
+                                                     quant: d.mem((1, N), W.F32, sc)}),
+        (_reorder(eng, (M, N), W.F32, W.F16), {api.ARG_FROM: d.mem((M, N), W.F32, x32), api.ARG_TO: d.mem((M, N), W.F16, h16)}),
+        (_reorder(eng, (M, N), W.F16, W.U8, dst=2), {api.ARG_FROM: d.mem((M, N), W.F16, h16), api.ARG_TO: d.mem((M, N), W.U8, qu),
+                                                     quant: d.mem((1, N), W.F32, sc)}),
+    ]
+    want = _in_a_row(d, strm, calls, [x32, sc, q8, h16, qu])
+    x = W.bf16_to_f32(x16)
+    scale = sc0.cpu().numpy().view(np.float32)
+    assert np.array_equal(want[2].view(np.int8).reshape(M, N), np.clip(np.rint(x / scale), -128, 127).astype(np.int8))
+    assert np.array_equal(want[4].reshape(M, N), np.clip(np.rint(x.astype(np.float16).astype(np.float32) / scale), 0, 255).astype(np.uint8))
