@@ -156,9 +156,9 @@ __device__ __forceinline__ void epilogue_rows(const MatmulArgs &a, const TcParam
     }
     if (t.row_scale) {
         if (FULL && a.src_scale.dt == DT_F32) {
-            const float *ss = (const float *)a.src_scale.ptr + m0;
+            const float *ss = (const float *)a.src_scale.ptr + m0; // (not __ldg: the call before may have written them)
 #pragma unroll
-            for (int j = 0; j < R; ++j) d[j] = __fmul_rn(d[j], __ldg(ss + j));
+            for (int j = 0; j < R; ++j) d[j] = __fmul_rn(d[j], ss[j]);
         } else {
 #pragma unroll
             for (int j = 0; j < R; ++j)

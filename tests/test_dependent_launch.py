@@ -64,7 +64,7 @@ def _reachable(file):
     return out
 
 
-@pytest.mark.parametrize("file", ["reorder.cu"])
+@pytest.mark.parametrize("file", ["reorder.cu", "gemm_split.cuh", "gemm_tc.cuh"])
 def test_dependent_kernels_read_with_coherent_loads(file):
     kernels = _reachable(file)
     assert kernels, "no kernel with a wait in " + file
@@ -150,3 +150,49 @@ def test_reorders_of_a_matrix_and_scales_that_the_calls_before_wrote(gpu, shape)
     scale = sc0.cpu().numpy().view(np.float32)
     assert np.array_equal(want[2].view(np.int8).reshape(M, N), np.clip(np.rint(x / scale), -128, 127).astype(np.int8))
     assert np.array_equal(want[4].reshape(M, N), np.clip(np.rint(x.astype(np.float16).astype(np.float32) / scale), 0, 255).astype(np.uint8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(33, 256, 512), (40, 512, 1024), (1900, 256, 1536)])
+def test_int8_layer_after_the_calls_that_quantize_its_src_and_write_its_parameters(gpu, shape):
+    """The src, its per-row scales, the weight scales and the residual of an int8 matmul with a post-op chain are each the
+    output of a call right before it (reorders), and its result is the input of a reorder: the split and the persistent
+    kernel, rows that fill the pieces of eight and rows that do not."""
+    from onednn_b200 import api, workloads as W
+    eng, strm = gpu
+    M, K, N = shape
+    r = np.random.Generator(np.random.PCG64(32))
+    d = _Device(eng)
+    f32 = lambda lo, hi, dims: r.uniform(lo, hi, dims).astype(np.float32)
+    x, xs = f32(-1, 1, (M, K)), f32(0.01, 0.02, (1, K))
+    given = [(x, (M, K)), (f32(0.001, 0.01, (M, 1)), (M, 1)), (f32(0.001, 0.01, (1, N)), (1, N)), (f32(-3, 3, (M, N)), (M, N))]
+    src8, row_scale, col_scale, resid = d.empty(M * K), d.empty(4 * M), d.empty(4 * N), d.empty(4 * M * N)
+    dst8, back = d.empty(M * N), d.empty(4 * M * N)
+    one = d.put(np.full(1, 0.06, np.float32))
+    wei = d.put(r.integers(-127, 128, (K, N), dtype=np.int8))
+    quant = api.ARG_ATTR_SCALES
+    calls = [(_reorder(eng, (M, K), W.F32, W.S8, dst=2), {api.ARG_FROM: d.mem((M, K), W.F32, d.put(x)), api.ARG_TO: d.mem((M, K), W.S8, src8),
+                                                          quant | api.ARG_DST: d.mem((1, K), W.F32, d.put(xs))})]
+    for (a, dims), t in zip(given[1:], (row_scale, col_scale, resid)):
+        calls.append((_reorder(eng, dims, W.F32, W.F32), {api.ARG_FROM: d.mem(dims, W.F32, d.put(a)), api.ARG_TO: d.mem(dims, W.F32, t)}))
+    attr = api.primitive_attr()
+    attr.set_scales(api.ARG_SRC, 1, (), W.F32)
+    attr.set_scales(api.ARG_WEIGHTS, 2, (), W.F32)
+    attr.set_scales(api.ARG_DST, 0, (), W.F32)
+    md = lambda dims, dt: api.memory.desc(dims, dt, api.tag.ab)
+    po = api.post_ops()
+    po.append_eltwise(W.ELTWISE["relu"], 0.0, 0.0)
+    po.append_binary(W.BINARY["add"], md((M, N), W.F32))
+    attr.set_post_ops(po)
+    pd = api.matmul.primitive_desc(eng, md((M, K), W.S8), md((K, N), W.S8), md((M, N), W.S8), None, attr)
+    assert pd.impl_info_str() == "cuda:tcgen05:int8"
+    calls.append((api.matmul(pd), {
+        api.ARG_SRC: d.mem((M, K), W.S8, src8), api.ARG_WEIGHTS: d.mem((K, N), W.S8, wei), api.ARG_DST: d.mem((M, N), W.S8, dst8),
+        quant | api.ARG_SRC: d.mem((M, 1), W.F32, row_scale), quant | api.ARG_WEIGHTS: d.mem((1, N), W.F32, col_scale),
+        quant | api.ARG_DST: d.mem((1,), W.F32, one),
+        api.ARG_ATTR_MULTIPLE_POST_OP(1) | api.ARG_SRC_1: d.mem((M, N), W.F32, resid)}))
+    calls.append((_reorder(eng, (M, N), W.S8, W.F32), {api.ARG_FROM: d.mem((M, N), W.S8, dst8), api.ARG_TO: d.mem((M, N), W.F32, back)}))
+    want = _in_a_row(d, strm, calls, [src8, row_scale, col_scale, resid, dst8, back])
+    s8 = np.clip(np.rint(x / xs), -128, 127).astype(np.int8)
+    assert np.array_equal(want[0].view(np.int8).reshape(M, K), s8)
+    assert np.unique(want[4]).size > 20  # (not a constant result)
