@@ -156,15 +156,15 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
 }
 
 // Loads that must be issued where they stand, well before their use: the compiler is free to move an
-// ordinary one down to it.
+// ordinary one down to it.  Coherent: the call before may have written the parameters.
 __device__ __forceinline__ uint32_t ld_early_u32(const uint32_t *p) {
     uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint32_t ld_early_u16(const unsigned short *p) {
     unsigned short v;
-    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
 // The zero-points of a lane's four columns (n .. n + 3) in group g, as loaded: four nibbles or four bytes

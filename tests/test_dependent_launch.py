@@ -64,7 +64,7 @@ def _reachable(file):
     return out
 
 
-@pytest.mark.parametrize("file", ["reorder.cu", "gemm_split.cuh", "gemm_tc.cuh"])
+@pytest.mark.parametrize("file", ["reorder.cu", "gemm_split.cuh", "gemm_tc.cuh", "grouped_tc.cu", "woq_decode.cu", "woq8_decode.cu", "woq_rows.cu"])
 def test_dependent_kernels_read_with_coherent_loads(file):
     kernels = _reachable(file)
     assert kernels, "no kernel with a wait in " + file
@@ -196,3 +196,99 @@ def test_int8_layer_after_the_calls_that_quantize_its_src_and_write_its_paramete
     s8 = np.clip(np.rint(x / xs), -128, 127).astype(np.int8)
     assert np.array_equal(want[0].view(np.int8).reshape(M, K), s8)
     assert np.unique(want[4]).size > 20  # (not a constant result)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [5, 40, 2000])
+def test_int4_layer_after_the_calls_that_write_its_src_and_parameters(gpu, M):
+    """The src, the group scales and the group zero-points of an int4 matmul are each the output of a call right before it
+    (4-bit zero-points, which no reorder copies, as eight 8-bit halves): the decode kernel, the same in blocks of rows, and
+    the kernel for many rows."""
+    from onednn_b200 import api, workloads as W
+    eng, strm = gpu
+    K, N, G = 512, 1056, 64
+    r = np.random.Generator(np.random.PCG64(33))
+    d = _Device(eng)
+    f32 = lambda lo, hi, dims: r.uniform(lo, hi, dims).astype(np.float32)
+    zp_bytes = r.integers(0, 256, (K // G, N // 2), dtype=np.uint8)
+    wei = d.put(r.integers(0, 256, (K, N // 2), dtype=np.uint8))
+    src, scale, zp, dst, back = d.empty(2 * M * K), d.empty(2 * (K // G) * N), d.empty(zp_bytes.size), d.empty(4 * M * N), d.empty(2 * M * N)
+    copy = lambda dims, sdt, ddt, a, t: (_reorder(eng, dims, sdt, ddt), {api.ARG_FROM: d.mem(dims, sdt, a), api.ARG_TO: d.mem(dims, ddt, t)})
+    calls = [copy((M, K), W.F32, W.BF16, d.put(f32(-1, 1, (M, K))), src),
+             copy((K // G, N), W.F32, W.BF16, d.put(f32(0.005, 0.02, (K // G, N))), scale),
+             copy(zp_bytes.shape, W.U8, W.U8, d.put(zp_bytes), zp)]
+    attr = api.primitive_attr()
+    attr.set_fpmath_mode(api.fpmath_mode.bf16, True)
+    attr.set_scales(api.ARG_WEIGHTS, 3, (G, 1), W.BF16)
+    attr.set_zero_points(api.ARG_WEIGHTS, 3, (G, 1), W.U4)
+    md = lambda dims, dt: api.memory.desc(dims, dt, api.tag.ab)
+    pd = api.matmul.primitive_desc(eng, md((M, K), W.BF16), md((K, N), W.U4), md((M, N), W.F32), None, attr)
+    assert pd.impl_info_str() == ("cuda:tcgen05:woq4" if M <= 32 else "cuda:tcgen05:woq4_rows")
+    calls.append((api.matmul(pd), {
+        api.ARG_SRC: d.mem((M, K), W.BF16, src), api.ARG_WEIGHTS: d.mem((K, N), W.U4, wei), api.ARG_DST: d.mem((M, N), W.F32, dst),
+        api.ARG_ATTR_SCALES | api.ARG_WEIGHTS: d.mem((K // G, N), W.BF16, scale),
+        api.ARG_ATTR_ZERO_POINTS | api.ARG_WEIGHTS: d.mem((K // G, N), W.U4, zp)}))
+    calls.append(copy((M, N), W.F32, W.BF16, dst, back))
+    want = _in_a_row(d, strm, calls, [src, scale, zp, dst, back])
+    # against f64
+    nib = lambda b: np.stack([b & 15, b >> 4], -1).reshape(b.shape[0], -1).astype(np.float64)
+    w = nib(wei.cpu().numpy().reshape(K, N // 2)) - np.repeat(nib(zp_bytes), G, 0)
+    w *= np.repeat(W.bf16_to_f32(want[1].view(np.uint16)).reshape(K // G, N), G, 0)
+    x = W.bf16_to_f32(want[0].view(np.uint16)).reshape(M, K).astype(np.float64)
+    got = want[3].view(np.float32).reshape(M, N)
+    assert np.all(np.abs(got - x @ w) <= K * 2.0 ** -24 * (np.abs(x) @ np.abs(w)))  # f32 sums of K exact products, any order
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,experts", [(24, 8), (50, 200), (700, 8)])
+def test_grouped_and_dense_s8_layers_after_the_calls_that_write_their_inputs(gpu, M, experts):
+    """Weight scales, src and the row offsets of a grouped s8-weight matmul are each the output of a call right before it,
+    and its result is the src of a dense s8-weight matmul: few rows and many."""
+    from onednn_b200 import api, workloads as W
+    eng, strm = gpu
+    K, N = 256, 320
+    r = np.random.Generator(np.random.PCG64(34))
+    d = _Device(eng)
+    f32 = lambda lo, hi, dims: r.uniform(lo, hi, dims).astype(np.float32)
+    ends = np.cumsum(r.multinomial(M, np.full(experts, 1.0 / experts))).astype(np.int32)
+    wei = r.integers(-127, 128, (experts, K, N), dtype=np.int8)
+    wei2 = r.integers(-127, 128, (N, K), dtype=np.int8)
+    src, offs, scale, scale2 = d.empty(2 * M * K), d.empty(4 * experts), d.empty(4 * experts * N), d.empty(4 * K)
+    mid, out = d.empty(2 * M * N), d.empty(4 * M * K)
+    copy = lambda dims, sdt, ddt, a, t: (_reorder(eng, dims, sdt, ddt), {api.ARG_FROM: d.mem(dims, sdt, a), api.ARG_TO: d.mem(dims, ddt, t)})
+    calls = [copy((M, K), W.F32, W.BF16, d.put(f32(-1, 1, (M, K))), src),
+             copy((experts, N), W.F32, W.F32, d.put(f32(0.001, 0.01, (experts, N))), scale),
+             copy((1, K), W.F32, W.F32, d.put(f32(0.001, 0.01, (1, K))), scale2),
+             copy((1, experts), W.S32, W.S32, d.put(ends), offs)]
+    attr = api.primitive_attr()
+    attr.set_fpmath_mode(api.fpmath_mode.bf16, True)
+    attr.set_scales(api.ARG_WEIGHTS, 0b101, (), W.F32)
+    grouped = lambda dims: api.memory.desc.grouped(dims, W.BF16, 0, experts)
+    abc = lambda dims, dt: api.memory.desc(dims, dt, api.tag.abc)
+    put = lambda md, t: api.memory(md, eng, t.data_ptr())
+    pd = api.matmul.primitive_desc(eng, grouped((M, K)), abc((experts, K, N), W.S8), grouped((M, N)), None, attr)
+    assert pd.impl_info_str() == "cuda:tcgen05:grouped"
+    calls.append((api.matmul(pd), {
+        api.ARG_SRC: api.memory(grouped((M, K)), eng, handles=[src.data_ptr(), offs.data_ptr()]),
+        api.ARG_DST: api.memory(grouped((M, N)), eng, handles=[mid.data_ptr(), offs.data_ptr()]),
+        api.ARG_WEIGHTS: put(abc((experts, K, N), W.S8), d.put(wei)),
+        api.ARG_ATTR_SCALES | api.ARG_WEIGHTS: put(abc((experts, 1, N), W.F32), scale)}))
+    attr2 = api.primitive_attr()
+    attr2.set_fpmath_mode(api.fpmath_mode.bf16, True)
+    attr2.set_scales(api.ARG_WEIGHTS, 2, (), W.F32)
+    md = lambda dims, dt: api.memory.desc(dims, dt, api.tag.ab)
+    pd2 = api.matmul.primitive_desc(eng, md((M, N), W.BF16), md((N, K), W.S8), md((M, K), W.F32), None, attr2)
+    assert pd2.impl_info_str() == "cuda:tcgen05:woq8"
+    calls.append((api.matmul(pd2), {
+        api.ARG_SRC: d.mem((M, N), W.BF16, mid), api.ARG_WEIGHTS: d.mem((N, K), W.S8, d.put(wei2)), api.ARG_DST: d.mem((M, K), W.F32, out),
+        api.ARG_ATTR_SCALES | api.ARG_WEIGHTS: d.mem((1, K), W.F32, scale2)}))
+    # (the offsets are cleared by hand to zeros between the runs: no rows, a valid call)
+    want = _in_a_row(d, strm, calls, [src, scale, scale2, offs, mid, out])
+    assert np.array_equal(want[3].view(np.int32), ends)
+    x = W.bf16_to_f32(want[0].view(np.uint16)).reshape(M, K).astype(np.float64)
+    sc = want[1].view(np.float32).reshape(experts, N)
+    got = W.bf16_to_f32(want[4].view(np.uint16)).reshape(M, N)
+    for e, (b, t) in enumerate(zip(np.concatenate([[0], ends[:-1]]), ends)):
+        exact = x[b:t] @ wei[e].astype(np.float64) * sc[e]
+        terms = np.abs(x[b:t]) @ np.abs(wei[e].astype(np.float64)) * sc[e]
+        assert np.all(np.abs(got[b:t] - exact) <= 2.0 ** -8 * np.abs(exact) + K * 2.0 ** -24 * terms)  # bf16 rounding, f32 sums
