@@ -92,6 +92,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); // recv_bar is ready
     // a programmatic dependent of whatever precedes it on the stream: what is above runs under the predecessor's end
     ptx::grid_dependency_wait();
+    bool late = false; // the wait for the other CTAs' sums ran out
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
@@ -176,7 +177,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             ptx::tmem_ld_wait();
             for (int q = 0; q < splits; ++q) send_b32(map_to_rank(colsum_at + (rank * BT_N + col) * 4, q), r[0], map_to_rank(bar, q));
         }
-        if (!ptx::mbar_wait(recv_bar, 0)) atomicExch(a.status, 5);
+        late = !ptx::mbar_wait(recv_bar, 0);
+        if (late) atomicExch(a.status, 5);
         if (INT && sp.ones && n < a.N) {
             int sum = 0;
             for (int q = 0; q < splits; ++q) sum += ((const int *)(smem + sp.off_colsum))[q * BT_N + col];
@@ -206,12 +208,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 
     // ---------------------------------------------------- teardown
     ptx::tc_fence_before_sync();
-    __syncthreads();
+    const bool some_late = __syncthreads_or(late);
     if (warp == 1) {
         __syncwarp();
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem_base, sp.tmem_cols);
+        __syncwarp();
     }
+    if (some_late && splits > 1) ptx::outlast_cluster(recv_bar);
 }
 
 template <int KIND, bool CHAIN, int DSTT = -1>

@@ -126,6 +126,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
         if (globaltimer() - t0 > limit_ns) return false;
     }
 }
+// For the CTAs of a cluster that send each other sums with st.async: called by every thread of a CTA in which a wait for
+// them (`bar`, its first phase) ran out, before the CTA ends.  Its shared memory has to stay while a slower CTA may still
+// send there: until every CTA of the cluster has come here or ended - all their waits are bounded, and they send whatever
+// happened to them - and what is then on its way has arrived.  A CTA that has received everything ends at once.
+__device__ __forceinline__ void outlast_cluster(uint64_t *bar) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    (void)mbar_wait(bar, 0);
+}
 // mbar_wait for a whole warp that may wait long: between polls the warp sleeps a few dozen
 // nanoseconds, so that a dozen waiting warps do not fill the SM's shared-memory instruction queue
 // with polls that the working warps' loads, arrives and tensor-memory stores then queue behind.

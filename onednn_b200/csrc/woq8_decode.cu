@@ -208,7 +208,8 @@ woq8_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
     // ---------------------------------------------------- this CTA's slice: the sum over the ranks, in order -> dst
     const int slice_log = NB_LOG - split_log, slice = 1 << slice_log;
-    if (!ptx::mbar_wait(sums_bar, 0)) atomicExch(a.status, 5);
+    const bool late = !ptx::mbar_wait(sums_bar, 0);
+    if (late) atomicExch(a.status, 5);
     const int nvec = rows << (slice_log - 2);
     for (int i = threadIdx.x; i < nvec; i += THREADS) {
         const int m = i >> (slice_log - 2), c = (i << 2) & (slice - 1);
@@ -244,6 +245,7 @@ woq8_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 if (n + e < a.N) finish_store_w8(a, d[e], mg, n + e, g);
         }
     }
+    if (__syncthreads_or(late) && splits > 1) ptx::outlast_cluster(sums_bar);
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,

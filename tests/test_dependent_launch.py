@@ -72,6 +72,22 @@ def test_dependent_kernels_read_with_coherent_loads(file):
         assert not NON_COHERENT.findall(text), "%s: %s" % (name, sorted(set(NON_COHERENT.findall(text))))
 
 
+@pytest.mark.parametrize("file", ["gemm_split.cuh", "woq_decode.cu", "woq8_decode.cu"])
+def test_a_cta_whose_peers_are_late_outlasts_them(file):
+    """The CTAs of a cluster send their sums into each other's shared memory.  One whose bounded wait for them ran out may
+    not end while a slower one can still send there: that store would go to memory that is gone.  A wait that runs out
+    cannot be staged on a GPU without breaking the kernel, so the test reads the sources: the wait's result is kept, the
+    kernel's last statement holds the whole CTA on it, and nothing returns between the two."""
+    (name, body), = [(n, b) for n, b in _functions(_source(file)).items() if n.endswith("_kernel")]
+    assert re.search(r"st_async_v4\(|send_v4\(", body)
+    wait = re.search(r"\blate = !ptx::mbar_wait\((\w+), 0\);", body)
+    assert wait, name + " drops the result of its wait for the other CTAs' sums"
+    tail = body[wait.end():]
+    assert re.search(r"(?:__syncthreads_or\(late\)|\bsome_late) && splits > 1\) ptx::outlast_cluster\(%s\);\s*\}\s*$" % wait.group(1), tail)
+    assert "some_late" not in tail or "some_late = __syncthreads_or(late);" in tail
+    assert "return" not in re.sub(r"\[[^\]]*\]\s*\([^()]*\)\s*\{[^{}]*\}", "", tail)  # (lambdas aside)
+
+
 class _Device:
     """Device buffers (torch tensors) behind memory objects of this library, and a stream of its own for the calls."""
 
