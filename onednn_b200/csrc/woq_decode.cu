@@ -405,6 +405,10 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     else if (a.src_scale.on_host) ssc = a.src_scale.host_value;
     const bool late = !ptx::mbar_wait(sums_bar, 0);
     if (late) atomicExch(a.status, 5);
+    if (__syncthreads_or(late)) {
+        if (splits > 1) ptx::outlast_cluster(sums_bar);
+        return;
+    }
     const int nvec = M << (slice_log - 2);
     for (int i = threadIdx.x; i < nvec; i += THREADS) {
         const int m = i >> (slice_log - 2), c = (i << 2) & (slice - 1);
@@ -442,7 +446,6 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             for (int e = 0; e < 4; ++e) finish_store_cold(a, d[e], m0 + m, n + e);
         }
     }
-    if (__syncthreads_or(late) && splits > 1) ptx::outlast_cluster(sums_bar);
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,

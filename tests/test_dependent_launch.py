@@ -76,16 +76,20 @@ def test_dependent_kernels_read_with_coherent_loads(file):
 def test_a_cta_whose_peers_are_late_outlasts_them(file):
     """The CTAs of a cluster send their sums into each other's shared memory.  One whose bounded wait for them ran out may
     not end while a slower one can still send there: that store would go to memory that is gone.  A wait that runs out
-    cannot be staged on a GPU without breaking the kernel, so the test reads the sources: the wait's result is kept, the
-    kernel's last statement holds the whole CTA on it, and nothing returns between the two."""
+    cannot be staged on a GPU without breaking the kernel, so the test reads the sources: the wait's result is kept, and
+    the whole CTA is held on it."""
     (name, body), = [(n, b) for n, b in _functions(_source(file)).items() if n.endswith("_kernel")]
     assert re.search(r"st_async_v4\(|send_v4\(", body)
     wait = re.search(r"\blate = !ptx::mbar_wait\((\w+), 0\);", body)
     assert wait, name + " drops the result of its wait for the other CTAs' sums"
     tail = body[wait.end():]
-    assert re.search(r"(?:__syncthreads_or\(late\)|\bsome_late) && splits > 1\) ptx::outlast_cluster\(%s\);\s*\}\s*$" % wait.group(1), tail)
-    assert "some_late" not in tail or "some_late = __syncthreads_or(late);" in tail
-    assert "return" not in re.sub(r"\[[^\]]*\]\s*\([^()]*\)\s*\{[^{}]*\}", "", tail)  # (lambdas aside)
+    if "some_late" in tail:  # at the kernel's end, where a barrier of the CTA stands anyway; nothing returns before it
+        assert "some_late = __syncthreads_or(late);" in tail
+        assert re.search(r"if \(some_late && splits > 1\) ptx::outlast_cluster\(%s\);\s*\}\s*$" % wait.group(1), tail)
+        assert "return" not in re.sub(r"\[[^\]]*\]\s*\([^()]*\)\s*\{[^{}]*\}", "", tail)  # (lambdas aside)
+    else:  # right behind the wait, before anything is stored
+        assert re.match(r"\s*if \(late\) atomicExch\(a\.status, 5\);\s*if \(__syncthreads_or\(late(?: \|\| some_wrong)?\)\) \{"
+                        r"\s*if \(splits > 1\) ptx::outlast_cluster\(%s\);\s*return;" % wait.group(1), tail)
 
 
 class _Device:

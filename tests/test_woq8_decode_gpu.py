@@ -59,3 +59,38 @@ def test_grouped_matches_oracle(gpu, name):
     got, impl = run_problem(p, eng, strm)
     assert impl == "cuda:tcgen05:grouped"
     assert_parity(got, O.run_port(p), p.dst_dt, name, summation_slack_grouped(p))
+
+
+BAD_OFFSETS = {
+    # (src ends, dst ends or None for the same): a step back, an end beyond the rows, fewer dst rows than src rows, a negative end
+    "step_back": (lambda M: [10, 5, M - 3, M], None),
+    "beyond_the_rows": (lambda M: [2, 7, M - 1, M + 1], None),
+    "last_of_many": (lambda M: list(range(1, 21)) + [M] * 178 + [M - 1], None),
+    "dst_rows_differ": (lambda M: [4, 9, 20, M], lambda M: [4, 10, 20, M]),
+    "negative": (lambda M: [-1, 3, 8, M], None),
+}
+
+
+@pytest.mark.parametrize("M", [40, 64, 65, 300])
+@pytest.mark.parametrize("name", sorted(BAD_OFFSETS))
+def test_grouped_bad_offsets_write_nothing(gpu, name, M):
+    """One wrong offset: the call reports invalid_arguments and dst stays as it was, for few rows (whose kernel reads the
+    offsets itself) as for many (which have a planning kernel)."""
+    from onednn_b200 import api
+    from onednn_b200.runner import Prepared
+    eng, strm = gpu
+    ends, dst_ends = (f(M) if f else None for f in BAD_OFFSETS[name])
+    n = len(ends)
+    p = W.moe_grouped(M, 128, 160, n, sizes=[M] + [0] * (n - 1))
+    p.offsets = np.array(ends, np.int32)
+    p.dst_init = np.full((M, p.N), 0x4242, np.uint16)
+    r = Prepared(p, eng).upload()
+    if dst_ends:
+        r.args[api.ARG_DST].write(np.array(dst_ends, np.int32), 1)
+    for _ in range(2):
+        r.execute(strm)
+        with pytest.raises(api.error) as ei:
+            strm.wait()
+        assert ei.value.status == api.invalid_arguments
+        assert np.array_equal(r.download(), p.dst_init)
+    strm.wait()  # the status word is cleared: the stream stays usable
