@@ -59,8 +59,8 @@ def test_cuda_reorder_matches_oracle(gpu, name):
 @pytest.mark.parametrize("dst_dt", [W.S8, W.U8])
 @pytest.mark.parametrize("tiles", [(1, 1), (2, 224)], ids=["few_rows_a_thread", "many_rows_a_thread"])
 def test_cuda_reorder_rounds_quotients_like_the_division(gpu, dst_dt, tiles):
-    """Small matrices divide, large ones (16 rows a thread or more) multiply with reciprocals where that is safe.
-    Columns whose scaled values lie on half integers and one unit beside them, saturate, or have a scale whose
+    """Few rows a thread and many (the quotient is the same code: reciprocal, remainder, correction; it divides where the
+    scale lies outside the range for which that is exact).  Columns whose scaled values lie on half integers and one unit beside them, saturate, or have a scale whose
     reciprocal is not a normal number: the 8-bit results are those of the IEEE division (element-wise, no tolerance)."""
     from onednn_b200.runner import run_reorder
     eng, strm = gpu
@@ -75,6 +75,62 @@ def test_cuda_reorder_rounds_quotients_like_the_division(gpu, dst_dt, tiles):
     ro = W.Reorder("ties", W.QTensor(x, W.F32, x.shape), dst_dt, quant={"dst_scale": W.Quant(sc.reshape(1, -1), W.F32, 2)})
     got, _ = run_reorder(ro, eng, strm)
     assert np.array_equal(got, O.run_port_reorder(ro))
+
+
+QUANTIZE_SHAPES = {
+    # rows of threads narrower than a warp, with idle lanes and without; one CTA; several column blocks, a ragged one;
+    # fewer and more rows than are in flight per thread, and not a multiple of them; leading dims
+    "one_chunk": (2000, 4), "three_chunks": (700, 12), "ten_chunks": (333, 40), "sixteen_chunks": (1, 64), "a_warp": (9, 128),
+    "a_warp_and_one": (50, 132), "ragged_block": (37, 1028), "many_rows": (5003, 516), "wide": (3, 14336), "4d": (3, 5, 7, 96),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scales", ["per_column", "common", "with_src_scale"])
+@pytest.mark.parametrize("dst_dt", [W.S8, W.U8], ids=["s8", "u8"])
+@pytest.mark.parametrize("src_dt", [W.F32, W.BF16, W.F16], ids=["f32", "bf16", "f16"])
+def test_cuda_quantizing_reorder_in_every_form(gpu, src_dt, dst_dt, scales):
+    """Every source type, result type and kind of scales at the edges of its rows and columns: the bits of the oracle
+    (element-wise, no tolerance).  The values include halves, both infinities and what saturates."""
+    from onednn_b200.runner import run_reorder
+    eng, strm = gpu
+    r = np.random.Generator(np.random.PCG64(83))
+    for name, dims in QUANTIZE_SHAPES.items():
+        n, last = int(np.prod(dims)), dims[-1]
+        mask = 1 << (len(dims) - 1)
+        sc = r.uniform(0.02, 0.06, last).astype(np.float32)
+        sc[::5] = 0.03125  # exact quotients: halves are ties
+        x = (r.standard_normal(n) * 3.0).astype(np.float32)
+        x[::7] = (r.integers(-300, 300, x[::7].size) + 0.5) * np.float32(0.03125)
+        x[::101] = np.inf
+        x[50::101] = -np.inf
+        q = {"dst_scale": W.Quant(sc.reshape((1,) * (len(dims) - 1) + (last,)), W.F32, mask)} if scales != "common" else \
+            {"dst_scale": W.Quant(np.array([0.03125], np.float32), W.F32, 0)}
+        if scales == "with_src_scale":
+            q["src_scale"] = W.Quant(r.uniform(0.5, 2.0, sc.size).astype(np.float32).reshape((1,) * (len(dims) - 1) + (last,)), W.F32, mask)
+        ro = W.Reorder(name, W.QTensor(W.to_storage(x, src_dt).reshape(dims), src_dt, dims), dst_dt, quant=q)
+        got, _ = run_reorder(ro, eng, strm)
+        want = O.run_port_reorder(ro)
+        assert np.array_equal(got.view(np.uint8).reshape(-1), want.view(np.uint8).reshape(-1)), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dst_dt", [W.S8, W.U8], ids=["s8", "u8"])
+@pytest.mark.parametrize("src_dt", [W.F32, W.BF16, W.F16], ids=["f32", "bf16", "f16"])
+def test_cuda_quantizing_reorder_of_nan(gpu, src_dt, dst_dt):
+    """A NaN becomes the type's lowest value, under usual scales and under those that divide, as in the general kernel
+    (reached by a scale per row)."""
+    from onednn_b200.runner import run_reorder
+    eng, strm = gpu
+    x = np.linspace(-2.0, 2.0, 64 * 64, dtype=np.float32)
+    x[::3] = np.nan
+    sc = np.full((1, 64), 0.05, np.float32)
+    sc[0, ::4] = 1e-39
+    lowest = -128 if dst_dt == W.S8 else 0
+    for quant in (W.Quant(sc, W.F32, 2), W.Quant(sc.reshape(64, 1).copy(), W.F32, 1)):
+        ro = W.Reorder("nan", W.QTensor(W.to_storage(x, src_dt).reshape(64, 64), src_dt, (64, 64)), dst_dt, quant={"dst_scale": quant})
+        got, _ = run_reorder(ro, eng, strm)
+        assert np.all(got.view(np.int8 if dst_dt == W.S8 else np.uint8).reshape(-1)[::3] == lowest)
 
 
 @pytest.mark.gpu
