@@ -566,6 +566,11 @@ bool woq_decode_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_d
     return M <= 16 || rb * NB * (wd_bits(scale_dt) + (zp_dt < 0 ? 0 : wd_bits(zp_dt))) / 8 < W_BYTES;
 }
 
+// 16-bit scales, and no zero-points or 4-bit ones per group: w - zero_point exactly, and the kernel's quick forms
+bool woq_decode_common_form(const MatmulArgs &a) {
+    return wd_bits(a.wei_scale.dt) == 16 && (!a.wei_zp.ptr || (a.wei_zp.mask && wd_bits(a.wei_zp.dt) == 4));
+}
+
 // Microseconds that a problem takes here, for the choice between this kernel and the one whose operand lies in tensor
 // memory (woq_rows.cu) when there are more than 32 rows: a stage costs an SM 0.82 for blocks of 32 rows (0.65 for 24), more
 // with small groups (a fold of the sums at each end), and the launch about 4.
