@@ -22,12 +22,15 @@
 //     under a zero upper byte is u * 2^-133 where it stands low and u * 2^-129 where it
 //     stands high (the step from subnormal to normal numbers included); f16: u * 2^-24 and
 //     u * 2^-20.  One LOP3 and one packed FMA make (w - zero_point) / 64 (f16: / 512) of two
-//     nibbles, and the group's sum is multiplied by the 64.  Zero-points of other types than
-//     s4 / u4 may leave the exact range: the sums then run over w, and zero_point * sum(src)
-//     is taken off the group's sum, the sum of src from one more MMA against a matrix of ones.
+//     nibbles, and the group's sum is multiplied by the 64.  What of a wide zero-point is not
+//     exact is taken off the sums at the end.
 // us a call, before (operand in tensor memory, two launches) -> now: 8192 x 28672, groups of 128, bf16, M = 1 49.3 -> 35.1,
 // 8 57.9 -> 36.2, 16 73.8 -> 49.5, 32 83.9 -> 82.4; 4096 x 11008 f16, groups of 64, M = 13 41.1 -> 11.7; 4096 x 1024, groups of
 // 32, M = 32 39.4 -> 14.6; 4096 x 4096, groups of 32, M = 4 21.6 -> 10.7.
+// Other parameters, 8192 x 28672, groups of 128, bf16, that kernel / this one with scales and zero-points read one at a time and
+// the zero-points taken off the sums / now: f32 scales M = 1 47 / 76 / 35, 16 71 / 113 / 48, 32 76 / 253 / 78; f32 scales
+// and u4 zero-points in groups of 32, M = 1 90 / 204 / 57, 32 179 / 612 / 145; one s8 zero-point M = 1 47 / 74 / 35, 32 77 / 253 / 78;
+// u8 ones per group (the only form still behind at 32 rows) M = 1 49 / 90 / 43, 16 73 / 144 / 60, 32 80 / 290 / 87.
 // What bounds it: issue and the pipes behind it.  A stage is 64 LOP3, 32 PRMT, 64 packed FMAs, 16 MMAs and 20 shared-memory
 // reads of a warp, about 350 cycles of a scheduler in a loop of nothing else, where the packed instructions of the two
 // pipes get in each other's way (192 would be the busiest pipe alone); M = 32 is bound by mma.sync (8 cycles each).
@@ -77,19 +80,50 @@ struct WdParams {
     int zp_common; // one zero-point for the whole tensor
     int sc_bits, zp_bits; // of an element of the parameter rows; zp_bits 0: no rows
     int stages, stage_bytes, off_sc, off_zp; // ring
-    int off_bars;
+    int off_bars, off_held;
 };
+
+// Scales held as f32, 8 a lane, are kept in shared memory (a place of the lane's own) where the registers do not hold them.
+template <int MT, bool SC32>
+constexpr bool scales_held = SC32 && MT >= 3;
+constexpr int HELD_BYTES = 32 * WARPS * 32;
 
 __device__ __noinline__ void finish_store_cold(const MatmulArgs &a, float d, int64_t m, int64_t n) {
     if (a.bias) d = __fadd_rn(d, load_float(a.bias_dt, a.bias, m * a.bias_sm + n * a.bias_sn));
     finish_store(a, d, m, n, false);
 }
-__device__ __noinline__ float load_scale_cold(int dt, const void *p, int i) { return load_float(dt, p, i); }
-__device__ __noinline__ float load_zp_cold(int dt, const void *p, int i) { return (float)load_int(dt, p, i); }
 
-// ZPM: 0 no zero-points, 1 s4 / u4 per (group, column), 2 any other, and scales of other types than bf16 / f16.  STEPS: k16 steps that surely belong to one
-// group (4: groups are multiples of 64 k, 2: of 32, 1: of 16).
-template <int MT, bool F16, int ZPM, int STEPS>
+// The part of a zero-point for which w - zero_point is exact in the src's type.  That is all of it but for s32 ones beyond these
+// bounds and, with a bf16 src and s4 weights, u8 ones above 248.
+template <bool F16>
+__device__ __forceinline__ int exact_part(int z, int sgn4) {
+    return F16 ? min(max(z, -1024), 1024) : min(max(z, -128), sgn4 ? 248 : 255);
+}
+// What the rest of the zero-points takes off the sums of src row m over k0 .. k1 - 1, in the columns n .. n + 7
+template <bool F16>
+__device__ __noinline__ void rest_terms(const MatmulArgs &a, const WdParams &p, int64_t m, int64_t n, int k0, int k1, float (&term)[8]) {
+    for (int i = 0; i < 8; ++i) term[i] = 0.f;
+    const int group = p.group_steps * 16;
+    for (int k = k0; k < k1;) {
+        const int g = k / group, end = min((g + 1) * group, k1);
+        float sum = 0.f;
+        for (; k < end; ++k) sum += load_float(a.src_dt, a.src, m * a.src_sm + k);
+        for (int i = 0; i < 8 && n + i < a.N; ++i) {
+            const int z = load_int(a.wei_zp.dt, a.wei_zp.ptr, p.zp_common ? 0 : g * a.wei_zp.ld + n + i);
+            const float scale = load_float(a.wei_scale.dt, a.wei_scale.ptr, (p.sc_grouped ? g * a.wei_scale.ld : 0) + n + i);
+            term[i] = fmaf((float)(z - exact_part<F16>(z, p.sgn4)) * scale, sum, term[i]);
+        }
+    }
+}
+
+// ZPM, zero-points: 0 none; 1 s4 / u4 per (group, column); 2 8-bit ones per (group, column); 3 those, or s32 ones, whose type has
+// values that are not exact (see exact_part); 4 none, or one for the tensor.  What is exact of a zero-point goes into the
+// weights; a warp that met a rest takes it off its sums after the loop, slowly.  SC32: the group's scales are held as f32
+// (any type), else as 16-bit pairs.  STEPS: k16 steps that surely belong to one group (4: groups are multiples of 64 k, 2: of
+// 32, 1: of 16).
+// (0 is a form of its own, for 16-bit scales: the constant from a zero-point in it cost 1 to 10 %, 13 x 4096 x 11008 11.65 ->
+// 12.08 us, 100 x 4096 x 4096 in groups of 32 33.8 -> 37.3.)
+template <int MT, bool F16, int ZPM, bool SC32, int STEPS>
 __global__ void __launch_bounds__(THREADS, WdCfg<MT>::CTAS)
 woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
         const __grid_constant__ MatmulArgs a, const __grid_constant__ WdParams p) {
@@ -204,13 +238,18 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         const int zp_dt = in_reg(a.wei_zp.dt), sc_dt = in_reg(a.wei_scale.dt);
         const uint32_t zflip = zp_dt == DT_S4 ? 0x88888888u : 0u, zmul = mul_lo | 0x80008000u;
         const uint32_t zadd = pack_const(bias0 + (zp_dt == DT_S4 ? 8.f : 0.f));
-        uint32_t zc[ZPM == 1 ? 8 : 1]; // -(bias + zero_point) / UNIT of the lane's columns
-        if (ZPM != 1) zc[0] = pack_const(bias0);
+        constexpr bool PER_COLUMN = ZPM >= 1 && ZPM <= 3;
+        uint32_t zc[PER_COLUMN ? 8 : 1]; // -(bias + zero_point) / UNIT of the lane's columns
+        if (!PER_COLUMN) zc[0] = pack_const(bias0);
         ptx::grid_dependency_wait();
-        const float zcommon = (ZPM == 2 && p.zp_common) ? (float)load_int(zp_dt, a.wei_zp.ptr, 0) : 0.f;
-        float zf[ZPM == 2 ? 8 : 1];
+        bool rest = false; // a zero-point was not exact
+        if (ZPM == 4 && p.zp_common) {
+            const int z = load_int(zp_dt, a.wei_zp.ptr, 0), exact = exact_part<F16>(z, p.sgn4);
+            zc[0] = pack_const(bias0 - (float)exact);
+            rest = z != exact;
+        }
         uint64_t tot[4][MT][2]; // pairs of rows of the columns 2 j and 2 j + 1
-        float acc[4][MT][4], accs[ZPM == 2 ? MT : 1][4];
+        float acc[4][MT][4];
         auto clear = [&]() {
 #pragma unroll
             for (int t = 0; t < MT; ++t) {
@@ -218,7 +257,6 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                 for (int e = 0; e < 4; ++e) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) acc[j][t][e] = 0.f;
-                    if (ZPM == 2) accs[t][e] = 0.f;
                 }
             }
         };
@@ -228,18 +266,53 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 #pragma unroll
             for (int t = 0; t < MT; ++t) tot[j][t][0] = tot[j][t][1] = 0ull;
         const int sc_pitch = NB * p.sc_bits / 8, zp_pitch = NB * p.zp_bits / 8;
-        uint32_t scp[ZPM == 2 ? 8 : 4]; // scales of the open group: 16-bit pairs, or (general form) f32 bits
+        constexpr bool HELD = scales_held<MT, SC32>;
+        const uint32_t held = ptx::smem_u32(smem + p.off_held) + 8 * (32 * warp + lane);
+        uint32_t scales[SC32 ? 8 : 4]; // of the open group: f32 bits, or 16-bit pairs
         auto begin_group = [&](uint32_t so, int row) {
-            if constexpr (ZPM == 2) {
-                const uint8_t *sc = smem + so + off_sc + row * sc_pitch, *zp = smem + so + off_zp + row * zp_pitch;
+            uint32_t held_here[HELD ? 8 : 1];
+            uint32_t *const scp = HELD ? held_here : scales;
+            const uint32_t sc = ring + so + off_sc + row * sc_pitch;
+            if constexpr (!SC32) {
+                const uint4 v = lds128(sc + 2 * col);
+                scp[0] = v.x; scp[1] = v.y; scp[2] = v.z; scp[3] = v.w;
+            } else if (sc_dt == DT_F32) {
+                const uint4 v = lds128(sc + 4 * col), w = lds128(sc + 4 * col + 16);
+                scp[0] = v.x; scp[1] = v.y; scp[2] = v.z; scp[3] = v.w;
+                scp[SC32 ? 4 : 0] = w.x; scp[SC32 ? 5 : 0] = w.y; scp[SC32 ? 6 : 0] = w.z; scp[SC32 ? 7 : 0] = w.w;
+            } else if (sc_dt == DT_BF16 || sc_dt == DT_F16) {
+                const uint4 v = lds128(sc + 2 * col);
+                const uint32_t h[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    scp[i] = __float_as_uint(load_scale_cold(sc_dt, sc, col + i));
-                    zf[i] = p.zp_bits ? load_zp_cold(zp_dt, zp, col + i) : zcommon;
+                    const uint32_t b = i & 1 ? h[i / 2] >> 16 : h[i / 2] & 0xffffu;
+                    scp[SC32 ? i : 0] = sc_dt == DT_BF16 ? b << 16 : __float_as_uint(__half2float(__ushort_as_half((unsigned short)b)));
                 }
             } else {
-                const uint4 v = lds128(ring + so + off_sc + row * sc_pitch + 2 * col);
-                scp[0] = v.x; scp[1] = v.y; scp[2] = v.z; scp[3] = v.w;
+                const uint32_t b[2] = {lds32(sc + col), lds32(sc + col + 4)};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const unsigned char c = (unsigned char)(b[i / 4] >> (8 * (i & 3)));
+                    scp[SC32 ? i : 0] = __float_as_uint(sc_dt == DT_F8_E4M3 ? e4m3_to_f32(c) : e5m2_to_f32(c));
+                }
+            }
+            if constexpr (HELD) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sts64(held + j * (8 * 32 * WARPS), held_here[HELD ? 2 * j : 0], held_here[HELD ? 2 * j + 1 : 0]);
+            }
+            if constexpr (ZPM == 2 || ZPM == 3) {
+                const uint32_t zp = ring + so + off_zp + row * zp_pitch;
+                const bool wide = ZPM == 3 && zp_dt == DT_S32;
+                uint32_t b[2] = {0, 0};
+                if (!wide) { b[0] = lds32(zp + col); b[1] = lds32(zp + col + 4); }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int u = (int)(b[i / 4] >> (8 * (i & 3))) & 255;
+                    const int z = wide ? (int)lds32(zp + 4 * (col + i)) : zp_dt == DT_S8 ? (int)(signed char)u : u;
+                    const int exact = ZPM == 3 ? exact_part<F16>(z, p.sgn4) : z;
+                    zc[PER_COLUMN ? i : 0] = pack_const(bias0 - (float)exact);
+                    rest |= z != exact;
+                }
             }
             if constexpr (ZPM == 1) {
                 const uint32_t zx = lds32(ring + so + off_zp + row * zp_pitch + (col >> 1)) ^ zflip;
@@ -257,14 +330,18 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 float s0, s1; // columns col + 2 j and + 1
-                if (ZPM == 2) {
-                    s0 = __uint_as_float(scp[(ZPM == 2 ? 2 : 1) * j]);
-                    s1 = __uint_as_float(scp[ZPM == 2 ? 2 * j + 1 : 0]);
+                if (HELD) {
+                    const uint2 v = lds64(held + j * (8 * 32 * WARPS));
+                    s0 = __uint_as_float(v.x);
+                    s1 = __uint_as_float(v.y);
+                } else if (SC32) {
+                    s0 = __uint_as_float(scales[SC32 ? 2 * j : 0]);
+                    s1 = __uint_as_float(scales[SC32 ? 2 * j + 1 : 0]);
                 } else if (sc_dt == DT_BF16) {
-                    s0 = __uint_as_float(scp[j] << 16);
-                    s1 = __uint_as_float(scp[j] & 0xffff0000u);
+                    s0 = __uint_as_float(scales[j] << 16);
+                    s1 = __uint_as_float(scales[j] & 0xffff0000u);
                 } else {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&scp[j]));
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&scales[j]));
                     s0 = f.x;
                     s1 = f.y;
                 }
@@ -274,10 +351,6 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 #pragma unroll
                     for (int e = 0; e < 4; e += 2) {
                         uint64_t v = mul_f32x2(pack2(acc[j][t][e], acc[j][t][e + 1]), unit2);
-                        if (ZPM == 2) {
-                            const float nz = -zf[ZPM == 2 ? 2 * j + (e >> 1) : 0];
-                            v = fma_f32x2(pack2(nz, nz), pack2(accs[ZPM == 2 ? t : 0][e], accs[ZPM == 2 ? t : 0][e + 1]), v);
-                        }
                         tot[j][t][e / 2] = fma_f32x2(e < 2 ? s02 : s12, v, tot[j][t][e / 2]);
                     }
                 }
@@ -307,7 +380,7 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                 const uint32_t sel = ((4 + j) << 12) | ((4 + j) << 8) | (j << 4) | j;
                 // byte j of two k-rows, each in a 16-bit half: low nibble = column col + 2 j, high = + 1
                 const uint32_t x01 = perm(x.w[0], x.w[1], sel), x23 = perm(x.w[2], x.w[3], sel);
-                const uint32_t z0 = zc[ZPM == 1 ? 2 * j : 0], z1 = zc[ZPM == 1 ? 2 * j + 1 : 0];
+                const uint32_t z0 = zc[PER_COLUMN ? 2 * j : 0], z1 = zc[PER_COLUMN ? 2 * j + 1 : 0];
                 uint32_t w[4];
                 w[0] = fma2<F16>(and_xor(x01, 0x000F000Fu, magic_lo), mul_lo, z0);
                 w[1] = fma2<F16>(and_xor(x01, 0x00F000F0u, magic_hi), mul_hi, z1);
@@ -315,12 +388,6 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
                 w[3] = fma2<F16>(and_xor(x23, 0x00F000F0u, magic_hi), mul_hi, z1);
 #pragma unroll
                 for (int t = 0; t < MT; ++t) mma<F16>(acc[j][t], w, x.b[2 * t], x.b[2 * t + 1]);
-            }
-            if (ZPM == 2) {
-                const uint32_t one = F16 ? 0x3C003C00u : 0x3F803F80u;
-                const uint32_t ones[4] = {one, one, one, one};
-#pragma unroll
-                for (int t = 0; t < MT; ++t) mma<F16>(accs[ZPM == 2 ? t : 0], ones, x.b[2 * t], x.b[2 * t + 1]);
             }
         };
 
@@ -378,6 +445,18 @@ woq_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
         if (!ok) atomicExch(a.status, 5);
         else if (!fresh) end_group(); // the share ends inside a group
+        if (ZPM >= 3 && __any_sync(0xffffffffu, rest)) {
+#pragma unroll
+            for (int t = 0; t < MT; ++t) {
+                float t0[8], t1[8];
+                const int m = 8 * t + 2 * t4;
+                if (m >= M) continue;
+                rest_terms<F16>(a, p, m0 + m, (int64_t)tile * NB + col, st0 * KS, min(st1 * KS, (int)a.K), t0);
+                rest_terms<F16>(a, p, m0 + min(m + 1, M - 1), (int64_t)tile * NB + col, st0 * KS, min(st1 * KS, (int)a.K), t1);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) tot[i / 2][t][i & 1] = fma_f32x2(pack2(-1.f, -1.f), pack2(t0[i], t1[i]), tot[i / 2][t][i & 1]);
+            }
+        }
 
         // -------------------------------------------- the sums go to the cluster's CTAs, a slice of the columns to each
         // (asynchronous stores that count themselves at the receiver's barrier: no CTA waits for another to read)
@@ -496,10 +575,10 @@ int wd_split_log(int64_t ntiles, int kstages, int mt, int sm_count) {
     return best;
 }
 
-template <int MT, bool F16, int ZPM, int STEPS>
+template <int MT, bool F16, int ZPM, bool SC32, int STEPS>
 int wd_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a, WdParams p, int ntiles, cudaStream_t st) {
     using C = WdCfg<MT>;
-    auto kern = woq_decode_kernel<MT, F16, ZPM, STEPS>;
+    auto kern = woq_decode_kernel<MT, F16, ZPM, SC32, STEPS>;
     const int rb = wd_rows_per_stage(p.group_steps);
     auto up128 = [](int v) { return (v + 127) / 128 * 128; };
     p.off_sc = W_BYTES + C::S_BYTES;
@@ -507,10 +586,12 @@ int wd_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a,
     p.stage_bytes = (p.off_zp + up128(rb * NB * p.zp_bits / 8) + 1023) / 1024 * 1024;
     const int sums_bytes = p.rows * NB * 4;
     // as many stages as the CTA's share of the SM holds; four where wide parameter rows leave fewer (then fewer CTAs fit an SM)
-    p.stages = (C::SMEM - BAR_BYTES - sums_bytes) / p.stage_bytes;
+    constexpr int held_bytes = scales_held<MT, SC32> ? HELD_BYTES : 0;
+    p.stages = (C::SMEM - BAR_BYTES - sums_bytes - held_bytes) / p.stage_bytes;
     p.stages = p.stages > MAX_STAGES ? MAX_STAGES : p.stages < 4 ? 4 : p.stages;
     p.off_bars = p.stages * p.stage_bytes + sums_bytes;
-    const int smem_bytes = p.off_bars + BAR_BYTES;
+    p.off_held = p.off_bars + BAR_BYTES;
+    const int smem_bytes = p.off_held + held_bytes;
     if (smem_bytes > SMEM_PER_SM) return 3; // (not reached: woq_decode_fits)
     static std::atomic<unsigned long long> configured;
     if (!opt_in_dynamic_smem(kern, SMEM_PER_SM, configured)) return 5;
@@ -539,12 +620,17 @@ int wd_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a,
 
 template <int MT, bool F16>
 int wd_choose(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a, const WdParams &p, int zpm, int ntiles, cudaStream_t st) {
-    if (zpm == 2) return wd_launch<MT, F16, 2, 1>(tw, ts, a, p, ntiles, st);
-#define QMM_WD(Z) \
-    (p.group_steps % 4 == 0 ? wd_launch<MT, F16, Z, 4>(tw, ts, a, p, ntiles, st) \
-                    : p.group_steps % 2 == 0 ? wd_launch<MT, F16, Z, 2>(tw, ts, a, p, ntiles, st) \
-                                             : wd_launch<MT, F16, Z, 1>(tw, ts, a, p, ntiles, st))
-    return zpm == 1 ? QMM_WD(1) : QMM_WD(0);
+#define QMM_WD(Z, S) \
+    (p.group_steps % 4 == 0 ? wd_launch<MT, F16, Z, S, 4>(tw, ts, a, p, ntiles, st) \
+                    : p.group_steps % 2 == 0 ? wd_launch<MT, F16, Z, S, 2>(tw, ts, a, p, ntiles, st) \
+                                             : wd_launch<MT, F16, Z, S, 1>(tw, ts, a, p, ntiles, st))
+    switch (zpm) {
+        case 0: return QMM_WD(0, false);
+        case 1: return p.sc_bits == 16 ? QMM_WD(1, false) : QMM_WD(1, true);
+        case 2: return QMM_WD(2, true);
+        case 3: return QMM_WD(3, true);
+        default: return QMM_WD(4, true);
+    }
 #undef QMM_WD
 }
 
@@ -566,7 +652,7 @@ bool woq_decode_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_d
     return M <= 16 || rb * NB * (wd_bits(scale_dt) + (zp_dt < 0 ? 0 : wd_bits(zp_dt))) / 8 < W_BYTES;
 }
 
-// 16-bit scales, and no zero-points or 4-bit ones per group: w - zero_point exactly, and the kernel's quick forms
+// 16-bit scales, and no zero-points or 4-bit ones per group: what woq_decode_us was fitted to
 bool woq_decode_common_form(const MatmulArgs &a) {
     return wd_bits(a.wei_scale.dt) == 16 && (!a.wei_zp.ptr || (a.wei_zp.mask && wd_bits(a.wei_zp.dt) == 4));
 }
@@ -626,8 +712,8 @@ int launch_woq_decode(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     p.zp_common = a.wei_zp.ptr && !a.wei_zp.mask;
     p.sc_bits = wd_bits(a.wei_scale.dt);
     p.zp_bits = zp_rows ? wd_bits(a.wei_zp.dt) : 0;
-    const bool zp4 = zp_rows && (a.wei_zp.dt == DT_S4 || a.wei_zp.dt == DT_U4);
-    const int zpm = (p.sc_bits != 16 || (a.wei_zp.ptr && !zp4)) ? 2 : zp4 ? 1 : 0;
+    const bool inexact = a.wei_zp.dt == DT_S32 || (a.wei_zp.dt == DT_U8 && a.src_dt == DT_BF16 && a.wei_dt == DT_S4);
+    const int zpm = zp_rows ? (p.zp_bits == 4 ? 1 : inexact ? 3 : 2) : p.zp_common || p.sc_bits != 16 ? 4 : 0;
     {
         const int es = a.dst_dt == DT_F32 ? 4 : 2;
         p.fast_store = a.n_po == 0 && !a.dst_scale.ptr && !a.dst_scale.on_host

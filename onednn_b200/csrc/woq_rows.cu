@@ -652,9 +652,8 @@ int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st) {
         // us a call, this kernel -> that one: 64 x 4096 x 4096 in groups of 128 37.9 -> 18.7, of 32 104 -> 29.3; 128 rows, f16, groups of
         // 64 71.7 -> 29.2; 300 rows, groups of 32 99 -> 87; 40 x 8192 x 1024 66.6 -> 11.8; 48 x 8192 x 28672 139 -> 105;
         // 300 x 4096 x 4096 in groups of 128 stays here (39.3).  Both models are for 16-bit scales with no or 4-bit zero-points per
-        // group.  All others stay here: that kernel takes 8-bit and common zero-points off the finished sums, where activations of
-        // one sign cancel, this one off the weights, exactly; and it reads their parameters slowly (us a call, here / there: f32 scales,
-        // 64 x 4096 x 11008 in groups of 128 32.7 / 100, 300 x 4096 x 4096 in groups of 32 111 / 423).
+        // group.  All others stay here: used for them too, the models were wrong by up to five times (f32 scales, when that kernel
+        // read them one at a time, here / there: 64 x 4096 x 11008 in groups of 128 32.7 / 100, 300 x 4096 x 4096 in groups of 32 111 / 423).
         const int64_t waves = ((a.M + RT_M - 1) / RT_M * ((a.N + RT_N - 1) / RT_N) + sm_count - 1) / sm_count;
         const float here = 4.f + (float)(waves * ((a.K + RK - 1) / RK)) * (0.45f + 102.f / (float)(group < 4 * RK ? group : 4 * RK));
         if (a.M <= 65536 && woq_decode_common_form(a) && woq_decode_pointers_ok(a) && woq_decode_fits(a.M, a.K, group, a.wei_scale.dt, a.wei_zp.ptr && a.wei_zp.mask ? a.wei_zp.dt : -1)

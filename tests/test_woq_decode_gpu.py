@@ -21,6 +21,14 @@ def _common_zp(p, value, dt):
     return p
 
 
+def _wide_zp(p, dt, lo, hi):
+    """Zero-points per (group, column) of another type, in [lo, hi)."""
+    q = p.quant["wei_zp"]
+    r = np.random.Generator(np.random.PCG64(17))
+    p.quant["wei_zp"] = W.Quant(W.to_storage(r.integers(lo, hi, (p.K // q.groups[0], p.N)), dt), dt, 3, q.groups)
+    return p
+
+
 def _one_scale_row(p):
     q = p.quant["wei_scale"]
     p.quant["wei_scale"] = W.Quant(np.ascontiguousarray(q.data.reshape(-1, p.N)[:1]), q.dt, 2)
@@ -54,6 +62,21 @@ CASES = {
     "f16_s4_s4zp": lambda: W.int4_decode(13, 1024, 288, zp_dt=W.S4, src_dt=W.F16, dst_dt=W.F32),
     "u8_zp_m20": lambda: W.int4_decode(20, 512, 288, zp_dt=W.U8),
     "s8_zp_f16_m30": lambda: W.int4_decode(30, 512, 288, wei_dt=W.U4, zp_dt=W.S8, src_dt=W.F16, dst_dt=W.F16),
+    "u8_zp_f32_scales_group32": lambda: _scales(W.int4_decode(9, 544, 160, group=32, zp_dt=W.U8), W.F32),
+    "s8_zp_group16_m27": lambda: W.int4_decode(27, 272, 288, group=16, wei_dt=W.U4, zp_dt=W.S8),
+    "f32_scales_m32_group16": lambda: _scales(W.int4_decode(32, 272, 160, group=16), W.F32),
+    "f32_scales_no_zp_m24": lambda: _scales(W.int4_decode(24, 1024, 288, group=64, with_zp=False), W.F32),
+    "u8_zp_u4_weights_up_to_255": lambda: _wide_zp(W.int4_decode(6, 512, 160, wei_dt=W.U4), W.U8, 200, 256),
+    "common_s8_zp_m32_group32": lambda: _common_zp(W.int4_decode(32, 512, 160, group=32), -128, W.S8),
+    "u8_zp_m32_group64_f16": lambda: _wide_zp(W.int4_decode(32, 1024, 288, group=64, src_dt=W.F16, dst_dt=W.F16), W.U8, 0, 256),
+    # zero-points of which a rest has to come off the sums: some columns of some groups, all of them, groups across stages
+    "u8_zp_above_248": lambda: _wide_zp(W.int4_decode(5, 2048, 288, group=64), W.U8, 230, 256),
+    "u8_zp_above_248_m32_group48": lambda: _wide_zp(W.int4_decode(32, 1104, 160, group=48), W.U8, 240, 256),
+    "s32_zp_mixed_m20": lambda: _wide_zp(W.int4_decode(20, 640, 160, group=32, wei_dt=W.U4), W.S32, -400, 300),
+    "s32_zp_f16_m3": lambda: _wide_zp(W.int4_decode(3, 512, 160, src_dt=W.F16, dst_dt=W.F32), W.S32, -1100, 1100),
+    "common_s32_zp": lambda: _common_zp(W.int4_decode(18, 512, 160), -7, W.S32),
+    "common_s32_zp_large": lambda: _common_zp(W.int4_decode(7, 1040, 160, group=16), 3000, W.S32),
+    "common_u8_zp_255_per_n_scale": lambda: _common_zp(_one_scale_row(W.int4_decode(11, 1072, 288, group=16)), 255, W.U8),
     "common_zp": lambda: _common_zp(W.int4_decode(7, 512, 160), -77, W.S8),
     "f32_scales_u4_zp": lambda: _scales(W.int4_decode(12, 640, 160, group=64), W.F32),
     "f16_scales": lambda: _scales(W.int4_decode(8, 640, 160), W.F16),
@@ -100,27 +123,28 @@ def test_more_rows_match_oracle(gpu, name):
     assert np.array_equal(got, got2)
 
 
-@pytest.mark.parametrize("M", [40, 300])
+@pytest.mark.parametrize("src_dt,M", [(W.F16, 4), (W.F16, 32), (W.BF16, 4), (W.BF16, 32), (W.F16, 40), (W.F16, 300)],
+                         ids=["f16_m4", "f16_m32", "bf16_m4", "bf16_m32", "f16_m40", "f16_m300"])
 @pytest.mark.parametrize("zp", ["common_u8", "u8_per_group", "u4_per_group"])
-def test_zero_points_come_off_the_weights(gpu, M, zp):
+def test_zero_points_come_off_the_weights(gpu, src_dt, M, zp):
     """Activations of one sign: w - zero_point is taken exactly before the products are summed.  Summing over w and taking
     zero_point * sum(src) off afterwards cancels: it costs a factor of twenty and more in accuracy here."""
     eng, strm = gpu
-    p = W.int4_decode(M, 4096, 160, group=512, wei_dt=W.U4, zp_dt=W.U4 if zp == "u4_per_group" else W.U8, src_dt=W.F16, dst_dt=W.F32)
-    p.src = W.QTensor(p.src.data & 0x7fff, W.F16, p.src.dims)  # |src|
+    p = W.int4_decode(M, 4096, 160, group=512, wei_dt=W.U4, zp_dt=W.U4 if zp == "u4_per_group" else W.U8, src_dt=src_dt, dst_dt=W.F32)
+    p.src = W.QTensor(p.src.data & 0x7fff, src_dt, p.src.dims)  # |src|
     r = np.random.Generator(np.random.PCG64(21))
     if zp == "common_u8":
         _common_zp(p, 8, W.U8)
     else:
         p.quant["wei_zp"] = W.Quant(W.to_storage(r.integers(7, 10, (8, 160)), p.quant["wei_zp"].dt), p.quant["wei_zp"].dt, 3, (512, 1))
     got, impl = run_problem(p, eng, strm)
-    assert impl == "cuda:tcgen05:woq4_rows"
+    assert impl == ("cuda:tcgen05:woq4" if M <= 32 else "cuda:tcgen05:woq4_rows")
     zq = p.quant["wei_zp"]
     z = np.broadcast_to(W.to_f32(zq.data, zq.dt).astype(np.float64).reshape(-1, 160 if zp != "common_u8" else 1), (8, 160))
     w = W.to_f32(p.wei.data, W.U4).astype(np.float64).reshape(4096, 160) - np.repeat(z, 512, 0)
     q = p.quant["wei_scale"]
     w *= np.repeat(W.to_f32(q.data, q.dt).astype(np.float64).reshape(8, 160), 512, 0)
-    exact = W.to_f32(p.src.data, W.F16).astype(np.float64).reshape(M, 4096) @ w
+    exact = W.to_f32(p.src.data, src_dt).astype(np.float64).reshape(M, 4096) @ w
     err = np.linalg.norm(got - exact) / np.linalg.norm(exact)
     # a group's 32 blocks of 16 exact products are added in f32 one after another; the tensor cores cut each sum off, by up to
     # 2^-23 of it, 2^-24 on average, and the running sum is half the last one on average: 32 * 2^-24 / 2 = 9.5e-7 at most where
