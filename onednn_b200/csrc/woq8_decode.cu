@@ -7,10 +7,12 @@
 // and the sums are multiplied by 64 -, a producer warp, several such CTAs per SM, and the CTAs of a tile's K shares a
 // cluster that adds its sums in rank order through distributed shared memory.  A tile is 128 columns x up to 32 rows.
 //
-// A grouped call has a CTA (cluster) for every (column tile, expert, block of 32 rows that the expert could have); those
-// without rows leave at once.  The rows come from the offsets on the device.  Those of every expert are checked by every
-// CTA that has rows before it stores, so that one wrong offset leaves all of dst unwritten, as with the planning kernel of
-// grouped_tc.cu.
+// A grouped call has a CTA (cluster) for every column tile and every block of up to 32 rows of one expert that there can be: no
+// more blocks than rows, nor than experts and a block more for every 32 rows.  Each finds its rows from the offsets on the
+// device, checking those of all experts: one wrong offset leaves all of dst unwritten, as with the planning kernel of
+// grouped_tc.cu.  (CTAs for every expert and block left at once where there were no rows, 0.09 us of an SM each: us a call, that
+// kernel / CTAs for all / now, 8 x 1024 x 2048, 512 experts 20 / 33 / 14; 40 x 512 x 1024, 1024 experts 27 / 38 / 25;
+// 1 x 4096 x 14336, 64 experts 36 / 48 / 14; 33 x 2048 x 4096, 128 experts 70 / 76 / 57; 37 x 4096 x 14336, 8 experts 112 / 104 / 96.)
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -31,30 +33,57 @@ constexpr int NB = 32 * WARPS, NB_LOG = 7; // columns per tile
 constexpr int KS = 64, W_BYTES = KS * NB; // k-rows and weight bytes per stage
 constexpr int MAX_STAGES = 12, MAX_CLUSTER = 8;
 constexpr int CTAS = 4; // per SM: 96 registers, 55 KB each
-constexpr int BAR_BYTES = 2 * MAX_STAGES * 8 + 64;
+constexpr int BAR_BYTES = 2 * MAX_STAGES * 8 + 64, FOUND_OFFSET = 2 * MAX_STAGES * 8 + 16;
 constexpr int SMEM = 55 * 1024;
 
 struct W8Params {
     int kstages; // ceil(K / 64)
     int rows; // src rows per CTA (at most 8 * MT)
     int split_log; // log2 of the CTAs per tile = cluster size
-    int row_blocks; // blocks of `rows` rows per expert (grouped)
     int fast_store; // the value is scaled, converted and stored, four columns at a time
     int stages, stage_bytes, off_bars;
 };
 
-// Whether the offsets of expert g are wrong
-__device__ __forceinline__ bool wrong_offsets(const MatmulArgs &a, int g) {
-    const int64_t b = g == 0 ? 0 : a.offsets[g - 1], e = a.offsets[g];
-    const int64_t db = g == 0 ? 0 : a.dst_offsets[g - 1], de = a.dst_offsets[g];
-    return b < 0 || e > a.M || e < b || db < 0 || de > a.M || de < db || de - db != e - b;
-}
-// (Out of line, and called by the producer warp, which has nothing left to do: inlined it changed the code of the consumers'
-// loop, 104.0 us for 37 rows over 8 experts became 106.7; 104.4 like this.)
-__device__ __noinline__ bool some_wrong_offsets(const MatmulArgs &a, int lane) {
+// Grouped: the `y`-th block of up to 32 rows of one expert, {expert, first src row, first dst row, rows}, by a warp; no rows where
+// there are not as many blocks, or where the offsets of any expert are wrong.  (Out of line, so that the code of the consumers'
+// loop does not change with it, which cost 2 %.)
+__device__ __noinline__ int4 find_rows(const MatmulArgs &a, int y, int lane) {
+    int4 mine = make_int4(0, 0, 0, 0);
+    int before = 0; // blocks of the experts before these 32
     bool wrong = false;
-    for (int i = lane; i < a.group_count; i += 32) wrong |= wrong_offsets(a, i);
-    return wrong;
+    for (int g0 = 0; g0 < a.group_count; g0 += 32) {
+        const int g = g0 + lane;
+        int rows = 0, src_row = 0, dst_row = 0;
+        if (g < a.group_count) {
+            const int64_t b = g == 0 ? 0 : a.offsets[g - 1], e = a.offsets[g];
+            const int64_t db = g == 0 ? 0 : a.dst_offsets[g - 1], de = a.dst_offsets[g];
+            const bool bad = b < 0 || e > a.M || e < b || db < 0 || de > a.M || de < db || de - db != e - b;
+            wrong |= bad;
+            rows = bad ? 0 : (int)(e - b);
+            src_row = (int)b;
+            dst_row = (int)db;
+        }
+        const int blocks = (rows + 31) >> 5;
+        int upto = blocks; // inclusive sum over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= d) upto += x;
+        }
+        const int at = y - before - (upto - blocks); // of this expert's blocks
+        const unsigned found = __ballot_sync(0xffffffffu, at >= 0 && at < blocks);
+        if (found) {
+            const int from = __ffs(found) - 1, r0 = __shfl_sync(0xffffffffu, at, from) * 32;
+            mine = make_int4(g0 + from, __shfl_sync(0xffffffffu, src_row, from) + r0, __shfl_sync(0xffffffffu, dst_row, from) + r0,
+                    min(32, __shfl_sync(0xffffffffu, rows, from) - r0));
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (__any_sync(0xffffffffu, wrong)) {
+        if (lane == 0) atomicExch(a.status, 2); // invalid_arguments, reported when the stream is waited on
+        mine.w = 0;
+    }
+    return mine;
 }
 // general store: bias (per expert row, or the dense problem's own broadcast), post-ops, any dst type
 __device__ __noinline__ void finish_store_w8(const MatmulArgs &a, float d, int64_t m, int64_t n, int g) {
@@ -90,28 +119,31 @@ woq8_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     ptx::grid_dependency_wait();
     int g = 0, src_row, dst_row, rows;
     if (a.group_count > 0) {
-        g = (int)blockIdx.y / p.row_blocks;
-        const int64_t b = g == 0 ? 0 : a.offsets[g - 1], e = a.offsets[g];
-        const int64_t db = g == 0 ? 0 : a.dst_offsets[g - 1], de = a.dst_offsets[g];
-        const int r0 = ((int)blockIdx.y - g * p.row_blocks) * p.rows;
-        const bool wrong = b < 0 || e > a.M || e < b || db < 0 || de > a.M || de < db || de - db != e - b;
-        if (wrong && threadIdx.x == 0) atomicExch(a.status, 2); // invalid_arguments, reported when the stream is waited on
-        rows = wrong ? 0 : min((int64_t)p.rows, e - b - r0);
-        src_row = (int)b + r0;
-        dst_row = (int)db + r0;
+        int4 *const found = reinterpret_cast<int4 *>(smem + p.off_bars + FOUND_OFFSET);
+        if (warp == 0) {
+            const int4 mine = find_rows(a, (int)blockIdx.y, lane);
+            if (lane == 0) {
+                *found = mine;
+                ptx::mbar_arrive_expect_tx(sums_bar, (uint32_t)mine.w * NB * 4); // every CTA's share of this CTA's slice
+            }
+        }
+        __syncthreads();
+        g = found->x;
+        src_row = found->y;
+        dst_row = found->z;
+        rows = found->w;
         if (rows <= 0) return; // (every CTA of the cluster)
     } else {
         src_row = dst_row = (int)blockIdx.y * p.rows;
         rows = min((int64_t)p.rows, a.M - src_row);
+        if (threadIdx.x == 0) ptx::mbar_arrive_expect_tx(sums_bar, (uint32_t)rows * NB * 4);
+        __syncthreads();
     }
-    if (threadIdx.x == 0) ptx::mbar_arrive_expect_tx(sums_bar, (uint32_t)rows * NB * 4); // every CTA's share of this CTA's slice
-    __syncthreads();
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); // sums_bar is ready
 
     const int st0 = (int)((unsigned)p.kstages * rank >> split_log), st1 = (int)((unsigned)p.kstages * (rank + 1) >> split_log);
     const uint32_t ring = ptx::smem_u32(smem), bars = ptx::smem_u32(full);
     const int stages = in_reg(p.stages), stage_bytes = in_reg(p.stage_bytes);
-    bool some_wrong = false; // offsets of any expert: nothing is stored
     if (warp == WARPS) {
         // ------------------------------------------------ producer
         if (ptx::elect_one()) {
@@ -130,7 +162,6 @@ woq8_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         }
         __syncwarp();
         asm volatile("griddepcontrol.launch_dependents;"); // the CTA's loads are all on their way
-        some_wrong = some_wrong_offsets(a, lane);
         if (splits > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {
         // ------------------------------------------------ consumers
@@ -226,7 +257,7 @@ woq8_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const int slice_log = NB_LOG - split_log, slice = 1 << slice_log;
     const bool late = !ptx::mbar_wait(sums_bar, 0);
     if (late) atomicExch(a.status, 5);
-    if (__syncthreads_or(late || some_wrong)) {
+    if (__syncthreads_or(late)) {
         if (splits > 1) ptx::outlast_cluster(sums_bar);
         return;
     }
@@ -316,8 +347,12 @@ int w8_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a,
     return 0;
 }
 
-// Blocks of rows that a call of this many rows needs, and experts that they can belong to
-int64_t w8_blocks(const MatmulArgs &a) { return a.group_count > 0 ? (a.M < a.group_count ? a.M : a.group_count) : (a.M + 31) / 32; }
+// Blocks of rows that a call can need
+int64_t w8_blocks(const MatmulArgs &a) {
+    if (a.group_count == 0) return (a.M + 31) / 32;
+    const int64_t most = a.group_count + a.M / 32;
+    return a.M < most ? a.M : most;
+}
 
 } // namespace
 
@@ -325,11 +360,13 @@ int64_t w8_blocks(const MatmulArgs &a) { return a.group_count > 0 ? (a.M < a.gro
 // (0.26 for more than 16 rows), a 64-k slot of a wave of tiles 0.22 there and more with its rows.  Grouped calls: up to 64 rows.
 // us a call, that kernel -> this one: dense 1 x 4096 x 4096 22.6 -> 6.7, 16 x 4096 x 11008 24.7 -> 15.7, 64 x 4096 x 4096
 // 26.7 -> 14.1, 128 x 8192 x 1024 45.2 -> 15.0, 256 x 1024 x 1024 20.5 -> 7.7, 32 x 8192 x 16384 42.9 -> 38.0; grouped 37 rows, 8 experts,
-// 4096 x 14336 111.7 -> 104.0 (72 are the stream), 64 rows, 16 experts, 2048 x 4096 40.1 -> 33.8, 9 rows, 8 experts, 1024 x 2048 12.7 -> 6.8.
+// 4096 x 14336 112 -> 96 (72 are the stream), 64 rows, 16 experts, 2048 x 4096 40.5 -> 33.8, 9 rows, 8 experts, 1024 x 2048 13.9 -> 7.
+// How the rows are spread is not known here.  All of them with one expert is the worst case: 64 rows, 8 experts, 4096 x 14336
+// 28.9 -> 48, of narrow layers 64 x 1024 x 1024 16.6 -> 7.7.
 bool woq8_decode_wins(const MatmulArgs &a, int sm_count) {
     if (a.wei_zp.ptr || (uintptr_t)a.wei % 16 || (uintptr_t)a.src % 16) return false;
     const float sms = (float)(sm_count > 0 ? sm_count : 148);
-    if (a.group_count > 0) return a.M <= 64 && a.group_count <= 16384;
+    if (a.group_count > 0) return a.M <= 64 && a.group_count <= 1024; // (every CTA looks through them: 3 rows, 2000 experts 33 us, there 29)
     const int64_t kst = (a.K + KS - 1) / KS, ntiles = (a.N + NB - 1) / NB, blocks = w8_blocks(a);
     if (blocks > 1024) return false;
     const int64_t tiles = ntiles * ((a.M + 207) / 208), waves = (int64_t)((tiles + sms - 1) / sms);
@@ -349,8 +386,7 @@ int launch_woq8_decode(const MatmulArgs &a, int sm_count, cudaStream_t st) {
     int ny;
     if (grouped) {
         p.rows = a.M < 32 ? (int)a.M : 32;
-        p.row_blocks = (int)((a.M + 31) / 32);
-        ny = a.group_count * p.row_blocks;
+        ny = (int)w8_blocks(a);
     } else {
         const int blocks = (int)((a.M + 31) / 32);
         p.rows = (int)((a.M + blocks - 1) / blocks);

@@ -38,6 +38,13 @@ GROUPED = {
     "block_edges": lambda: W.moe_grouped(64, 320, 272, 5, sizes=[32, 0, 7, 25, 0]),
     "two_blocks_of_an_expert": lambda: W.moe_grouped(50, 1088, 160, 3, sizes=[1, 41, 8]),
     "many_experts": lambda: W.moe_grouped(40, 128, 64, 70),
+    # blocks found across the 32s of experts that a warp looks through; experts of one, two and no blocks; as many experts as
+    # the kernel takes, and one more
+    "second_32_of_experts": lambda: W.moe_grouped(64, 96, 80, 41, sizes=[0] * 30 + [1, 0, 33, 0, 0, 0, 0, 0, 0, 1, 29]),
+    "all_rows_last": lambda: W.moe_grouped(64, 64, 32, 65, sizes=[0] * 64 + [64]),
+    "one_row_each": lambda: W.moe_grouped(64, 64, 48, 64, sizes=[1] * 64),
+    "1024_experts": lambda: W.moe_grouped(63, 32, 32, 1024),
+    "1025_experts": lambda: W.moe_grouped(63, 32, 32, 1025),
 }
 
 
