@@ -51,7 +51,7 @@ size_t woq_skinny_scratch_bytes(int64_t N, int64_t K, int sm_count);
 int launch_woq_decode(const MatmulArgs &a, int sm_count, cudaStream_t st);
 bool woq_decode_pointers_ok(const MatmulArgs &a);
 bool woq_decode_common_form(const MatmulArgs &a);
-float woq_decode_us(int64_t M, int64_t N, int64_t K, int64_t group, int sm_count);
+float woq_decode_us(int64_t M, int64_t N, int64_t K, int64_t group, bool zero_points, int sm_count);
 bool woq_decode_fits(int64_t M, int64_t K, int64_t group, int scale_dt, int zp_dt);
 
 // int4 weight-decompression GEMM for M > 32 on tcgen05 (woq_rows.cu)

@@ -660,14 +660,18 @@ bool woq_decode_common_form(const MatmulArgs &a) {
 }
 
 // Microseconds that a problem takes here, for the choice between this kernel and the one whose operand lies in tensor
-// memory (woq_rows.cu) when there are more than 32 rows: a stage costs an SM 0.82 for blocks of 32 rows (0.65 for 24), more
-// with small groups (a fold of the sums at each end), and the launch about 4.
-float woq_decode_us(int64_t M, int64_t N, int64_t K, int64_t group, int sm_count) {
-    const int64_t blocks = (M + 31) / 32, rows = (M + blocks - 1) / blocks;
-    const float stage = (rows > 24 ? 0.82f : 0.65f) * (group < 64 ? 1.35f : group < 128 ? 1.1f : 1.f);
-    const int64_t stages = blocks * ((N + NB - 1) / NB) * ((K + KS - 1) / KS);
-    const float share = (float)stages / (float)(sm_count > 0 ? sm_count : 148), alone = (float)((K + KS - 1) / KS) / MAX_CLUSTER * 1.3f;
-    return 4.f + stage * (share > alone ? share : alone);
+// memory (woq_rows.cu) when there are more than 32 rows.  The busiest SM's stages, with its CTAs' starts and ends, at 0.42 (0.62 for
+// more than 24 rows), more with groups below 64 (a fold of the sums at each end).  Fitted, with that kernel's model, to 156
+// problems (33 to 512 rows, K 1024 to 8192, N 1024 to 28672, groups of 32 to 128) timed with both: within 25 % of the time (10 % for
+// eight of ten), and the choice costs 0.03 % on average, 3 % at most.
+float woq_decode_us(int64_t M, int64_t N, int64_t K, int64_t group, bool zero_points, int sm_count) {
+    if (sm_count < 1) sm_count = 148;
+    const int64_t blocks = (M + 31) / 32, rows = (M + blocks - 1) / blocks, mt = (rows + 7) / 8;
+    const int64_t tiles = (N + NB - 1) / NB * blocks, kstages = (K + KS - 1) / KS;
+    const int l = wd_split_log(tiles, (int)kstages, (int)mt, sm_count);
+    const float busiest = (float)(((tiles << l) + sm_count - 1) / sm_count), share = (float)((kstages + (1 << l) - 1) >> l);
+    const float stage = (mt > 3 ? 0.62f : 0.42f) * (group >= 64 ? 1.f : zero_points ? 1.71f : 1.35f);
+    return 3.2f + stage * (busiest > 1.1f ? busiest : 1.1f) * (share + 1.9f + 0.64f * (float)mt);
 }
 
 int launch_woq_decode(const MatmulArgs &a, int sm_count, cudaStream_t st) {

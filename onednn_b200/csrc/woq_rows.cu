@@ -647,17 +647,20 @@ int launch_woq_rows(const MatmulArgs &a, int sm_count, cudaStream_t st) {
             : (a.wei_zp.ptr && (a.wei_zp.mask & 1))                    ? a.wei_zp.g0
                                                                        : a.K;
     {
-        // The decode kernel in blocks of up to 32 rows, where it is the faster one.  This kernel takes 0.45 us a stage of a wave
-        // of tiles, and 0.8 more for every group end in it; nothing splits its K.
-        // us a call, this kernel -> that one: 64 x 4096 x 4096 in groups of 128 37.9 -> 18.7, of 32 104 -> 29.3; 128 rows, f16, groups of
-        // 64 71.7 -> 29.2; 300 rows, groups of 32 99 -> 87; 40 x 8192 x 1024 66.6 -> 11.8; 48 x 8192 x 28672 139 -> 105;
+        // The decode kernel in blocks of up to 32 rows, where it is the faster one.  This kernel takes 0.4 us a stage of a wave of
+        // tiles, and for every group end in it 0.38 and 0.0027 a row of the tile; nothing splits its K.
+        // us a call, this kernel -> that one: 64 x 4096 x 4096 in groups of 128 31.6 -> 18.8, of 32 102 -> 29; 128 rows, f16, groups of
+        // 64 63.6 -> 27; 40 x 8192 x 1024 66.6 -> 11.8; 48 x 8192 x 28672 139 -> 105; (a model without the CTAs' starts and ends sent
+        // there, too:) 300 x 1024 x 4096 in groups of 64 20.6 -> 27.7, 128 x 1024 x 28672 in groups of 32 71 -> 92.
         // 300 x 4096 x 4096 in groups of 128 stays here (39.3).  Both models are for 16-bit scales with no or 4-bit zero-points per
         // group.  All others stay here: used for them too, the models were wrong by up to five times (f32 scales, when that kernel
         // read them one at a time, here / there: 64 x 4096 x 11008 in groups of 128 32.7 / 100, 300 x 4096 x 4096 in groups of 32 111 / 423).
-        const int64_t waves = ((a.M + RT_M - 1) / RT_M * ((a.N + RT_N - 1) / RT_N) + sm_count - 1) / sm_count;
-        const float here = 4.f + (float)(waves * ((a.K + RK - 1) / RK)) * (0.45f + 102.f / (float)(group < 4 * RK ? group : 4 * RK));
+        const int64_t mtiles = (a.M + RT_M - 1) / RT_M, rows = ((a.M + mtiles - 1) / mtiles + 15) / 16 * 16;
+        const int64_t waves = (mtiles * ((a.N + RT_N - 1) / RT_N) + sm_count - 1) / sm_count;
+        const float ends = (float)RK / (float)(group < 4 * RK ? group : 4 * RK), zp = a.wei_zp.ptr ? 0.07f : 0.f; // of groups in a stage
+        const float here = 7.5f + (float)(waves * ((a.K + RK - 1) / RK)) * (0.4f + ends * (0.38f + 0.0027f * (float)rows + zp));
         if (a.M <= 65536 && woq_decode_common_form(a) && woq_decode_pointers_ok(a) && woq_decode_fits(a.M, a.K, group, a.wei_scale.dt, a.wei_zp.ptr && a.wei_zp.mask ? a.wei_zp.dt : -1)
-                && woq_decode_us(a.M, a.N, a.K, group, sm_count) < here)
+                && woq_decode_us(a.M, a.N, a.K, group, a.wei_zp.ptr != nullptr, sm_count) < here)
             return launch_woq_decode(a, sm_count, st);
     }
     RowsParams p {};
