@@ -354,10 +354,25 @@ int64_t w8_blocks(const MatmulArgs &a) {
     return a.M < most ? a.M : most;
 }
 
+// log2 of the CTAs per tile, as in woq_decode.cu: the busiest SM's stages, a CTA's start and end counted as 3 + mt, a stage alone on an
+// SM as 2.5
+int w8_split_log(int64_t tiles, int kstages, int mt, int sms) {
+    int best = 0;
+    int64_t cost = INT64_MAX;
+    for (int l = 0; 1 << l <= MAX_CLUSTER && 1 << l <= kstages; ++l) {
+        const int64_t busiest = ((tiles << l) + sms - 1) / sms, share = 2 * busiest > 5 ? 2 * busiest : 5;
+        const int64_t c = share * (((kstages + (1 << l) - 1) >> l) + 3 + mt);
+        if (c < cost) { cost = c; best = l; }
+    }
+    return best;
+}
+
 } // namespace
 
-// Whether this kernel is the faster one (else grouped_tc.cu), by a model of both in microseconds: a stage costs an SM 0.2 here
-// (0.26 for more than 16 rows), a 64-k slot of a wave of tiles 0.22 there and more with its rows.  Grouped calls: up to 64 rows.
+// Whether this kernel is the faster one (else grouped_tc.cu), by a model of both in microseconds: the busiest SM's stages with its
+// CTAs' starts and ends at 0.18 here (0.205 for more than 24 rows), a 64-k slot of a wave of tiles 0.14 there and more with its rows.
+// Fitted to 130 problems (24 to 1000 rows, K 512 to 8192, N 1024 to 16384) timed with both kernels: the choice costs 0.1 % on average, and
+// 15 % once, 3 % at most otherwise (a model of stages alone 0.9 % and 27 %: 256 x 4096 x 4096 36.8 for 29.0).  Grouped calls: up to 64 rows.
 // us a call, that kernel -> this one: dense 1 x 4096 x 4096 22.6 -> 6.7, 16 x 4096 x 11008 24.7 -> 15.7, 64 x 4096 x 4096
 // 26.7 -> 14.1, 128 x 8192 x 1024 45.2 -> 15.0, 256 x 1024 x 1024 20.5 -> 7.7, 32 x 8192 x 16384 42.9 -> 38.0; grouped 37 rows, 8 experts,
 // 4096 x 14336 112 -> 96 (72 are the stream), 64 rows, 16 experts, 2048 x 4096 40.5 -> 33.8, 9 rows, 8 experts, 1024 x 2048 13.9 -> 7.
@@ -365,14 +380,15 @@ int64_t w8_blocks(const MatmulArgs &a) {
 // 28.9 -> 48, of narrow layers 64 x 1024 x 1024 16.6 -> 7.7.
 bool woq8_decode_wins(const MatmulArgs &a, int sm_count) {
     if (a.wei_zp.ptr || (uintptr_t)a.wei % 16 || (uintptr_t)a.src % 16) return false;
-    const float sms = (float)(sm_count > 0 ? sm_count : 148);
+    const int sms = sm_count > 0 ? sm_count : 148;
     if (a.group_count > 0) return a.M <= 64 && a.group_count <= 1024; // (every CTA looks through them: 3 rows, 2000 experts 33 us, there 29)
     const int64_t kst = (a.K + KS - 1) / KS, ntiles = (a.N + NB - 1) / NB, blocks = w8_blocks(a);
     if (blocks > 1024) return false;
-    const int64_t tiles = ntiles * ((a.M + 207) / 208), waves = (int64_t)((tiles + sms - 1) / sms);
-    const int64_t per = (a.M + (a.M + 207) / 208 - 1) / ((a.M + 207) / 208);
-    const float here = 4.f + (float)(blocks * ntiles * kst) / sms * (a.M <= 16 ? 0.2f : 0.26f);
-    const float there = 6.f + (float)(waves * kst) * (0.22f + 0.0016f * (float)per);
+    const int mt = (int)(((a.M + blocks - 1) / blocks + 7) / 8), l = w8_split_log(ntiles * blocks, (int)kst, mt, sms);
+    const float busiest = (float)(((ntiles * blocks << l) + sms - 1) / sms), share = (float)((kst + (1 << l) - 1) >> l);
+    const float here = 3.8f + (mt > 3 ? 0.205f : 0.18f) * busiest * (share + 3.8f + 1.4f * (float)mt);
+    const int64_t mtiles = (a.M + 207) / 208, waves = (ntiles * mtiles + sms - 1) / sms, rows = ((a.M + mtiles - 1) / mtiles + 15) / 16 * 16;
+    const float there = 9.f + (float)(waves * kst) * (0.14f + 0.0014f * (float)rows);
     return here < there;
 }
 
@@ -423,16 +439,7 @@ int launch_woq8_decode(const MatmulArgs &a, int sm_count, cudaStream_t st) {
                 && a.dst_sm % 4 == 0 && (uintptr_t)a.dst % (4 * es) == 0;
     }
     const int ntiles = (int)((a.N + NB - 1) / NB);
-    // CTAs per tile, as in woq_decode.cu: the busiest SM's stages, a CTA's start and end counted as 3 + mt, a stage alone on an SM as 2.5
-    {
-        const int64_t sms = sm_count > 0 ? sm_count : 148, tiles = ntiles * w8_blocks(a);
-        int64_t cost = INT64_MAX;
-        for (int l = 0; 1 << l <= MAX_CLUSTER && 1 << l <= p.kstages; ++l) {
-            const int64_t busiest = ((tiles << l) + sms - 1) / sms, share = 2 * busiest > 5 ? 2 * busiest : 5;
-            const int64_t c = share * (((p.kstages + (1 << l) - 1) >> l) + 3 + mt);
-            if (c < cost) { cost = c; p.split_log = l; }
-        }
-    }
+    p.split_log = w8_split_log(ntiles * w8_blocks(a), p.kstages, mt, sm_count > 0 ? sm_count : 148);
     switch (mt) {
         case 1: return w8_launch<1>(tw, ts, a, p, ntiles, ny, st);
         case 2: return w8_launch<2>(tw, ts, a, p, ntiles, ny, st);
