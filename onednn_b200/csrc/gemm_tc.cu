@@ -108,7 +108,8 @@ void split_smem(const GemmPlan &plan, bool ones, SplitParams &sp) {
 // measured, on average.  With one tile per CTA a stage costs 89 + 2.3 bt (or, where fewer bytes are in flight, 203 per SM),
 // the epilogue 33 a row of a CTA's share (67 with a post-op chain), the exchange 8 a row and 135 a CTA of the cluster, a second
 // wave 4500; the persistent kernel's stages cost 133 + 1.7 bt (248 at least), its last tile's epilogue 20 a row, and
-// separate column-sum kernels 4050.  us a call, before -> now: int8 256 x 1024 x 1024 with a src zero-point 12.0 -> 5.7,
+// separate column-sum kernels 4050.  (A second wave of clusters takes as long as the first: 144 CTAs in clusters of three, of which
+// 135 find a place at a time, took 33.5 us for a chain 384 x 8192 x 2048 that two CTAs a tile do in 23.4.)  us a call, before -> now: int8 256 x 1024 x 1024 with a src zero-point 12.0 -> 5.7,
 // int8 17 x 4096 x 11008 20.5 -> 13.0, fp8 161 x 576 x 1824 10.2 -> 5.1, chain 3 x 6512 x 2912 27 -> 9.3.
 GemmPlan gemm_plan(int64_t M, int ntiles, int kblocks, int sm_count, bool chain, bool want_colsum, bool may_split) {
     if (sm_count < 1) sm_count = 148;
@@ -123,7 +124,9 @@ GemmPlan gemm_plan(int64_t M, int ntiles, int kblocks, int sm_count, bool chain,
             ns += 3270 + (want_colsum ? 4050 : 0) + (tiles + sm_count - 1) / sm_count * tile + 20 * rows;
         } else {
             const int64_t ctas = tiles * splits, places = (int64_t)cluster_places[per_sm - 1][splits - 1] * sm_count / 148;
-            const int64_t waves = (ctas + places - 1) / (places ? places : 1), busiest = (ctas + sm_count - 1) / sm_count;
+            const int64_t waves = (ctas + places - 1) / (places ? places : 1);
+            // CTAs that one SM runs: clusters that find no place wait for the end of a whole wave
+            const int64_t busiest = (waves - 1) * per_sm + (ctas - (waves - 1) * places + sm_count - 1) / sm_count;
             const int64_t alone = 203 / (busiest < per_sm ? busiest : per_sm), full = 89 + 23 * bt / 10;
             ns += 4090 + (waves - 1) * 4530 + 135 * splits
                     + busiest * ((kblocks + splits - 1) / splits * (full > alone ? full : alone) + rows * (chain ? 67 : 33) / splits + (splits > 1 ? 8 * rows : 0));
