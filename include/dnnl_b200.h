@@ -536,6 +536,10 @@ dnnl_status_t dnnl_cuda_interop_memory_create(dnnl_memory_t *memory, const_dnnl_
 uint64_t dnnl_cuda_interop_launch_count(void);
 /* Human-readable text of the last CUDA error seen by the calling thread. */
 const char *dnnl_cuda_interop_last_error(void);
+/* The kernel that did the calling thread's last matmul, where an implementation has several to choose from: "gemm_tc",
+ * "gemm_split", "woq_decode", "woq_rows", "woq_skinny", "woq8_decode", "grouped_tc" or "ref"; "" before the first.  (The
+ * implementation's name says which entry of the list a primitive uses, not which kernel a call of it took.) */
+const char *dnnl_cuda_interop_last_kernel(void);
 
 /* dst[M,N] (s32) = (src[M,K] (u8) - src_zero_point) x weights[K,N] (s8), all
  * row-major device buffers, enqueued on `cuda_stream` (a cudaStream_t).

@@ -83,6 +83,7 @@ def lib():
         L.dnnl_data_type_size.restype = C.c_size_t
         L.dnnl_cuda_interop_launch_count.restype = C.c_uint64
         L.dnnl_cuda_interop_last_error.restype = C.c_char_p
+        L.dnnl_cuda_interop_last_kernel.restype = C.c_char_p
         L.dnnl_primitive_desc_query_md.restype = C.c_void_p
         L.dnnl_version.restype = C.c_void_p
         L.dnnl_post_ops_append_eltwise.argtypes = [C.c_void_p, C.c_int, C.c_float, C.c_float]
@@ -440,3 +441,8 @@ class reorder(matmul):
 
 def launch_count():
     return int(lib().dnnl_cuda_interop_launch_count())
+
+
+def last_kernel():
+    """Name of the kernel that did this thread's last matmul."""
+    return lib().dnnl_cuda_interop_last_kernel().decode()

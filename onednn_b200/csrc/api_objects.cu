@@ -20,7 +20,12 @@ int g_cache_capacity = 0;
 } // namespace
 
 namespace qmm {
-void count_launch(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
+static thread_local const char *g_last_kernel = "";
+void count_launch(const char *kernel) {
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    if (kernel) g_last_kernel = kernel;
+}
+const char *last_kernel() { return g_last_kernel; }
 void set_last_error(const std::string &s) { g_last_error = s; }
 bool cuda_ok(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return true;
@@ -244,6 +249,7 @@ dnnl_status_t dnnl_set_primitive_cache_capacity(int capacity) {
 }
 uint64_t dnnl_cuda_interop_launch_count(void) { return g_launches.load(); }
 const char *dnnl_cuda_interop_last_error(void) { return g_last_error.c_str(); }
+const char *dnnl_cuda_interop_last_kernel(void) { return qmm::last_kernel(); }
 
 /* ------------------------------------------------------- memory descriptor */
 static dnnl_status_t md_check_common(int ndims, const dnnl_dims_t dims, dnnl_data_type_t dt) {

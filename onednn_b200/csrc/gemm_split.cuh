@@ -237,7 +237,7 @@ int launch_split_cfg(const CUtensorMap &mw, const CUtensorMap &ms, const MatmulA
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     if (cudaLaunchKernelEx(&cfg, kern, mw, ms, a, tp, sp) != cudaSuccess) return 5;
-    count_launch();
+    count_launch("gemm_split");
     return 0;
 }
 

@@ -287,7 +287,7 @@ int launch_cfg(const CUtensorMap &mw, const CUtensorMap &ms, const MatmulArgs &a
     // (long problems gain nothing from it and lost 1.5 %: fp8 4096 x 4096 x 14336 211.6 -> 214.9 us)
     cfg.numAttrs = tiles <= 2 * sm_count || tp.after_prekernel ? 1 : 0;
     if (cudaLaunchKernelEx(&cfg, kern, mw, ms, a, tp) != cudaSuccess) return 5;
-    count_launch();
+    count_launch("gemm_tc");
     return 0;
 }
 

@@ -647,7 +647,7 @@ int launch_grouped_tc(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
             kern<<<sms, G_THREADS, G_SMEM_BYTES, st>>>(tw, ts, ts2, ts3, a, plan, rowsum, num_k_blocks, dense);
         }
     }
-    count_launch();
+    count_launch("grouped_tc");
     return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
 

@@ -10,8 +10,9 @@
 
 namespace qmm {
 
-// bumps the per-process kernel launch counter (dnnl_cuda_interop_launch_count)
-void count_launch(int n = 1);
+// bumps the per-process kernel launch counter (dnnl_cuda_interop_launch_count) and, where the kernel is named (a literal), keeps
+// the name for the calling thread (dnnl_cuda_interop_last_kernel)
+void count_launch(const char *kernel = nullptr);
 
 // Opt-in to more than 48 KB of dynamic shared memory for `kern`.  The attribute
 // belongs to the (kernel, device) pair, so `done` - one word per kernel, a bit

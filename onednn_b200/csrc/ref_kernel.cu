@@ -214,14 +214,14 @@ int launch_ref(const MatmulArgs &a, cudaStream_t st) {
     dim3 block(256), grid((unsigned)nblocks);
     if (a.group_count > 0) {
         grouped_check_offsets<<<(a.group_count + 127) / 128, 128, 0, st>>>(a);
-        count_launch();
+        count_launch("ref");
         ref_grouped_kernel<<<grid, block, 0, st>>>(a);
     } else if (a.src_dt == DT_S8 || a.src_dt == DT_U8) {
         ref_int8_kernel<<<grid, block, 0, st>>>(a);
     } else {
         ref_fp_kernel<<<grid, block, 0, st>>>(a);
     }
-    count_launch();
+    count_launch("ref");
     return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }
 

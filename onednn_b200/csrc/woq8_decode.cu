@@ -343,7 +343,7 @@ int w8_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a,
         set_last_error(std::string("cuda:tcgen05:woq8 launch: ") + cudaGetErrorString(e));
         return 5;
     }
-    count_launch();
+    count_launch("woq8_decode");
     return 0;
 }
 

@@ -614,7 +614,7 @@ int wd_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &a,
         set_last_error(std::string("cuda:tcgen05:woq4 launch: ") + cudaGetErrorString(e));
         return 5;
     }
-    count_launch();
+    count_launch("woq_decode");
     return 0;
 }
 

@@ -622,7 +622,7 @@ int rows_launch(const CUtensorMap &tw, const CUtensorMap &ts, const MatmulArgs &
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, ts, a, p);
-    count_launch();
+    count_launch("woq_rows");
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         set_last_error(std::string("cuda:tcgen05:woq4_rows launch: ") + cudaGetErrorString(e));

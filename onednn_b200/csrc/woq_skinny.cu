@@ -536,7 +536,7 @@ int launch_woq_skinny(const MatmulArgs &a, void *scratch, int sm_count, cudaStre
         p.m_base = m0;
         p.M = (int)((a.M - m0) < MB ? (a.M - m0) : MB);
         kern<<<pl.grid, WARPS * 32, SMEM_BYTES, st>>>(tm, a, p);
-        count_launch();
+        count_launch("woq_skinny");
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 5;
 }

@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from onednn_b200 import api
 from onednn_b200 import workloads as W
 from onednn_b200.runner import run_problem
 from oracle import oracle as O
@@ -48,12 +49,30 @@ GROUPED = {
 }
 
 
+# enough rows for the other kernel, whose tile plan for a dense problem comes from the host
+DENSE_ROWS = {
+    "full_blocks": lambda: _dense(2900, 200, 1168),  # 14 x 10 tiles of up to 208 rows in one wave, 16 x 10 of up to 192 in two
+    "low_blocks": lambda: _dense(3000, 128, 1040, dst_dt=W.F32),  # one wave either way
+    "several_waves": lambda: _dense(3328, 136, 4112, per_tensor=True),
+    "bias_relu": lambda: _bias_relu(_dense(3100, 144, 1056)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(DENSE_ROWS))
+def test_dense_many_rows_match_oracle(gpu, name):
+    eng, strm = gpu
+    p = DENSE_ROWS[name]()
+    got, impl = run_problem(p, eng, strm)
+    assert (impl, api.last_kernel()) == ("cuda:tcgen05:woq8", "grouped_tc")
+    assert_parity(got, O.run_port(p), p.dst_dt, name, summation_slack(p))
+
+
 @pytest.mark.parametrize("name", sorted(DENSE))
 def test_dense_matches_oracle(gpu, name):
     eng, strm = gpu
     p = DENSE[name]()
     got, impl = run_problem(p, eng, strm)
-    assert impl == "cuda:tcgen05:woq8"
+    assert (impl, api.last_kernel()) == ("cuda:tcgen05:woq8", "woq8_decode")
     assert_parity(got, O.run_port(p), p.dst_dt, name, summation_slack(p))
     got2, _ = run_problem(p, eng, strm)
     assert np.array_equal(got, got2)
@@ -64,7 +83,7 @@ def test_grouped_matches_oracle(gpu, name):
     eng, strm = gpu
     p = GROUPED[name]()
     got, impl = run_problem(p, eng, strm)
-    assert impl == "cuda:tcgen05:grouped"
+    assert (impl, api.last_kernel()) == ("cuda:tcgen05:grouped", "grouped_tc" if name == "1025_experts" else "woq8_decode")
     assert_parity(got, O.run_port(p), p.dst_dt, name, summation_slack_grouped(p))
 
 
@@ -83,7 +102,6 @@ BAD_OFFSETS = {
 def test_grouped_bad_offsets_write_nothing(gpu, name, M):
     """One wrong offset: the call reports invalid_arguments and dst stays as it was, for few rows (whose kernel reads the
     offsets itself) as for many (which have a planning kernel)."""
-    from onednn_b200 import api
     from onednn_b200.runner import Prepared
     eng, strm = gpu
     ends, dst_ends = (f(M) if f else None for f in BAD_OFFSETS[name])

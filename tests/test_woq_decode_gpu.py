@@ -1,10 +1,13 @@
-"""int4 weight decompression for at most 32 rows: the edges of the kernel's row blocks, column tiles, K stages and groups."""
+"""int4 weight decompression: the edges of the decode kernel's row blocks, column tiles, K stages and groups, and, for more than
+32 rows, both kernels that the choice falls on."""
 import numpy as np
 import pytest
 
+from onednn_b200 import api
 from onednn_b200 import workloads as W
 from onednn_b200.runner import run_problem
 from oracle import oracle as O
+from test_parity_gpu import _requantized, _src_scale, _with_bias_relu
 from util import assert_parity, summation_slack
 
 pytestmark = pytest.mark.gpu
@@ -98,26 +101,44 @@ def test_matches_oracle(gpu, name):
 
 ROWS_CASES = {
     # blocks of rows of the decode kernel: 2 x 17, 2 x 32, 3 x 22 with a short last one, ...
-    "m33": lambda: W.int4_decode(33, 1024, 288),
-    "m64_group32": lambda: W.int4_decode(64, 512, 160, group=32),
-    "m65_f16": lambda: W.int4_decode(65, 768, 544, wei_dt=W.U4, src_dt=W.F16, dst_dt=W.F16, group=64),
-    "m97_k_tail": lambda: W.int4_decode(97, 1104, 96, group=16),
+    "m33": ("woq_decode", lambda: W.int4_decode(33, 1024, 288)),
+    "m64_group32": ("woq_decode", lambda: W.int4_decode(64, 512, 160, group=32)),
+    "m65_f16": ("woq_decode", lambda: W.int4_decode(65, 768, 544, wei_dt=W.U4, src_dt=W.F16, dst_dt=W.F16, group=64)),
+    "m97_k_tail": ("woq_decode", lambda: W.int4_decode(97, 1104, 96, group=16)),
     # enough tiles and short K for the kernel with the operand in tensor memory
-    "m1000_group128": lambda: W.int4_decode(1000, 512, 1056),
-    "m2040_group64": lambda: W.int4_decode(2040, 256, 1024, group=64),
-    "m2048_group32_u4": lambda: W.int4_decode(2048, 256, 1024, group=32, wei_dt=W.U4),
-    "m2000_group48": lambda: W.int4_decode(2000, 288, 1024, group=48),
-    "m1024_f16_u8zp": lambda: W.int4_decode(1024, 512, 1024, group=256, zp_dt=W.U8, src_dt=W.F16, dst_dt=W.F16),
-    "m1024_no_zp": lambda: W.int4_decode(1024, 528, 1024, group=528, with_zp=False, dst_dt=W.F32),
+    "m1000_group128": ("woq_rows", lambda: W.int4_decode(1000, 512, 1056)),
+    "m2040_group64": ("woq_rows", lambda: W.int4_decode(2040, 256, 1024, group=64)),
+    "m2048_group32_u4": ("woq_rows", lambda: W.int4_decode(2048, 256, 1024, group=32, wei_dt=W.U4)),
+    "m2000_group48": ("woq_rows", lambda: W.int4_decode(2000, 288, 1024, group=48)),
+    "m1024_f16_u8zp": ("woq_rows", lambda: W.int4_decode(1024, 512, 1024, group=256, zp_dt=W.U8, src_dt=W.F16, dst_dt=W.F16)),
+    "m1024_no_zp": ("woq_rows", lambda: W.int4_decode(1024, 528, 1024, group=528, with_zp=False, dst_dt=W.F32)),
+    "m1024_f16_group64": ("woq_rows", lambda: W.int4_decode(1024, 768, 1056, group=64, wei_dt=W.U4, src_dt=W.F16, dst_dt=W.F16, with_zp=False)),
+    "m1000_group64_ring_turns": ("woq_rows", lambda: W.int4_decode(1000, 1536, 1056, group=64)),
+    "m1024_one_scale_row": ("woq_rows", lambda: _one_scale_row(W.int4_decode(1024, 384, 1056))),
+    # that kernel takes scales of other types at any size: long K (the ten stages of weights turn twice), several tiles per
+    # CTA, groups of every kind, options of the epilogue
+    "f32_scales_32_groups": ("woq_rows", lambda: _scales(W.int4_decode(70, 4096, 256), W.F32)),
+    "f32_scales_long_k_tail": ("woq_rows", lambda: _scales(W.int4_decode(50, 2896, 160, group=16), W.F32)),
+    "f32_scales_group64_s4zp": ("woq_rows", lambda: _scales(W.int4_decode(129, 3072, 160, group=64, wei_dt=W.U4, zp_dt=W.S4), W.F32)),
+    "f32_scales_group256": ("woq_rows", lambda: _scales(W.int4_decode(48, 4096, 128, group=256), W.F32)),
+    "f32_scales_two_tiles_per_cta": ("woq_rows", lambda: _scales(W.int4_decode(33, 2816, 19072), W.F32)),
+    "f32_scales_bias_relu": ("woq_rows", lambda: _with_bias_relu(_scales(W.int4_decode(48, 512, 256), W.F32))),
+    "f32_scales_src_scale": ("woq_rows", lambda: _src_scale(_scales(W.int4_decode(72, 384, 160), W.F32))),
+    "f32_scales_requantized_s8": ("woq_rows", lambda: _requantized(_scales(W.int4_decode(55, 256, 160, dst_dt=W.S8), W.F32))),
+    "f8_scales": ("woq_rows", lambda: _scales(W.int4_decode(38, 512, 160, with_zp=False), W.F8_E4M3)),
+    "common_zp_f16": ("woq_rows", lambda: _common_zp(W.int4_decode(64, 2944, 160, src_dt=W.F16, dst_dt=W.F32), -128, W.S8)),
+    "u8_zp_f16_long_k": ("woq_rows", lambda: W.int4_decode(80, 2944, 256, zp_dt=W.U8, src_dt=W.F16, dst_dt=W.F32)),
 }
 
 
 @pytest.mark.parametrize("name", sorted(ROWS_CASES))
 def test_more_rows_match_oracle(gpu, name):
     eng, strm = gpu
-    p = ROWS_CASES[name]()
+    kernel, make = ROWS_CASES[name]
+    p = make()
     got, impl = run_problem(p, eng, strm)
     assert impl == "cuda:tcgen05:woq4_rows"
+    assert api.last_kernel() == kernel  # (both report that name: a change of the choice would move cases unnoticed)
     assert_parity(got, O.run_port(p), p.dst_dt, name, summation_slack(p))
     got2, _ = run_problem(p, eng, strm)
     assert np.array_equal(got, got2)
