@@ -308,15 +308,14 @@ __global__ void __launch_bounds__(256) reorder_cols4_kernel(const __grid_constan
 // dividends around every half-integer up to 255.5: no difference.)  Adding 1.5 * 2^23 rounds it to the integer in the low
 // byte.  Scales outside [2^-100, 2^100], negative ones and NaN divide.
 // Bound by the stream: 4 rows of 16 bytes (f32) or 8 of 8 in flight per thread, one wave of CTAs, equal shares, a ragged end
-// read four (eight) rows at a time too.  us a call, division or reciprocal and check -> now: f32 4096 x 14336 67.6 -> 48.1
-// (6.1 of 6.56 TB/s measured copy bandwidth), 2936 x 7192 30.8 -> 20.7, 904 x 968 8.2 -> 4.1;
-// bf16 5646 x 8896 63.5 -> 37.3, 826 x 7696 12.6 -> 7.2.
+// read four (eight) rows at a time too.  us a call, division or reciprocal and check -> now: f32 4096 x 14336 67.6 -> 47.5 to
+// 53 (0.85 to 0.94 of the measured copy bandwidth, by the box), 2936 x 7192 30.8 -> 21.1, 904 x 968 8.2 -> 4.2;
+// bf16 5646 x 8896 63.5 -> 39.0, 826 x 7696 12.6 -> 6.6.
 // It starts before its predecessor on the stream has ended, which may be what writes the matrix and its scales: both are read
 // behind the wait, by loads that stay there (the other kernels of this file are ordinary launches and may use __ldg).
 constexpr int quantize_ctas(int sdt, bool ss) { return sdt == DT_F32 && !ss ? 5 : 4; } // per SM: what the registers allow
 template <int SDT, int DDT, bool SS>
 __global__ void __launch_bounds__(256, quantize_ctas(SDT, SS)) reorder_quantize_kernel(const __grid_constant__ ReorderArgs a) {
-    asm volatile("griddepcontrol.launch_dependents;");
     constexpr float LO = DDT == DT_S8 ? -128.f : 0.f, HI = DDT == DT_S8 ? 127.f : 255.f;
     constexpr int U = SDT == DT_F32 ? 4 : 8; // rows in flight
     const int d0 = a.order[0];
@@ -390,6 +389,8 @@ __global__ void __launch_bounds__(256, quantize_ctas(SDT, SS)) reorder_quantize_
                 ((unsigned *)a.dst)[((r + u * walkers) * cols + i0) >> 2] = usual ? convert(f) : divide(f);
         }
     }
+    // the successor may start.  (As the kernel's first instruction it cost 1 to 4 %: the successor's CTAs take slots too early)
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // Layout-changing reorder of a matrix (or a batch of them): the src is contiguous along dim dr,
