@@ -551,10 +551,10 @@ dnnl_status_t select_impl(dnnl_primitive_desc &pd, int first) {
             pd.scratch_bytes = 0;
             if (i == IMPL_TCGEN05_GEMM && (pd.attr.zp(DNNL_ARG_SRC).set || pd.attr.zp(DNNL_ARG_WEIGHTS).set))
                 pd.scratch_bytes = gemm_tc_scratch_bytes(pd.M(), pd.N());
-            // the skinny GEMM keeps split-K partial sums and arrival counters there
             // the decode kernel adds its split sums through shared memory; a program that brings the scratchpad
             // itself goes on being asked for one (it need not be cleared)
             if (i == IMPL_WOQ_TC && pd.attr.scratchpad_mode == dnnl_scratchpad_mode_user) pd.scratch_bytes = 256;
+            // the skinny GEMM keeps split-K partial sums and arrival counters there
             if (i == IMPL_WOQ_GEMV)
                 pd.scratch_bytes = woq_skinny_scratch_bytes(
                         pd.N(), pd.K(), pd.engine->sm_count > 0 ? pd.engine->sm_count : 148);

@@ -109,8 +109,8 @@ void split_smem(const GemmPlan &plan, bool ones, SplitParams &sp) {
 // the epilogue 33 a row of a CTA's share (67 with a post-op chain), the exchange 8 a row and 135 a CTA of the cluster, a second
 // wave 4500; the persistent kernel's stages cost 133 + 1.7 bt (248 at least), its last tile's epilogue 20 a row, and
 // separate column-sum kernels 4050.  (A second wave of clusters takes as long as the first: 144 CTAs in clusters of three, of which
-// 135 find a place at a time, took 33.5 us for a chain 384 x 8192 x 2048 that two CTAs a tile do in 23.4.)  us a call, before -> now: int8 256 x 1024 x 1024 with a src zero-point 12.0 -> 5.7,
-// int8 17 x 4096 x 11008 20.5 -> 13.0, fp8 161 x 576 x 1824 10.2 -> 5.1, chain 3 x 6512 x 2912 27 -> 9.3.
+// 135 find a place at a time, took 33.5 us for a chain 384 x 8192 x 2048 that two CTAs a tile do in 23.4.)  us a call, before -> now: int8 256 x 1024 x 1024 with a src zero-point 12.0 -> 6.1,
+// int8 17 x 4096 x 11008 20.5 -> 13.5, fp8 161 x 576 x 1824 10.2 -> 5.1, chain 3 x 6512 x 2912 27 -> 9.3.
 GemmPlan gemm_plan(int64_t M, int ntiles, int kblocks, int sm_count, bool chain, bool want_colsum, bool may_split) {
     if (sm_count < 1) sm_count = 148;
     GemmPlan best {128, 0, 1};
@@ -305,8 +305,9 @@ bool static_scratch_of_current_device(StaticScratchSlot *out) {
 // Host side of the static scratch: the array's NAME is only a host-side
 // stand-in here; kernels need its device address, looked up once per device
 // (with that device current) by cudaGetSymbolAddress.  The call allocates
-// nothing: it enqueues a memset of the column sums, three small kernels and
-// the GEMM on the caller's stream.
+// nothing: it enqueues a header kernel and the GEMM on the caller's stream, and
+// before the persistent GEMM (enough tiles to fill the GPU) a memset of the
+// column sums and the kernel that makes them.
 extern "C" dnnl_status_t dnnl_cuda_interop_matmul_u8s8s32_zp_static(void *cuda_stream, int64_t M, int64_t N,
         int64_t K, const uint8_t *src, const int8_t *weights, int32_t src_zero_point, int32_t *dst) {
     using namespace qmm;

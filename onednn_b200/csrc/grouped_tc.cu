@@ -45,8 +45,9 @@
 // 26 KB of src rows per 64 k).  Measured on a B200, us per call, before -> now, the
 // earlier form being four issuing warps that handed the stage order on, eight
 // converter warps with three LOP3 more per pair and blocks of up to 192 rows:
-// 8192 rows over 64 experts (Zipf), K = 4096, N = 14336: 1662 -> 1384; 37 rows over 8
-// experts: 162 -> 119; dense, 777 rows, K = N = 4096: 71 -> 42.  Four converter sets
+// 8192 rows over 64 experts (Zipf), K = 4096, N = 14336: 1662 -> 1384 (first calls; 1.7 ms
+// after seconds of them, under the power cap); 37 rows over 8 experts 162 -> 119 (woq8_decode.cu now does these); dense, 777
+// rows, K = N = 4096: 71 -> 42, 38 with the host's plan and a dependent launch.  Four converter sets
 // with four slots and 192-row blocks, conversion unchanged: 1514 / 140 / 66.
 #include <cuda.h>
 

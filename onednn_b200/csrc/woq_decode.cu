@@ -24,7 +24,7 @@
 //     u * 2^-20.  One LOP3 and one packed FMA make (w - zero_point) / 64 (f16: / 512) of two
 //     nibbles, and the group's sum is multiplied by the 64.  What of a wide zero-point is not
 //     exact is taken off the sums at the end.
-// us a call, before (operand in tensor memory, two launches) -> now: 8192 x 28672, groups of 128, bf16, M = 1 49.3 -> 35.1,
+// us a call, before (operand in tensor memory, two launches) -> now: 8192 x 28672, groups of 128, bf16, M = 1 49.3 -> 36.1,
 // 8 57.9 -> 36.2, 16 73.8 -> 49.5, 32 83.9 -> 82.4; 4096 x 11008 f16, groups of 64, M = 13 41.1 -> 11.7; 4096 x 1024, groups of
 // 32, M = 32 39.4 -> 14.6; 4096 x 4096, groups of 32, M = 4 21.6 -> 10.7.
 // Other parameters, 8192 x 28672, groups of 128, bf16, that kernel / this one with scales and zero-points read one at a time and

@@ -26,14 +26,14 @@
 // Roles (28 warps): 0 weight tiles by TMA, 1 src tiles by TMA, 2 issues all MMAs, 4-11 converters (two per lane
 // quarter, taking the stages in turn), 12-27 epilogue (four per lane quarter, each a quarter of the rows).  Every mbarrier wait is bounded.
 //
-// Measured on a B200, us a call at K = N = 4096, bf16, zero-points per group, by the group size (every group costs a
-// fold of the whole accumulator and two hand-offs):
+// Measured on a B200, us a call of this kernel at K = N = 4096, bf16, zero-points per group, by the group size (every group costs
+// a fold of the whole accumulator and two hand-offs; launch_woq_rows gives most of these problems to woq_decode.cu):
 //   group            32    64   128   256
 //   M = 64          118    66    40    33
 //   M = 128         136    76    43    35
 //   M = 300         116    70    43    36
 //   M = 512         137    77    44    37
-// 32 tiles and 96 at M = 64 and 300 leave SMs idle: K is not split (launch_woq_rows says what goes to woq_decode.cu).  300 rows in groups of 128 without zero-points 37;
+// 32 tiles and 96 at M = 64 and 300 leave SMs idle: K is not split.  300 rows in groups of 128 without zero-points 37;
 // the generic kernel takes 54.3 ms for them.
 #include <cuda.h>
 #include <cuda_bf16.h>

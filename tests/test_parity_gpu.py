@@ -159,14 +159,14 @@ WOQ_CASES.update({
 @pytest.mark.parametrize("kernel", ["cuda:tcgen05:woq4", "cuda:woq:skinny"])
 @pytest.mark.parametrize("name", sorted(WOQ_CASES))
 def test_woq_decode_matches_oracle(gpu, name, kernel):
-    """Both int4 decompression kernels (tensor-memory operand; mma.sync) on every case."""
+    """Both int4 decompression kernels for few rows on every case."""
     eng, strm = gpu
     p = WOQ_CASES[name]()
     want = O.run_port(p)
     got, impl = run_problem(p, eng, strm, impl=kernel)
     assert impl == kernel
     assert_parity(got, want, p.dst_dt, name, slack_for(p, impl))
-    # the arrival counters are left at zero: a second execution gives the same bits
+    # nothing is left behind (the second kernel's arrival counters are at zero again): a second execution gives the same bits
     got2, _ = run_problem(p, eng, strm, impl=kernel)
     assert np.array_equal(got, got2)
 
@@ -435,7 +435,7 @@ def test_tcgen05_dense_woq8_matches_oracle(gpu, name):
 
 SCRATCHPAD_CASES = {
     "int8_zero_points": lambda: _wei_zp(W.int8_zp(200, 272, 176), True),  # column and row sums
-    "int4_split_k": lambda: W.int4_decode(3, 4096, 512),  # partial sums and arrival counters
+    "int4_split_k": lambda: W.int4_decode(3, 4096, 512),  # asks for a few bytes, which it does not read
     "moe_plan": lambda: W.moe_grouped(96, 256, 128, 8),  # per-expert tile ranges
     "fp8_none": lambda: W.fp8_prefill(64, 256, 128),  # asks for no scratchpad
 }
@@ -498,8 +498,7 @@ def test_runtime_m_matches_oracle(gpu, name):
 
 
 def test_one_int4_primitive_goes_from_decode_to_rows_and_back(gpu):
-    """A primitive with open M takes the decode kernel (partial sums and arrival counters in the scratchpad) or the
-    kernel for more rows (no scratchpad), by the M of each call."""
+    """A primitive with open M takes the decode kernel or the kernel for more rows, by the M of each call."""
     from onednn_b200.runner import Prepared
     eng, strm = gpu
     prim = None
